@@ -231,7 +231,7 @@ struct ScatterArgs {
 // that element's H (elcon gives the permutation of the face nodes), then
 // streams the block's entries in Hg order (rows fastest, coalesced stores).
 template <int NPF, int NCH, int NFE>
-__global__ void __launch_bounds__(256) scatter_H_block_kernel(ScatterArgs A) {
+static __global__ void __launch_bounds__(256) scatter_H_block_kernel(ScatterArgs A) {
     constexpr int BSZ = NPF * NCH, NDF = NPF * NFE, NB = NDF * NCH;
     constexpr int WARPS = 8;
     __shared__ long long s_col[WARPS][2][NPF];
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256) scatter_H_block_kernel(ScatterArgs A) {
     }
 }
 
-__global__ void scatter_R_kernel(ScatterArgs A) {
+static __global__ void scatter_R_kernel(ScatterArgs A) {
     const int bsz = A.npf * A.nch, ndf = A.npf * A.nfe;
     const int total = A.nf * bsz;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
@@ -300,7 +300,7 @@ __global__ void scatter_R_kernel(ScatterArgs A) {
 }
 
 // Partial sums of ru2 and Rr^2 per CTA (fixed grid-stride order).
-__global__ void rnorm_partial_kernel(int ne, const double* __restrict__ ru2, long long nr,
+static __global__ void rnorm_partial_kernel(int ne, const double* __restrict__ ru2, long long nr,
                                      const double* __restrict__ rr, double* __restrict__ part) {
     __shared__ double red[32];
     double s = 0.0;
@@ -318,7 +318,7 @@ __global__ void rnorm_partial_kernel(int ne, const double* __restrict__ ru2, lon
 }
 
 // out = sqrt(sum of the n partial sums), in order.
-__global__ void rnorm_final_kernel(int n, const double* __restrict__ part, double* out) {
+static __global__ void rnorm_final_kernel(int n, const double* __restrict__ part, double* out) {
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int i = 0; i < n; i++) t += part[i];
@@ -358,7 +358,7 @@ struct QSmem {
 
 // getQ (elementassembly.cpp:1414-1479), optionally preceded by getU (solutionupdate.cpp:6-68).
 template <class S>
-__global__ void __launch_bounds__(NT) getq_kernel(QArgs A) {
+static __global__ void __launch_bounds__(NT) getq_kernel(QArgs A) {
     constexpr int ND = S::ND, NPV = S::NPV, NCU = S::NCU, NC = S::NC, NCH = S::NCH, NDF = S::NDF, N = S::N, NB = S::NB;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     QSmem<S>& sm = *reinterpret_cast<QSmem<S>*>(smem_raw);
@@ -412,13 +412,13 @@ __global__ void __launch_bounds__(NT) getq_kernel(QArgs A) {
     }
 }
 
-__global__ void axpy_kernel(long long n, double alpha, const double* x, double* y) {
+static __global__ void axpy_kernel(long long n, double alpha, const double* x, double* y) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         y[i] += alpha * x[i];
 }
 
 // y += alpha[prob[i / per]] x  (per-problem step lengths on the trace unknowns)
-__global__ void axpy_prob_kernel(long long n, int per, const int* __restrict__ prob, const double* __restrict__ alpha,
+static __global__ void axpy_prob_kernel(long long n, int per, const int* __restrict__ prob, const double* __restrict__ alpha,
                                  const double* x, double* y) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         y[i] += alpha[prob[i / per]] * x[i];

@@ -22,12 +22,10 @@
 #include "krylov_kernels.cuh"
 #include "krylov_seg.cuh"
 #include "schur_kernels.cuh"
-#include "elem_kernel.cuh"
+#include "launch.cuh"
 #include "lift.cuh"
-#include "schur_tc.cuh"
 #include "bilu0.cuh"
 #include "inverse_blocked.cuh"
-#include "schur_fused.cuh"
 
 using namespace hfem;
 
@@ -39,55 +37,6 @@ struct KernelTimer {
     bool on = false;
     std::map<std::string, std::pair<double, int>> acc;
     std::vector<std::pair<std::string, std::pair<cudaEvent_t, cudaEvent_t>>> pending;
-};
-
-// Element shapes with compiled kernels: (nd, npv, npf, ngv, ngf).
-#define HFEM_SHAPES(X)          \
-    X(2, 3, 2, 3, 2)            \
-    X(2, 6, 3, 6, 3)            \
-    X(2, 10, 4, 12, 4)          \
-    X(2, 15, 5, 16, 5)          \
-    X(3, 4, 3, 4, 3)            \
-    X(3, 10, 6, 14, 6)          \
-    X(3, 20, 10, 24, 12)
-
-// GEMM tile choices per shape (m-tiles, n-tiles per warp, warps): g1 for D^-1 F
-// (n x nb, K = n), g2 for H - K D^-1 F (nb x nb, K = n); the fastest of the
-// candidates below on a B200, timed on 20k-51k-element meshes of each shape.
-// Small CTAs (1-3 warps, 2-stage) win: many resident CTAs hide the short
-// (K <= 100) main loops' fill and drain.
-template <class S> struct SchurCfg;
-template <> struct SchurCfg<Shape<2, 3, 2, 3, 2>> { using g1 = GemmCfg<2, 3, 1>; using g2 = GemmCfg<3, 3, 1>; };
-template <> struct SchurCfg<Shape<2, 6, 3, 6, 3>> { using g1 = GemmCfg<3, 5, 1>; using g2 = GemmCfg<5, 3, 2>; };
-template <> struct SchurCfg<Shape<2, 10, 4, 12, 4>> { using g1 = GemmCfg<5, 3, 2>; using g2 = GemmCfg<6, 3, 2>; };
-template <> struct SchurCfg<Shape<2, 15, 5, 16, 5>> { using g1 = GemmCfg<4, 4, 2>; using g2 = GemmCfg<4, 2, 4>; };
-template <> struct SchurCfg<Shape<3, 4, 3, 4, 3>> { using g1 = GemmCfg<3, 4, 2>; using g2 = GemmCfg<4, 2, 4>; };
-template <> struct SchurCfg<Shape<3, 10, 6, 14, 6>> { using g1 = GemmCfg<4, 4, 2>; using g2 = GemmCfg<4, 2, 4>; };
-template <> struct SchurCfg<Shape<3, 20, 10, 24, 12>> { using g1 = GemmCfg<5, 3, 3>; using g2 = GemmCfg<5, 3, 2>; };
-
-struct GemmLaunch {
-    int bm, bn, threads;
-    size_t smem;
-    const void* fn;
-    void (*run)(cudaStream_t, int, int, int, int, double, const double*, int, long long, const double*, int,
-                long long, double, double*, int, long long);
-};
-
-template <class G, int MT, int WN, int NW, int BK, int ST>
-void run_gemm(cudaStream_t st, int batch, int M, int N, int K, double alpha, const double* A, int lda, long long sA,
-              const double* B, int ldb, long long sB, double beta, double* C, int ldc, long long sC) {
-    const int tiles = ((M + G::BM - 1) / G::BM) * ((N + G::BN - 1) / G::BN);
-    batched_dgemm_kernel<MT, WN, NW, BK, ST><<<(unsigned)(tiles * batch), G::THREADS, G::SMEM, st>>>(
-        M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC);
-}
-
-template <class G> struct GemmParams;
-template <int MT, int WN, int NW, int BK, int ST> struct GemmParams<GemmCfg<MT, WN, NW, BK, ST>> {
-    static GemmLaunch make() {
-        using G = GemmCfg<MT, WN, NW, BK, ST>;
-        return GemmLaunch{G::BM, G::BN, G::THREADS, G::SMEM, (const void*)batched_dgemm_kernel<MT, WN, NW, BK, ST>,
-                          run_gemm<G, MT, WN, NW, BK, ST>};
-    }
 };
 
 // Every batched-GEMM tiling compiled into the library; any of them is valid
@@ -104,105 +53,6 @@ const std::vector<GemmLaunch>& gemm_candidates() {
         GemmParams<GemmCfg<5, 5, 5, 12, 4>>::make(), GemmParams<GemmCfg<5, 3, 2, 20, 3>>::make(),
     };
     return v;
-}
-
-struct Launch {
-    int nd, npv, npf, ngv, ngf;
-    size_t ws;                  // workspace doubles per CTA slot (element_kernel)
-    size_t q_smem;
-    void (*getq)(dim3, size_t, cudaStream_t, const QArgs&);
-    void (*inverse)(dim3, cudaStream_t, int, double*, const double*, double*, int*);
-    void (*element)(dim3, size_t, cudaStream_t, const ElemArgs&);
-    // [tf][gen]: 3xTF32 contractions; Lax-Friedrichs / Roe tensor or Sutherland's law compiled in
-    void (*element_v[2][2])(dim3, size_t, cudaStream_t, const ElemArgs&);
-    size_t elem_smem;
-    const void* elem_fn;
-    const void* elem_fn_v[2][2];
-    int inv_threads;
-    size_t inv_smem;
-    const void *q_fn, *inv_fn;
-    GemmLaunch g1, g2;
-    void (*schur_tc)(dim3, size_t, cudaStream_t, const SchurTcArgs&);
-    size_t tc_smem;
-    int tc_tmem;                // tensor-memory columns of one tensor-core Schur CTA
-    const void* tc_fn;
-    void (*scatter_h)(dim3, cudaStream_t, const ScatterArgs&);
-    void (*schur_fused)(cudaStream_t, int, const double*, const double*, const double*, double*, double*);
-    size_t fused_smem;
-    const void* fused_fn;
-};
-
-template <int N>
-void launch_inverse(dim3 g, cudaStream_t st, int ne, double* D, const double* Ru, double* RuOut, int* info) {
-    inverse_blocked_kernel<N><<<g, InvBlk<N>::THREADS, InvBlk<N>::SMEM, st>>>(ne, D, Ru, RuOut, info);
-}
-
-template <class S, bool TF, bool GEN>
-void launch_element(dim3 g, size_t sm, cudaStream_t st, const ElemArgs& a) {
-    element_kernel<S, TF, GEN><<<g, NT, sm, st>>>(a);
-}
-template <class S>
-void launch_getq(dim3 g, size_t sm, cudaStream_t st, const QArgs& a) { getq_kernel<S><<<g, NT, sm, st>>>(a); }
-template <class S>
-void launch_scatter_h(dim3 g, cudaStream_t st, const ScatterArgs& a) {
-    scatter_H_block_kernel<S::NPF, S::NCH, S::NFE><<<g, 256, 0, st>>>(a);
-}
-template <class S>
-void launch_schur_tc(dim3 g, size_t sm, cudaStream_t st, const SchurTcArgs& a) {
-    schur_tc_kernel<S::N, S::NB><<<g, TC_THREADS, sm, st>>>(a);
-}
-
-// strip width and warps of the fused FP64 condensation per shape
-template <class S>
-struct FusedPick {
-    static constexpr int BN = S::NB >= 40 ? 40 : ((S::NB + 7) / 8) * 8;
-    static constexpr int MT = (S::N + 7) / 8;
-    static constexpr int NW = MT >= 4 ? 4 : MT;
-    using Cfg = FusedCfg<S::N, S::NB, BN, NW>;
-};
-template <class S>
-void launch_schur_fused(cudaStream_t st, int ne, const double* Dinv, const double* F, const double* K, double* H,
-                        double* DinvF) {
-    static_assert(S::NB <= LIFT_MAXNB, "the lift stages one column of H per warp");
-    using P = FusedPick<S>;
-    schur_fused_kernel<S::N, S::NB, P::BN, P::NW>
-        <<<(unsigned)(ne * P::Cfg::STRIPS), P::Cfg::THREADS, P::Cfg::SMEM, st>>>(ne, Dinv, F, K, H, DinvF);
-}
-
-template <class S>
-Launch make_launch() {
-    Launch L;
-    L.nd = S::ND; L.npv = S::NPV; L.npf = S::NPF; L.ngv = S::NGV; L.ngf = S::NGF;
-    L.ws = EK<S>::WS;
-    L.q_smem = sizeof(QSmem<S>);
-    L.getq = launch_getq<S>;
-    L.q_fn = (const void*)getq_kernel<S>;
-    L.inverse = launch_inverse<S::N>;
-    L.element = launch_element<S, false, false>;
-    L.element_v[0][0] = launch_element<S, false, false>;
-    L.element_v[0][1] = launch_element<S, false, true>;
-    L.element_v[1][0] = launch_element<S, true, false>;
-    L.element_v[1][1] = launch_element<S, true, true>;
-    L.elem_smem = sizeof(ElemSmem<S>);
-    L.elem_fn = (const void*)element_kernel<S, false, false>;
-    L.elem_fn_v[0][0] = (const void*)element_kernel<S, false, false>;
-    L.elem_fn_v[0][1] = (const void*)element_kernel<S, false, true>;
-    L.elem_fn_v[1][0] = (const void*)element_kernel<S, true, false>;
-    L.elem_fn_v[1][1] = (const void*)element_kernel<S, true, true>;
-    L.inv_threads = InvBlk<S::N>::THREADS;
-    L.inv_smem = InvBlk<S::N>::SMEM;
-    L.inv_fn = (const void*)inverse_blocked_kernel<S::N>;
-    L.g1 = GemmParams<typename SchurCfg<S>::g1>::make();
-    L.g2 = GemmParams<typename SchurCfg<S>::g2>::make();
-    L.schur_tc = launch_schur_tc<S>;
-    L.tc_smem = TcCfg<S::N, S::NB>::SMEM;
-    L.tc_tmem = (int)TcCfg<S::N, S::NB>::TMEM_COLS;
-    L.tc_fn = (const void*)schur_tc_kernel<S::N, S::NB>;
-    L.scatter_h = launch_scatter_h<S>;
-    L.schur_fused = launch_schur_fused<S>;
-    L.fused_smem = FusedPick<S>::Cfg::SMEM;
-    L.fused_fn = (const void*)schur_fused_kernel<S::N, S::NB, FusedPick<S>::BN, FusedPick<S>::NW>;
-    return L;
 }
 
 const std::vector<Launch>& launches() {

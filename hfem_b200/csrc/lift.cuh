@@ -66,7 +66,7 @@ __device__ __forceinline__ double lift_add_col(const LiftArgs& L, const LiftTabl
 constexpr int LIFT_WARPS = 8;
 constexpr int LIFT_MAXNB = 200;                  // trace dofs per element (tetrahedron p = 3)
 
-__global__ void __launch_bounds__(32 * LIFT_WARPS) lift_inplace_kernel(int ne, int rows, LiftArgs L,
+static __global__ void __launch_bounds__(32 * LIFT_WARPS) lift_inplace_kernel(int ne, int rows, LiftArgs L,
                                                                        double* __restrict__ T) {
     __shared__ LiftTable tab;
     __shared__ double hs[LIFT_WARPS][LIFT_MAXNB];

@@ -54,7 +54,7 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
 
 template <int MT, int WN, int NW, int BK_ = 20, int STAGES_ = 2>
-__global__ void __launch_bounds__(32 * NW) batched_dgemm_kernel(int M, int N, int K, double alpha,
+static __global__ void __launch_bounds__(32 * NW) batched_dgemm_kernel(int M, int N, int K, double alpha,
                                                                 const double* __restrict__ A, int lda, long long sA,
                                                                 const double* __restrict__ B, int ldb, long long sB,
                                                                 double beta, double* __restrict__ C, int ldc,
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(32 * NW) batched_dgemm_kernel(int M, int N, in
 }
 
 // y_e = y_e + alpha A_e x_e   (A_e: M x K column-major)
-__global__ void batched_dgemv_kernel(int batch, int M, int K, double alpha, const double* __restrict__ A,
+static __global__ void batched_dgemv_kernel(int batch, int M, int K, double alpha, const double* __restrict__ A,
                                      long long sA, const double* __restrict__ x, long long sx, double* __restrict__ y,
                                      long long sy) {
     const long long total = (long long)batch * M;
