@@ -66,6 +66,15 @@ const std::vector<Launch>& launches() {
 
 }  // namespace
 
+// Pieces of a segmented Krylov vector (krylov_seg.cuh) on the device.
+struct SegTab {
+    int npieces = 0, nseg = 0, rows = 0;    // rows: entries per thread of a piece's CTA
+    long long* pstart = nullptr;
+    int *pseg = nullptr, *p0 = nullptr, *ticket = nullptr;
+    double* part = nullptr;
+    size_t part_n = 0;
+};
+
 struct hfem_ctx {
     hfem_dims dims{};
     int device = 0;
@@ -82,9 +91,6 @@ struct hfem_ctx {
     std::vector<cudaEvent_t> chunk_ev;
     std::vector<int> chunk_lo;              // first element of each piece, plus ne
     int pending_chunks = 0;
-    double* seg_partk = nullptr;            // CGS2 partial dots, npieces x (restart + 1)
-    size_t seg_partk_n = 0;
-    int seg_hP = 0;
     // 0 FP64; 1 3xTF32 element contractions, TF32 tensor-core Schur GEMMs, FP32
     // preconditioner; 2 FP32 preconditioner only; 3 3xTF32 element contractions,
     // FP64 Schur, FP32 preconditioner
@@ -120,7 +126,7 @@ struct hfem_ctx {
     double *ru2 = nullptr, *Hg = nullptr, *Rg = nullptr, *Rr = nullptr, *rnorm = nullptr, *ws = nullptr;
     int* info = nullptr;
     // Krylov
-    double *Minv = nullptr, *V = nullptr, *w = nullptr, *x = nullptr, *pb = nullptr, *scal = nullptr, *part = nullptr;
+    double *Minv = nullptr, *V = nullptr, *w = nullptr, *x = nullptr, *pb = nullptr;
     float* Minv32 = nullptr;    // FP32 block-Jacobi inverses (mixed mode)
     int* binfo = nullptr;
     int krylov_restart = 0;
@@ -130,19 +136,17 @@ struct hfem_ctx {
     bool palpha_on = false;
     int *eprob = nullptr, *fprob = nullptr;
     double *pparam = nullptr, *palpha = nullptr;
-    // per-problem Krylov segments (faces of each problem contiguous)
-    int npieces = 0;
-    long long* seg_pstart = nullptr;
-    int *seg_pseg = nullptr, *seg_p0 = nullptr, *seg_ticket = nullptr;
-    double *seg_part = nullptr, *seg_h = nullptr, *seg_y = nullptr, *seg_nrm = nullptr;
-    // GMRES bookkeeping on the device (GmState): Hessenberg, rotations, g, rhs norms, states
+    // Krylov segments: the whole trace vector as one segment, and one segment
+    // per problem (set_problem_map, when each problem's faces are contiguous)
+    SegTab seg_one, seg_map;
+    // GMRES bookkeeping on the device (GmState): Hessenberg, rotations, g, rhs norms, column factors, states,
+    // the projections of a step, the cycle's coefficients y and step counts
     double *gm_H = nullptr, *gm_cs = nullptr, *gm_sn = nullptr, *gm_g = nullptr, *gm_nrmb = nullptr, *gm_hist = nullptr;
-    int *gm_state = nullptr, *gm_its = nullptr, *gm_jc = nullptr;
+    double *gm_sc = nullptr, *gm_h = nullptr, *gm_y = nullptr;
+    int *gm_state = nullptr, *gm_its = nullptr, *gm_jc = nullptr, *gm_k = nullptr;
+    unsigned char* gm_act = nullptr;
     size_t gm_hist_n = 0;
-    unsigned char* seg_act = nullptr;
-    int* seg_k = nullptr;
-    int seg_restart = 0;
-    bool seg_single = false;    // segment tables describe one segment over the whole vector
+    int gm_restart = 0, gm_P = 0;
     // BILU0: ordering (computed once, from the first system), level schedule, factors
     bool have_order = false;
     std::vector<int> h_o2u, h_u2o, lvl_lo, lvl_up;
@@ -155,7 +159,6 @@ struct hfem_ctx {
     cudaGraphExec_t bilu_exec = nullptr;    // the factorisation's per-level launches, replayed as one graph
     double *Mg = nullptr, *bl_t = nullptr, *bl_y = nullptr;
     float* Mg32 = nullptr;              // FP32 copy of the BILU0 factors (mixed precision)
-    int prec_kind = 2;                  // preconditioner of the current GMRES: 2 BJ, 0 BILU0, -1 none
     KernelTimer timer;
 };
 
@@ -605,12 +608,6 @@ int launch_getq(hfem_ctx* c, const double* duh, double alpha) {
 
 long long nvec(hfem_ctx* c) { return (long long)c->dims.nf * c->bsz; }
 
-int dot(hfem_ctx* c, const double* a, const double* b, double* out, bool sq) {
-    dot_partial_kernel<<<DOT_CTAS, DOT_THREADS, 0, c->stream>>>(nvec(c), a, b, c->part);
-    dot_final_kernel<<<1, 256, 0, c->stream>>>(c->part, out, sq ? 1 : 0);
-    return check_launch(c, "dot");
-}
-
 // ---------------------------------------------------------------- BILU0
 // Block sizes with one-CTA (scheduled) instances of the factorisation and the
 // solves; they run when the levels are short (few rows per level, as the MDF
@@ -1035,24 +1032,6 @@ int bilu0_apply(hfem_ctx* c, const double* x, double* v) {
     return check_launch(c, "bilu0_apply");
 }
 
-int matvec_prec(hfem_ctx* c, const double* x, double* z, bool prec) {
-    Timed t(c, "matvec");
-    if (prec && c->prec_kind == 0) {
-        bsr_matvec_bj_kernel<double><<<std::min(c->dims.nf, sms(c->device) * 16), 64, sizeof(double) * 64, c->stream>>>(
-            c->dims.nf, c->bsz, c->rowstart, c->colidx, c->Hg, (const double*)nullptr, x, c->bl_t);
-        int rc = check_launch(c, "matvec");
-        if (rc) return rc;
-        return bilu0_apply(c, c->bl_t, z);
-    }
-    if (prec && c->precision >= 1)
-        bsr_matvec_bj_kernel<float><<<std::min(c->dims.nf, sms(c->device) * 16), 64, sizeof(double) * 64, c->stream>>>(
-            c->dims.nf, c->bsz, c->rowstart, c->colidx, c->Hg, c->Minv32, x, z);
-    else
-        bsr_matvec_bj_kernel<double><<<std::min(c->dims.nf, sms(c->device) * 16), 64, sizeof(double) * 64, c->stream>>>(
-            c->dims.nf, c->bsz, c->rowstart, c->colidx, c->Hg, prec ? c->Minv : nullptr, x, z);
-    return check_launch(c, "matvec");
-}
-
 int ensure_krylov(hfem_ctx* c, int restart) {
     int rc;
     const size_t n = nvec(c);
@@ -1061,12 +1040,10 @@ int ensure_krylov(hfem_ctx* c, int restart) {
         if ((rc = dalloc(c, &c->w, n))) return rc;
         if ((rc = dalloc(c, &c->pb, n))) return rc;
         if ((rc = dalloc(c, &c->Minv, (size_t)c->dims.nf * c->bsz * c->bsz))) return rc;
-        if ((rc = dalloc(c, &c->part, DOT_CTAS))) return rc;
         if ((rc = dalloc(c, &c->binfo, c->dims.nf))) return rc;
     }
     if (c->krylov_restart < restart) {
         if ((rc = dalloc(c, &c->V, n * (restart + 1)))) return rc;
-        if ((rc = dalloc(c, &c->scal, (size_t)(restart + 2) * (restart + 2)))) return rc;
         c->krylov_restart = restart;
     }
     return 0;
@@ -1115,327 +1092,240 @@ int bj_factor(hfem_ctx* c) {
     return check_launch(c, "bj_inverse");
 }
 
-int gmres_seg_impl(hfem_ctx* c, int precond, int restart, double tol, int maxit, int* conv, int* iters,
-                   double* hist, int hist_len);
-
-int gmres_impl(hfem_ctx* c, int precond, int restart, double tol, int maxit, int* conv, int* iters, double* hist,
-               int hist_len) {
-    // one problem, block Jacobi or none: the fused single-segment kernels
-    if (c->nprob == 0 && precond != 0 && c->assembled)
-        return gmres_seg_impl(c, precond, restart, tol, maxit, conv, iters, hist, hist_len);
-    int rc;
-    if (!c->assembled) return fail(c, HFEM_E_STATE, "assemble before gmres");
-    if (restart < 1 || maxit < 1 || !(tol > 0.0)) return fail(c, HFEM_E_ARG, "restart, maxit and tol must be positive");
-    if (precond != -1 && precond != 0 && precond != 2)
-        return fail(c, HFEM_E_ARG, "precond must be -1 (none), 0 (BILU0) or 2 (block Jacobi)");
-    if ((rc = ensure_krylov(c, restart))) return rc;
-    const long long n = nvec(c);
-    const int g = sms(c->device) * 4;
-    const bool prec = precond != -1;
-    c->prec_kind = precond;
-    if (precond == 0) {
-        if (!c->have_order && (rc = compute_ordering(c))) return rc;
-        if ((rc = bilu0_factor(c))) return rc;
-        if ((rc = bilu0_apply(c, c->Rg, c->pb))) return rc;
-    } else if (prec) {
-        if ((rc = bj_factor(c))) return rc;
-        std::vector<int> bi(c->dims.nf);
-        CK(cudaMemcpyAsync(bi.data(), c->binfo, sizeof(int) * bi.size(), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        for (int i = 0; i < c->dims.nf; i++)
-            if (bi[i]) return fail(c, HFEM_E_SINGULAR, "diagonal block of face %d is singular", i);
-        if (c->precision >= 1) {
-            const long long nm = (long long)c->dims.nf * c->bsz * c->bsz;
-            if (!c->Minv32 && (rc = dalloc(c, &c->Minv32, (size_t)nm))) return rc;
-            to_float_kernel<<<g, 256, 0, c->stream>>>(nm, c->Minv, c->Minv32);
-            bj_apply_kernel<float><<<g, 256, 0, c->stream>>>(c->dims.nf, c->bsz, c->Minv32, c->Rg, c->pb);
-        } else {
-            bj_apply_kernel<double><<<g, 256, 0, c->stream>>>(c->dims.nf, c->bsz, c->Minv, c->Rg, c->pb);
-        }
-    } else {
-        CK(cudaMemcpyAsync(c->pb, c->Rg, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-    }
-    CK(cudaMemsetAsync(c->x, 0, sizeof(double) * n, c->stream));
-    // scal layout: [0] nrmb, [1] beta, [2 .. 2+restart] current Hessenberg column, [..] y
-    double* d_nrmb = c->scal;
-    double* d_beta = c->scal + 1;
-    double* d_h = c->scal + 2;
-    double* d_y = c->scal + 3 + restart;
-    if ((rc = dot(c, c->pb, c->pb, d_nrmb, true))) return rc;
-    double nrmb = 0.0;
-    CK(cudaMemcpyAsync(&nrmb, d_nrmb, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (nrmb == 0.0) nrmb = 1.0;
-    std::vector<double> h((size_t)(restart + 1) * restart), cs(restart), sn(restart), gv(restart + 1), y(restart),
-        hcol(restart + 2);
-    int it = 0, flag = -2;
-    while (flag == -2) {
-        // r = M^-1 (b - A x) computed as M^-1 b - M^-1 A x (the same left-preconditioned residual)
-        if ((rc = matvec_prec(c, c->x, c->w, prec))) return rc;
-        sub_from_kernel<<<g, 256, 0, c->stream>>>(n, c->pb, c->w);
-        if ((rc = dot(c, c->w, c->w, d_beta, true))) return rc;
-        double beta = 0.0;
-        CK(cudaMemcpyAsync(&beta, d_beta, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        if (beta / nrmb <= tol) { flag = 0; break; }
-        scale_dev_kernel<<<g, 256, 0, c->stream>>>(n, d_beta, c->w, c->V);
-        std::fill(gv.begin(), gv.end(), 0.0);
-        gv[0] = beta;
-        int j = 0;
-        for (; j < restart; j++) {
-            double* vj = c->V + (size_t)j * n;
-            double* vn = c->V + (size_t)(j + 1) * n;
-            if ((rc = matvec_prec(c, vj, vn, prec))) return rc;
-            {
-                Timed t(c, "orthogonalise");
-                for (int i = 0; i <= j; i++) {             // modified Gram-Schmidt
-                    if ((rc = dot(c, c->V + (size_t)i * n, vn, d_h + i, false))) return rc;
-                    axpy_dev_kernel<<<g, 256, 0, c->stream>>>(n, d_h + i, c->V + (size_t)i * n, vn);
-                }
-                if ((rc = dot(c, vn, vn, d_h + j + 1, true))) return rc;
-                scale_dev_kernel<<<g, 256, 0, c->stream>>>(n, d_h + j + 1, vn, vn);
-            }
-            CK(cudaMemcpyAsync(hcol.data(), d_h, sizeof(double) * (j + 2), cudaMemcpyDeviceToHost, c->stream));
-            CK(cudaStreamSynchronize(c->stream));
-            for (int i = 0; i <= j + 1; i++) h[i + (restart + 1) * j] = hcol[i];
-            const double nn = hcol[j + 1];
-            for (int i = 0; i < j; i++) {
-                const double a = h[i + (restart + 1) * j], b = h[i + 1 + (restart + 1) * j];
-                h[i + (restart + 1) * j] = cs[i] * a + sn[i] * b;
-                h[i + 1 + (restart + 1) * j] = -sn[i] * a + cs[i] * b;
-            }
-            const double a = h[j + (restart + 1) * j], b = h[j + 1 + (restart + 1) * j];
-            const double rr = std::sqrt(a * a + b * b);
-            cs[j] = a / rr;
-            sn[j] = b / rr;
-            h[j + (restart + 1) * j] = rr;
-            h[j + 1 + (restart + 1) * j] = 0.0;
-            gv[j + 1] = -sn[j] * gv[j];
-            gv[j] = cs[j] * gv[j];
-            const double res = std::fabs(gv[j + 1]);
-            if (hist && it < hist_len) hist[it] = res / nrmb;
-            it++;
-            if (res / nrmb <= tol) { flag = 0; j++; break; }
-            if (it >= maxit) { flag = 1; j++; break; }
-            if (nn == 0.0) { flag = -1; j++; break; }
-        }
-        for (int i = j - 1; i >= 0; i--) {
-            double s = gv[i];
-            for (int k = i + 1; k < j; k++) s -= h[i + (restart + 1) * k] * y[k];
-            y[i] = s / h[i + (restart + 1) * i];
-        }
-        CK(cudaMemcpyAsync(d_y, y.data(), sizeof(double) * j, cudaMemcpyHostToDevice, c->stream));
-        combine_kernel<<<g, 256, 0, c->stream>>>(n, j, c->V, d_y, c->x);
-        if ((rc = check_launch(c, "combine"))) return rc;
-    }
-    CK(cudaStreamSynchronize(c->stream));
-    flush_timer(c);
-    if (iters) *iters = it;
-    if (conv) *conv = (flag == 0) ? 1 : (flag == 1 ? 0 : -1);
-    return 0;
-}
-
-// z = M^-1 Hg x (M^-1 omitted when !prec) by the warp-per-row kernel, rows
-// of problems with act[p] == 0 skipped.
-int matvec_warp(hfem_ctx* c, const double* x, double* z, bool prec, const unsigned char* act) {
-    Timed t(c, "matvec_warp");
-    const int grid = std::max(1, std::min((c->dims.nf + 7) / 8, sms(c->device) * 8));
+// z = xsc M^-1 Hg x (M^-1 omitted when !prec), rows of problems with
+// act[p] == 0 skipped; xsc: a factor per segment (NULL: 1).
+int matvec(hfem_ctx* c, const double* x, double* z, bool prec, const double* xsc, const unsigned char* act) {
+    Timed t(c, "matvec");
+    const int nf = c->dims.nf;
     const double* M = prec ? c->Minv : nullptr;
+    const bool f32 = prec && c->precision >= 1;
     const int* rseg = act ? c->fprob : nullptr;
+    const int grid = std::max(1, std::min((nf + 7) / 8, sms(c->device) * 8));
     switch (c->bsz) {
-#define HFEM_MV(B)                                                                                                \
-    case B:                                                                                                       \
-        if (prec && c->precision >= 1)                                                                            \
-            bsr_matvec_warp_kernel<B, float><<<grid, 256, 0, c->stream>>>(c->dims.nf, c->rowstart, c->colidx,      \
-                                                                            c->Hg, c->Minv32, x, z, rseg, act);   \
-        else                                                                                                      \
-            bsr_matvec_warp_kernel<B, double><<<grid, 256, 0, c->stream>>>(c->dims.nf, c->rowstart, c->colidx,     \
-                                                                             c->Hg, M, x, z, rseg, act);          \
+        // small or odd block sizes: a warp per block row
+#define HFEM_MV(B)                                                                                                   \
+    case B:                                                                                                          \
+        if (f32)                                                                                                     \
+            bsr_matvec_warp_kernel<B, float><<<grid, 256, 0, c->stream>>>(nf, c->rowstart, c->colidx, c->Hg,          \
+                                                                          c->Minv32, x, xsc, z, rseg, act);          \
+        else                                                                                                         \
+            bsr_matvec_warp_kernel<B, double><<<grid, 256, 0, c->stream>>>(nf, c->rowstart, c->colidx, c->Hg, M, x,   \
+                                                                           xsc, z, rseg, act);                       \
         break;
-        HFEM_MV(8) HFEM_MV(12) HFEM_MV(15) HFEM_MV(16) HFEM_MV(20) HFEM_MV(30) HFEM_MV(50)
+        HFEM_MV(8) HFEM_MV(12) HFEM_MV(15) HFEM_MV(16)
+#undef HFEM_MV
+        // larger ones: a CTA per block row
+#define HFEM_MV(B)                                                                                                   \
+    case B:                                                                                                          \
+        if (f32)                                                                                                     \
+            bsr_matvec_row_kernel<B, float><<<nf, RowMv<B>::THREADS, 0, c->stream>>>(                                 \
+                nf, c->rowstart, c->colidx, c->Hg, c->Minv32, x, xsc, z, rseg, act);                                 \
+        else                                                                                                         \
+            bsr_matvec_row_kernel<B, double><<<nf, RowMv<B>::THREADS, 0, c->stream>>>(                                \
+                nf, c->rowstart, c->colidx, c->Hg, M, x, xsc, z, rseg, act);                                         \
+        break;
+        HFEM_MV(20) HFEM_MV(30) HFEM_MV(50)
 #undef HFEM_MV
         default: return fail(c, HFEM_E_UNSUPPORTED, "no block matvec for block size %d", c->bsz);
     }
-    return check_launch(c, "matvec_warp");
+    return check_launch(c, "matvec");
 }
 
-// Restarted, left-preconditioned GMRES with modified Gram-Schmidt run for
-// every problem of the context at once (kernel/gmres_bilu0.m:17-105 per
-// problem).  Each problem has its own Krylov basis (its segment of the
-// vectors), Hessenberg matrix, Givens rotations and stopping test, so it takes
-// exactly the iterations it takes alone; the launches are shared, and a
-// problem that has stopped is skipped by every kernel.
-// Segment tables for one segment over the whole trace vector (GMRES of a
-// context without a problem map runs on the same fused kernels).
-int ensure_single_segment(hfem_ctx* c) {
-    if (c->seg_single) return 0;
-    const long long ntot = (long long)c->dims.nf * c->bsz;
-    long long piece = 1024;
-    while (piece < SEG_PIECE && piece * 4 * sms(c->device) < ntot) piece *= 2;
+// The pieces of `count[p]` consecutive entries per segment p: a power of two of
+// SEG_THREADS up to SEG_PIECE entries each, about one CTA per SM.
+int build_segments(hfem_ctx* c, SegTab& T, const std::vector<long long>& count) {
+    long long ntot = 0;
+    for (long long v : count) ntot += v;
+    long long piece = SEG_THREADS;
+    while (piece < SEG_PIECE && piece * 2 * sms(c->device) < ntot) piece *= 2;
     std::vector<long long> pstart;
-    std::vector<int> pseg;
-    for (long long s = 0; s < ntot; s += piece) {
-        pstart.push_back(s);
-        pseg.push_back(0);
+    std::vector<int> pseg, p0;
+    long long a = 0;
+    for (size_t p = 0; p < count.size(); p++) {
+        p0.push_back((int)pseg.size());
+        for (long long s = a; s < a + count[p]; s += piece) {
+            pstart.push_back(s);
+            pseg.push_back((int)p);
+        }
+        a += count[p];
     }
-    pstart.push_back(ntot);
-    const int p0[2] = {0, (int)pseg.size()};
+    p0.push_back((int)pseg.size());
+    pstart.push_back(a);
     int rc;
-    if ((rc = upload(c, &c->seg_pstart, pstart.data(), pstart.size())) ||
-        (rc = upload(c, &c->seg_pseg, pseg.data(), pseg.size())) || (rc = upload(c, &c->seg_p0, p0, 2)) ||
-        (rc = dalloc(c, &c->seg_ticket, 1)) || (rc = dalloc(c, &c->seg_part, pseg.size())) ||
-        (rc = dalloc(c, &c->seg_nrm, 2)) || (rc = dalloc(c, &c->seg_act, 1)) || (rc = dalloc(c, &c->seg_k, 1)))
+    if ((rc = upload(c, &T.pstart, pstart.data(), pstart.size())) ||
+        (rc = upload(c, &T.pseg, pseg.data(), pseg.size())) || (rc = upload(c, &T.p0, p0.data(), p0.size())) ||
+        (rc = dalloc(c, &T.ticket, count.size())))
         return rc;
-    CK(cudaMemsetAsync(c->seg_ticket, 0, sizeof(int), c->stream));
-    c->npieces = (int)pseg.size();
-    c->seg_restart = 0;
-    c->seg_single = true;
+    CK(cudaMemsetAsync(T.ticket, 0, sizeof(int) * count.size(), c->stream));
+    CK(cudaStreamSynchronize(c->stream));       // the host tables above are read until here
+    T.npieces = (int)pseg.size();
+    T.nseg = (int)count.size();
+    T.rows = (int)(piece / SEG_THREADS);
     return 0;
 }
 
-int gmres_seg_impl(hfem_ctx* c, int precond, int restart, double tol, int maxit, int* conv, int* iters,
-                   double* hist = nullptr, int hist_len = 0) {
+// The preconditioner of one GMRES: factors of the current Hg, and pb = M^-1 Rg.
+int prepare_preconditioner(hfem_ctx* c, int precond) {
     int rc;
-    if (!c->assembled) return fail(c, HFEM_E_STATE, "assemble before gmres");
-    const bool single = c->nprob == 0;
-    if (single && (rc = ensure_single_segment(c))) return rc;
-    if (!single && (!c->npieces || c->seg_single))
-        return fail(c, HFEM_E_STATE, "per-problem GMRES needs a problem map with each problem's faces contiguous");
-    if (restart < 1 || maxit < 1 || !(tol > 0.0)) return fail(c, HFEM_E_ARG, "restart, maxit and tol must be positive");
-    if (precond != -1 && precond != 2) return fail(c, HFEM_E_ARG, "precond must be -1 (none) or 2 (block Jacobi)");
-    if ((rc = ensure_krylov(c, restart))) return rc;
-    const int P = single ? 1 : c->nprob;
-    const unsigned char* mv_act = single ? nullptr : c->seg_act;   // row -> problem map only with a problem map
-    if (c->seg_restart < restart || c->seg_hP < P) {
-        // Hessenberg column (restart + 2 rows) and the second projection of
-        // CGS2 (restart + 1 rows), P problems each
-        if ((rc = dalloc(c, &c->seg_h, (size_t)(2 * restart + 3) * P))) return rc;
-        if ((rc = dalloc(c, &c->seg_y, (size_t)restart * P))) return rc;
-        if ((rc = dalloc(c, &c->gm_H, (size_t)(restart + 1) * restart * P)) ||
-            (rc = dalloc(c, &c->gm_cs, (size_t)restart * P)) || (rc = dalloc(c, &c->gm_sn, (size_t)restart * P)) ||
-            (rc = dalloc(c, &c->gm_g, (size_t)(restart + 1) * P)) || (rc = dalloc(c, &c->gm_nrmb, (size_t)P)) ||
-            (rc = dalloc(c, &c->gm_state, (size_t)P)) || (rc = dalloc(c, &c->gm_its, (size_t)P)) ||
-            (rc = dalloc(c, &c->gm_jc, (size_t)P)))
-            return rc;
-        c->seg_restart = restart;
-        c->seg_hP = P;
-    }
     const long long n = nvec(c);
     const int g = sms(c->device) * 4;
-    const bool prec = precond == 2;
-    // classical Gram-Schmidt with one reorthogonalisation (CGS2): 5 launches per
-    // Arnoldi step instead of j + 3 for modified Gram-Schmidt.  It wins while
-    // the steps are launch-bound, for small systems (measured on B200: 2D p=2,
-    // 37k unknowns, 9.1 -> 5.9 ms per 62 steps); for larger ones the fused MGS
-    // steps, which move the same bytes with more memory parallelism, win (3D
-    // p=3, 2.5M unknowns: 33 ms with MGS, 75 ms with CGS2 per 69 steps; batches
-    // of 2D requests, 0.3-2M unknowns, were slower with CGS2 too).
-    const bool cgs2 = restart + 1 <= 64 && n <= (1ll << 17);
-    if (hist && hist_len > 0 && c->gm_hist_n < (size_t)hist_len) {
+    if (precond == 0) {
+        if (!c->have_order && (rc = compute_ordering(c))) return rc;
+        if ((rc = bilu0_factor(c))) return rc;
+        return bilu0_apply(c, c->Rg, c->pb);
+    }
+    if (precond == -1) {
+        CK(cudaMemcpyAsync(c->pb, c->Rg, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
+        return 0;
+    }
+    if ((rc = bj_factor(c))) return rc;
+    std::vector<int> bi(c->dims.nf);
+    CK(cudaMemcpyAsync(bi.data(), c->binfo, sizeof(int) * bi.size(), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    for (int i = 0; i < c->dims.nf; i++)
+        if (bi[i]) return fail(c, HFEM_E_SINGULAR, "diagonal block of face %d is singular", i);
+    if (c->precision >= 1) {
+        const long long nm = (long long)c->dims.nf * c->bsz * c->bsz;
+        if (!c->Minv32 && (rc = dalloc(c, &c->Minv32, (size_t)nm))) return rc;
+        to_float_kernel<<<g, 256, 0, c->stream>>>(nm, c->Minv, c->Minv32);
+        bj_apply_kernel<float><<<g, 256, 0, c->stream>>>(c->dims.nf, c->bsz, c->Minv32, c->Rg, c->pb);
+    } else {
+        bj_apply_kernel<double><<<g, 256, 0, c->stream>>>(c->dims.nf, c->bsz, c->Minv, c->Rg, c->pb);
+    }
+    return check_launch(c, "bj_apply");
+}
+
+// One Arnoldi step's three kernels and the cycle's start and end, for pieces of
+// R entries per thread.
+template <int R>
+struct SegRun {
+    static void start(hfem_ctx* c, const SegPieces& P, const GmState& S, bool first) {
+        seg_start_kernel<R><<<P.npieces, SEG_THREADS, 0, c->stream>>>(P, S, first, c->pb, c->V);
+    }
+    static void step(hfem_ctx* c, const SegPieces& P, const GmState& S, long long n, int j) {
+        double* w = c->V + (size_t)(j + 1) * n;
+        const size_t ld = (size_t)(S.restart + 1) * S.P;
+        double *h1 = c->gm_h, *c1 = h1 + ld, *h2 = c1 + ld, *c2 = h2 + ld;
+        seg_project_kernel<R, false><<<P.npieces, SEG_THREADS, 0, c->stream>>>(P, n, j + 1, S.P, c->V, w, nullptr, S.sc,
+                                                                               h1, c1);
+        seg_project_kernel<R, true><<<P.npieces, SEG_THREADS, 0, c->stream>>>(P, n, j + 1, S.P, c->V, w, c1, S.sc, h2,
+                                                                              c2);
+        seg_finish_step_kernel<R><<<P.npieces, SEG_THREADS, 0, c->stream>>>(P, S, n, j, c->V, w, c2, h1, h2);
+    }
+    static void end(hfem_ctx* c, const SegPieces& P, const GmState& S, long long n) {
+        gm_solve_kernel<<<S.P, 32, 0, c->stream>>>(S, c->gm_y, c->gm_k);
+        seg_combine_kernel<R><<<P.npieces, SEG_THREADS, 0, c->stream>>>(P, n, c->gm_k, S.restart, c->V, c->gm_y, c->x);
+    }
+};
+struct SegLaunch {
+    void (*start)(hfem_ctx*, const SegPieces&, const GmState&, bool);
+    void (*step)(hfem_ctx*, const SegPieces&, const GmState&, long long, int);
+    void (*end)(hfem_ctx*, const SegPieces&, const GmState&, long long);
+};
+SegLaunch seg_launch(int rows) {
+    switch (rows) {
+        case 1: return {SegRun<1>::start, SegRun<1>::step, SegRun<1>::end};
+        case 2: return {SegRun<2>::start, SegRun<2>::step, SegRun<2>::end};
+        case 4: return {SegRun<4>::start, SegRun<4>::step, SegRun<4>::end};
+        default: return {SegRun<8>::start, SegRun<8>::step, SegRun<8>::end};
+    }
+}
+
+// Restarted, left-preconditioned GMRES run for every segment at once
+// (kernel/gmres_bilu0.m:17-105 per problem): the whole system as one problem
+// (`map` false), or every problem of the context's problem map.  Each problem
+// has its own Krylov basis (its segment of the vectors), Hessenberg matrix,
+// Givens rotations and stopping test, so it takes exactly the iterations it
+// takes alone; the launches are shared, and a problem that has stopped is
+// skipped by every kernel.  Orthogonalisation: classical Gram-Schmidt applied
+// twice (krylov_seg.cuh).
+int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int maxit, int* conv, int* iters,
+               double* hist, int hist_len) {
+    int rc;
+    if (!c->assembled) return fail(c, HFEM_E_STATE, "assemble before gmres");
+    SegTab& T = map ? c->seg_map : c->seg_one;
+    if (map && !T.npieces)
+        return fail(c, HFEM_E_STATE, "per-problem GMRES needs a problem map with each problem's faces contiguous");
+    if (restart < 1 || maxit < 1 || !(tol > 0.0)) return fail(c, HFEM_E_ARG, "restart, maxit and tol must be positive");
+    if (map && precond != -1 && precond != 2)
+        return fail(c, HFEM_E_ARG, "precond must be -1 (none) or 2 (block Jacobi)");
+    if (precond != -1 && precond != 0 && precond != 2)
+        return fail(c, HFEM_E_ARG, "precond must be -1 (none), 0 (BILU0) or 2 (block Jacobi)");
+    const long long n = nvec(c);
+    if (!map && !T.npieces && (rc = build_segments(c, T, {n}))) return rc;
+    if ((rc = ensure_krylov(c, restart))) return rc;
+    const int P = T.nseg;
+    const unsigned char* mv_act = map ? c->gm_act : nullptr;   // row -> problem only with a problem map
+    if (c->gm_restart < restart || c->gm_P < P) {
+        const size_t r1 = (size_t)std::max(restart, c->gm_restart) + 1, PP = (size_t)std::max(P, c->gm_P);
+        if ((rc = dalloc(c, &c->gm_h, 4 * r1 * PP)) || (rc = dalloc(c, &c->gm_y, r1 * PP)) ||
+            (rc = dalloc(c, &c->gm_H, r1 * r1 * PP)) || (rc = dalloc(c, &c->gm_cs, r1 * PP)) ||
+            (rc = dalloc(c, &c->gm_sn, r1 * PP)) || (rc = dalloc(c, &c->gm_g, r1 * PP)) ||
+            (rc = dalloc(c, &c->gm_sc, r1 * PP)) || (rc = dalloc(c, &c->gm_nrmb, PP)) ||
+            (rc = dalloc(c, &c->gm_state, PP)) || (rc = dalloc(c, &c->gm_its, PP)) ||
+            (rc = dalloc(c, &c->gm_jc, PP)) || (rc = dalloc(c, &c->gm_k, PP)) || (rc = dalloc(c, &c->gm_act, PP)))
+            return rc;
+        c->gm_restart = (int)r1 - 1;
+        c->gm_P = (int)PP;
+        mv_act = map ? c->gm_act : nullptr;
+    }
+    if (T.part_n < (size_t)T.npieces * (restart + 1)) {
+        T.part_n = 0;
+        if ((rc = dalloc(c, &T.part, (size_t)T.npieces * (restart + 1)))) return rc;
+        T.part_n = (size_t)T.npieces * (restart + 1);
+    }
+    const bool want_hist = hist && hist_len > 0;
+    if (want_hist && c->gm_hist_n < (size_t)hist_len) {
+        c->gm_hist_n = 0;
         if ((rc = dalloc(c, &c->gm_hist, (size_t)hist_len))) return rc;
         c->gm_hist_n = (size_t)hist_len;
     }
-    if (cgs2 && c->seg_partk_n < (size_t)c->npieces * (restart + 1)) {
-        if ((rc = dalloc(c, &c->seg_partk, (size_t)c->npieces * (restart + 1)))) return rc;
-        c->seg_partk_n = (size_t)c->npieces * (restart + 1);
-    }
-    if (prec) {
-        if ((rc = bj_factor(c))) return rc;
-        std::vector<int> bi(c->dims.nf);
-        CK(cudaMemcpyAsync(bi.data(), c->binfo, sizeof(int) * bi.size(), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        for (int i = 0; i < c->dims.nf; i++)
-            if (bi[i]) return fail(c, HFEM_E_SINGULAR, "diagonal block of face %d is singular", i);
-        if (c->precision >= 1) {
-            const long long nm = (long long)c->dims.nf * c->bsz * c->bsz;
-            if (!c->Minv32 && (rc = dalloc(c, &c->Minv32, (size_t)nm))) return rc;
-            to_float_kernel<<<g, 256, 0, c->stream>>>(nm, c->Minv, c->Minv32);
-            bj_apply_kernel<float><<<g, 256, 0, c->stream>>>(c->dims.nf, c->bsz, c->Minv32, c->Rg, c->pb);
-        } else {
-            bj_apply_kernel<double><<<g, 256, 0, c->stream>>>(c->dims.nf, c->bsz, c->Minv, c->Rg, c->pb);
-        }
-    } else {
-        CK(cudaMemcpyAsync(c->pb, c->Rg, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-    }
+    const bool prec = precond == 2;
+    if ((rc = prepare_preconditioner(c, precond))) return rc;
     CK(cudaMemsetAsync(c->x, 0, sizeof(double) * n, c->stream));
-    const SegPieces SP{c->npieces, c->seg_pstart, c->seg_pseg, c->seg_p0, c->seg_ticket, c->seg_part, c->seg_act};
-    const int np = c->npieces;
-    double* d_h = c->seg_h;                   // Hessenberg column, entry (i, p) at i * P + p
-    double* d_h2 = c->seg_h + (size_t)(restart + 2) * P;   // CGS2's second projection, same layout
+    const SegPieces SP{T.npieces, T.pstart, T.pseg, T.p0, T.ticket, T.part, c->gm_act};
+    const GmState GS{P, restart, maxit, tol, c->gm_H, c->gm_cs, c->gm_sn, c->gm_g, c->gm_nrmb, c->gm_sc, c->gm_state,
+                     c->gm_its, c->gm_jc, c->gm_act, want_hist ? c->gm_hist : nullptr, want_hist ? hist_len : 0};
+    const SegLaunch run = seg_launch(T.rows);
+    // out = xsc M^-1 Hg x
+    auto op = [&](const double* x, double* out, const double* xsc) -> int {
+        if (precond != 0) return matvec(c, x, out, prec, xsc, mv_act);
+        int r = matvec(c, x, c->bl_t, false, xsc, mv_act);
+        return r ? r : bilu0_apply(c, c->bl_t, out);
+    };
     // the Givens rotations, residual estimates and stopping tests run on the
-    // device (gm_* kernels, one thread per problem); the host reads the
-    // problems' masks back only every GM_CHECK steps and at the start of a
-    // cycle, so the Arnoldi steps are enqueued without a round trip each
-    constexpr int GM_CHECK = 8;
-    const GmState GS{P, restart, maxit, tol, c->gm_H, c->gm_cs, c->gm_sn, c->gm_g, c->gm_nrmb, c->gm_state,
-                     c->gm_its, c->gm_jc, c->seg_act, (hist && hist_len > 0) ? c->gm_hist : nullptr,
-                     (hist && hist_len > 0) ? hist_len : 0};
-    const int gb = (P + 127) / 128;
-    std::vector<unsigned char> act(P, 1);
-    auto set_act = [&]() -> int {
-        CK(cudaMemcpyAsync(c->seg_act, act.data(), P, cudaMemcpyHostToDevice, c->stream));
-        return 0;
-    };
-    auto any_active = [&](bool& live) -> int {
-        CK(cudaMemcpyAsync(act.data(), c->seg_act, P, cudaMemcpyDeviceToHost, c->stream));
+    // device; the host reads the problems' states back only every GM_CHECK
+    // steps and at the end of a cycle, so the Arnoldi steps are enqueued without
+    // a round trip each
+    const int GM_CHECK = precond == 0 ? 1 : 8;  // a BILU0 apply costs more than the read
+    std::vector<int> state(P, 2);
+    auto any_running = [&](bool& live) -> int {
+        CK(cudaMemcpyAsync(state.data(), c->gm_state, sizeof(int) * P, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
-        live = false;
-        for (int p = 0; p < P; p++) live = live || act[p];
+        live = std::find(state.begin(), state.end(), 2) != state.end();
         return 0;
     };
-    auto axpy_dot = [&](const double* hprev, const double* vprev, double* w, const double* b, double* out, int sq) {
-        seg_axpy_dot_kernel<<<np, SEG_THREADS, 0, c->stream>>>(SP, hprev, vprev, w, b, out, sq);
-    };
-    if ((rc = set_act())) return rc;
-    axpy_dot(nullptr, nullptr, c->pb, c->pb, c->seg_nrm, 1);
-    gm_init_kernel<<<gb, 128, 0, c->stream>>>(GS, c->seg_nrm);
-    while (true) {
-        // r = M^-1 b - M^-1 A x, beta = |r| per problem, on the problems still running
-        gm_running_kernel<<<gb, 128, 0, c->stream>>>(GS);
-        if ((rc = matvec_warp(c, c->x, c->w, prec, mv_act))) return rc;
-        seg_sub_from_kernel<<<np, SEG_THREADS, 0, c->stream>>>(SP, c->pb, c->w);
-        axpy_dot(nullptr, nullptr, c->w, c->w, c->seg_nrm, 1);
-        gm_cycle_kernel<<<gb, 128, 0, c->stream>>>(GS, c->seg_nrm);
-        bool live = false;
-        if ((rc = any_active(live))) return rc;
-        if (!live) break;
-        seg_scale_kernel<<<np, SEG_THREADS, 0, c->stream>>>(SP, c->seg_nrm, c->w, c->V);
+    bool live = true;
+    for (bool first = true; live; first = false) {
+        // V_0 = M^-1 b - M^-1 A x (x = 0 in the first cycle), beta = |V_0|
+        if (!first && (rc = op(c->x, c->V, nullptr))) return rc;
+        run.start(c, SP, GS, first);
         for (int j = 0; j < restart && live; j++) {
-            double* vj = c->V + (size_t)j * n;
-            double* vn = c->V + (size_t)(j + 1) * n;
-            if ((rc = matvec_warp(c, vj, vn, prec, mv_act))) return rc;
+            if ((rc = op(c->V + (size_t)j * n, c->V + (size_t)(j + 1) * n, c->gm_sc + (size_t)j * P))) return rc;
             {
-                Timed t(c, "orthogonalise_seg");
-                if (cgs2) {
-                    const int k = j + 1;
-                    seg_multidot_kernel<<<np, SEG_THREADS, 0, c->stream>>>(SP, n, k, P, c->V, vn, c->seg_partk, d_h);
-                    seg_update_kernel<<<np, SEG_THREADS, 0, c->stream>>>(SP, n, k, P, c->V, d_h, vn, nullptr);
-                    seg_multidot_kernel<<<np, SEG_THREADS, 0, c->stream>>>(SP, n, k, P, c->V, vn, c->seg_partk,
-                                                                           d_h2);
-                    seg_update_kernel<<<np, SEG_THREADS, 0, c->stream>>>(SP, n, k, P, c->V, d_h2, vn,
-                                                                         d_h + (size_t)(j + 1) * P);
-                } else {
-                    for (int i = 0; i <= j; i++)
-                        axpy_dot(i ? d_h + (size_t)(i - 1) * P : nullptr, i ? c->V + (size_t)(i - 1) * n : nullptr,
-                                 vn, c->V + (size_t)i * n, d_h + (size_t)i * P, 0);
-                    axpy_dot(d_h + (size_t)j * P, vj, vn, vn, d_h + (size_t)(j + 1) * P, 1);
-                }
-                seg_scale_kernel<<<np, SEG_THREADS, 0, c->stream>>>(SP, d_h + (size_t)(j + 1) * P, vn, vn);
+                Timed t(c, "orthogonalise");
+                run.step(c, SP, GS, n, j);
             }
-            gm_givens_kernel<<<gb, 128, 0, c->stream>>>(GS, j, d_h, cgs2 ? d_h2 : nullptr);
             if ((rc = check_launch(c, "arnoldi"))) return rc;
-            if ((j + 1) % GM_CHECK == 0 && j + 1 < restart && (rc = any_active(live))) return rc;
+            if (((j + 1) % GM_CHECK == 0 || j + 1 == restart) && (rc = any_running(live))) return rc;
         }
         // x += V y for every problem that took part in this cycle
-        gm_solve_kernel<<<gb, 128, 0, c->stream>>>(GS, c->seg_y, c->seg_k);
-        seg_combine_kernel<<<np, SEG_THREADS, 0, c->stream>>>(SP, n, c->seg_k, restart, c->V, c->seg_y, c->x);
-        if ((rc = check_launch(c, "combine_seg"))) return rc;
+        run.end(c, SP, GS, n);
+        if ((rc = check_launch(c, "combine"))) return rc;
     }
-    std::vector<int> state(P), its(P);
-    CK(cudaMemcpyAsync(state.data(), c->gm_state, sizeof(int) * P, cudaMemcpyDeviceToHost, c->stream));
+    std::vector<int> its(P);
     CK(cudaMemcpyAsync(its.data(), c->gm_its, sizeof(int) * P, cudaMemcpyDeviceToHost, c->stream));
-    if (hist && hist_len > 0)
-        CK(cudaMemcpyAsync(hist, c->gm_hist, sizeof(double) * hist_len, cudaMemcpyDeviceToHost, c->stream));
+    if (want_hist) CK(cudaMemcpyAsync(hist, c->gm_hist, sizeof(double) * hist_len, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     flush_timer(c);
     for (int p = 0; p < P; p++) {
@@ -1599,9 +1489,10 @@ int hfem_destroy(hfem_ctx* c) {
     void* ptrs[] = {c->shapvt, c->shapvg, c->svsv, c->shapft, c->shapfg, c->sfsf, c->perm, c->dgnodes, c->elcon,
                     c->rowstart, c->colidx, c->blk_src, c->face_src, c->rowface, c->colface, c->udg, c->uh, c->sh,
                     c->D, c->F, c->K, c->H, c->Ru, c->DinvRu, c->Rh, c->Ro, c->ru2, c->Hg, c->Rg, c->Rr, c->rnorm, c->ws, c->DinvF,
-                    c->info, c->Minv, c->V, c->w, c->x, c->pb, c->scal, c->part, c->binfo, c->udgi,
-                    c->eprob, c->fprob, c->pparam, c->palpha, c->seg_pstart, c->seg_pseg, c->seg_p0,
-                    c->seg_ticket, c->seg_part, c->seg_partk, c->seg_h, c->seg_y, c->seg_nrm, c->seg_act, c->seg_k, c->tc_err, c->rn_part, c->bf, c->bcm, c->bcs, c->Minv32,
+                    c->info, c->Minv, c->V, c->w, c->x, c->pb, c->binfo, c->udgi,
+                    c->eprob, c->fprob, c->pparam, c->palpha, c->seg_one.pstart, c->seg_one.pseg, c->seg_one.p0,
+                    c->seg_one.ticket, c->seg_one.part, c->seg_map.pstart, c->seg_map.pseg, c->seg_map.p0,
+                    c->seg_map.ticket, c->seg_map.part, c->gm_sc, c->gm_h, c->gm_y, c->gm_k, c->gm_act, c->tc_err, c->rn_part, c->bf, c->bcm, c->bcs, c->Minv32,
                     c->d_u2o, c->d_rows_lo, c->d_rows_up, c->d_fptr, c->d_fpos, c->Mg, c->bl_t, c->bl_y,
                     c->d_lvl_lo, c->d_lvl_up, c->Mg32, c->d_frec, c->d_lrec, c->d_urec, c->gm_H, c->gm_cs, c->gm_sn, c->gm_g, c->gm_nrmb, c->gm_hist,
                     c->gm_state, c->gm_its, c->gm_jc};
@@ -1889,7 +1780,7 @@ int hfem_residual(hfem_ctx* c, double* rnorm) { return run_assembly(c, false, rn
 int hfem_gmres(hfem_ctx* c, int precond, int restart, double tol, int maxit, int* conv, int* iters, double* hist,
                int hist_len) {
     if (!c) return HFEM_E_ARG;
-    return gmres_impl(c, precond, restart, tol, maxit, conv, iters, hist, hist_len);
+    return gmres_impl(c, false, precond, restart, tol, maxit, conv, iters, hist, hist_len);
 }
 
 int hfem_update(hfem_ctx* c, double alpha) {
@@ -1916,7 +1807,7 @@ int hfem_newton(hfem_ctx* c, double newton_tol, int newton_maxiter, int precond,
         if (std::isnan(oldNorm) || std::isinf(oldNorm))
             return fail(c, HFEM_E_SINGULAR, "residual norm of Newton iterate %d is NaN or Inf", iter);
         int conv = 0, its = 0;
-        if ((rc = gmres_impl(c, precond, restart, gmres_tol, gmres_maxit, &conv, &its, nullptr, 0))) return rc;
+        if ((rc = gmres_impl(c, false, precond, restart, gmres_tol, gmres_maxit, &conv, &its, nullptr, 0))) return rc;
         if (conv == -1) break;
         if (iter == 1 && oldNorm < newton_tol) {
             rNorm = oldNorm;
@@ -2022,45 +1913,16 @@ int hfem_set_problem_map(hfem_ctx* c, int nprob, const int* eprob, const int* fp
         return rc;
     // Krylov segments (hfem_gmres_problems): when fprob is non-decreasing and
     // every problem owns a face, problem p's slice of the trace vector is one
-    // contiguous segment, cut into pieces of <= SEG_PIECE entries.
-    c->npieces = 0;
-    c->seg_single = false;
+    // contiguous segment.
+    c->seg_map.npieces = 0;
     bool sorted = true;
-    std::vector<int> fcount(nprob, 0);
+    std::vector<long long> count(nprob, 0);
     for (int f = 0; f < d.nf; f++) {
-        fcount[fprob[f]]++;
+        count[fprob[f]] += c->bsz;
         if (f && fprob[f] < fprob[f - 1]) sorted = false;
     }
-    for (int p = 0; p < nprob; p++) sorted = sorted && fcount[p] > 0;
-    if (sorted) {
-        // piece length: a power of two in [1024, SEG_PIECE] giving about 4 CTAs per SM
-        const long long ntot = (long long)d.nf * c->bsz;
-        long long piece = 1024;
-        while (piece < SEG_PIECE && piece * 4 * sms(c->device) < ntot) piece *= 2;
-        std::vector<long long> pstart;
-        std::vector<int> pseg, p0(nprob + 1);
-        long long a = 0;
-        for (int p = 0; p < nprob; p++) {
-            p0[p] = (int)pseg.size();
-            const long long b = a + (long long)fcount[p] * c->bsz;
-            for (long long s = a; s < b; s += piece) {
-                pstart.push_back(s);
-                pseg.push_back(p);
-            }
-            a = b;
-        }
-        p0[nprob] = (int)pseg.size();
-        pstart.push_back(a);
-        c->npieces = (int)pseg.size();
-        if ((rc = upload(c, &c->seg_pstart, pstart.data(), pstart.size())) ||
-            (rc = upload(c, &c->seg_pseg, pseg.data(), pseg.size())) ||
-            (rc = upload(c, &c->seg_p0, p0.data(), p0.size())) || (rc = dalloc(c, &c->seg_ticket, (size_t)nprob)) ||
-            (rc = dalloc(c, &c->seg_part, pseg.size())) || (rc = dalloc(c, &c->seg_nrm, (size_t)2 * nprob)) ||
-            (rc = dalloc(c, &c->seg_act, (size_t)nprob)) || (rc = dalloc(c, &c->seg_k, (size_t)nprob)))
-            return rc;
-        CK(cudaMemsetAsync(c->seg_ticket, 0, sizeof(int) * nprob, c->stream));
-        c->seg_restart = 0;
-    }
+    for (int p = 0; p < nprob; p++) sorted = sorted && count[p] > 0;
+    if (sorted && (rc = build_segments(c, c->seg_map, count))) return rc;
     CK(cudaStreamSynchronize(c->stream));
     c->nprob = nprob;
     return 0;
@@ -2275,7 +2137,7 @@ int hfem_matvec(hfem_ctx* c, const double* x, double* y) {
     if (!c || !x || !y) return HFEM_E_ARG;
     if (!c->assembled) return fail(c, HFEM_E_STATE, "assemble before a matvec");
     CK(cudaSetDevice(c->device));
-    int rc = matvec_warp(c, x, y, false, nullptr);
+    int rc = matvec(c, x, y, false, nullptr, nullptr);
     if (rc) return rc;
     CK(cudaStreamSynchronize(c->stream));
     return 0;
@@ -2325,7 +2187,7 @@ int hfem_set_precision(hfem_ctx* c, int mode) {
 
 int hfem_gmres_problems(hfem_ctx* c, int precond, int restart, double tol, int maxit, int* conv, int* iters) {
     if (!c) return HFEM_E_ARG;
-    return gmres_seg_impl(c, precond, restart, tol, maxit, conv, iters);
+    return gmres_impl(c, true, precond, restart, tol, maxit, conv, iters, nullptr, 0);
 }
 
 int device_buffer(hfem_ctx* c, int what, const double** src, size_t* need) {
