@@ -1,6 +1,6 @@
 // Shared pieces of the HDG element kernels for sm_100a: element shapes and
 // arguments, geometry and q-equation matrices, the Cholesky helpers, the
-// face-block scatter, the residual norm, q recovery and the solution update.
+// face-block scatter, q recovery and the solution update.
 // The element assembly itself is element_kernel (elem_kernel.cuh).
 //
 // Structure of the element blocks (restating elementassembly.cpp faceint
@@ -296,33 +296,6 @@ static __global__ void scatter_R_kernel(ScatterArgs A) {
         }
         if (A.Rg) A.Rg[t] = s;
         if (A.Rr) A.Rr[t] = so;
-    }
-}
-
-// Partial sums of ru2 and Rr^2 per CTA (fixed grid-stride order).
-static __global__ void rnorm_partial_kernel(int ne, const double* __restrict__ ru2, long long nr,
-                                     const double* __restrict__ rr, double* __restrict__ part) {
-    __shared__ double red[32];
-    double s = 0.0;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ne; i += stride) s += ru2[i];
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nr; i += stride) s += rr[i] * rr[i];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-        part[blockIdx.x] = t;
-    }
-}
-
-// out = sqrt(sum of the n partial sums), in order.
-static __global__ void rnorm_final_kernel(int n, const double* __restrict__ part, double* out) {
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int i = 0; i < n; i++) t += part[i];
-        *out = sqrt(t);
     }
 }
 

@@ -23,6 +23,7 @@
 #include "krylov_seg.cuh"
 #include "schur_kernels.cuh"
 #include "launch.cuh"
+#include "norms.cuh"
 #include "lift.cuh"
 #include "bilu0.cuh"
 #include "inverse_blocked.cuh"
@@ -30,8 +31,6 @@
 using namespace hfem;
 
 namespace {
-
-constexpr int RNORM_CTAS = 296;
 
 struct KernelTimer {
     bool on = false;
@@ -104,7 +103,9 @@ struct hfem_ctx {
     int conv_stab = 0;          // app.convStabMethod: 0 constant tau, 1 Lax-Friedrichs, 2 Roe
     int visc_model = 0;         // app.viscosityModel: 0 constant, 1 Sutherland's law
     int* tc_err = nullptr;              // 1: a tcgen05 MMA wait expired; 2: an element bulk-copy wait expired
-    double* rn_part = nullptr;
+    NormPart* rn_part = nullptr;
+    int* rn_ticket = nullptr;
+    PassStatus* status = nullptr;       // outcome of the last pass
     // master tables
     double *shapvt = nullptr, *shapvg = nullptr, *svsv = nullptr, *shapft = nullptr, *shapfg = nullptr, *sfsf = nullptr;
     int* perm = nullptr;
@@ -123,7 +124,7 @@ struct hfem_ctx {
     double *D = nullptr, *F = nullptr, *K = nullptr, *H = nullptr, *Ru = nullptr, *Rh = nullptr, *Ro = nullptr;
     double* DinvRu = nullptr;           // D^-1 Ru of the last matrix pass (the update's input)
     double* DinvF = nullptr;
-    double *ru2 = nullptr, *Hg = nullptr, *Rg = nullptr, *Rr = nullptr, *rnorm = nullptr, *ws = nullptr;
+    double *ru2 = nullptr, *Hg = nullptr, *Rg = nullptr, *Rr = nullptr, *ws = nullptr;
     int* info = nullptr;
     // Krylov
     double *Minv = nullptr, *V = nullptr, *w = nullptr, *x = nullptr, *pb = nullptr;
@@ -136,6 +137,8 @@ struct hfem_ctx {
     bool palpha_on = false;
     int *eprob = nullptr, *fprob = nullptr;
     double *pparam = nullptr, *palpha = nullptr;
+    int *pn_range = nullptr, *pn_ticket = nullptr;      // per-problem norms (ProblemNormArgs)
+    double *pn_part = nullptr, *pn_out = nullptr;
     // Krylov segments: the whole trace vector as one segment, and one segment
     // per problem (set_problem_map, when each problem's faces are contiguous)
     SegTab seg_one, seg_map;
@@ -387,8 +390,10 @@ int ensure_assembly_buffers(hfem_ctx* c) {
     if ((rc = dalloc(c, &c->info, ne))) return rc;
     if ((rc = dalloc(c, &c->ws, (size_t)c->grid_elem * c->L->ws))) return rc;
     if ((rc = dalloc(c, &c->tc_err, 1))) return rc;
-    if ((rc = dalloc(c, &c->rn_part, RNORM_CTAS))) return rc;
+    if ((rc = dalloc(c, &c->rn_part, NORM_CTAS))) return rc;
+    if ((rc = dalloc(c, &c->rn_ticket, 1))) return rc;
     CK(cudaMemsetAsync(c->tc_err, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->rn_ticket, 0, sizeof(int), c->stream));
     return 0;
 }
 
@@ -547,33 +552,27 @@ int enqueue_assembly(hfem_ctx* c, bool matrix) {
         scatter_R_kernel<<<sms(c->device) * 4, 256, 0, c->stream>>>(sa);
         if ((rc = check_launch(c, "scatter_R"))) return rc;
     }
-    rnorm_partial_kernel<<<RNORM_CTAS, 256, 0, c->stream>>>(c->dims.ne, c->ru2, (long long)c->dims.nf * c->bsz,
-                                                            c->Rr, c->rn_part);
-    rnorm_final_kernel<<<1, 32, 0, c->stream>>>(RNORM_CTAS, c->rn_part, c->rnorm);
-    return check_launch(c, "rnorm");
+    const long long nr = (long long)c->dims.nf * c->bsz;
+    const long long want = (std::max<long long>(nr, c->dims.ne) + 4 * NORM_THREADS - 1) / (4 * NORM_THREADS);
+    pass_status_kernel<<<(int)std::min<long long>(NORM_CTAS, want), NORM_THREADS, 0, c->stream>>>(
+        NormArgs{c->dims.ne, nr, c->ru2, c->Rr, matrix ? c->info : nullptr, c->tc_err, c->rn_part, c->rn_ticket,
+                 c->status});
+    return check_launch(c, "pass_status");
 }
 
 // Wait for an enqueued assembly, check the element LUs (and the tensor-core
 // kernel) and read the residual norm.
 int finish_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
-    if (matrix) {
-        std::vector<int> info(c->dims.ne);
-        CK(cudaMemcpyAsync(info.data(), c->info, sizeof(int) * info.size(), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        for (int e = 0; e < c->dims.ne; e++)
-            if (info[e]) return fail(c, HFEM_E_SINGULAR, "element %d: singular local matrix (pivot %d)", e, info[e]);
-    }
-    int terr = 0;
-    CK(cudaMemcpyAsync(&terr, c->tc_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    PassStatus st;
+    CK(cudaMemcpyAsync(&st, c->status, sizeof st, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    if (terr == 1) return fail(c, HFEM_E_CUDA, "tensor-core Schur kernel: an MMA completion wait expired");
-    if (terr == 2) return fail(c, HFEM_E_CUDA, "element kernel: a bulk-copy completion wait expired");
+    if (matrix && st.bad_elem >= 0)
+        return fail(c, HFEM_E_SINGULAR, "element %d: singular local matrix (pivot %d)", st.bad_elem, st.bad_pivot);
+    if (st.wait_err == 1) return fail(c, HFEM_E_CUDA, "tensor-core Schur kernel: an MMA completion wait expired");
+    if (st.wait_err == 2) return fail(c, HFEM_E_CUDA, "element kernel: a bulk-copy completion wait expired");
     if (matrix) c->assembled = true;
-    double rn = 0.0;
-    CK(cudaMemcpyAsync(&rn, c->rnorm, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
     flush_timer(c);
-    if (rnorm_out) *rnorm_out = rn;
+    if (rnorm_out) *rnorm_out = st.rnorm;
     return 0;
 }
 
@@ -1467,7 +1466,7 @@ int hfem_create(const hfem_dims* dims, int device, hfem_ctx** out) {
     cudaFuncSetAttribute(L.inv_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.inv_smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.inv_fn, L.inv_threads, L.inv_smem);
     c->grid_inv = std::max(1, std::min(d.ne, sms(device) * std::max(occ, 1)));
-    if (pool_alloc(device, (void**)&c->rnorm, sizeof(double)) != cudaSuccess) {
+    if (pool_alloc(device, (void**)&c->status, sizeof(PassStatus)) != cudaSuccess) {
         cudaStreamDestroy(c->own);
         delete c;
         return HFEM_E_NOMEM;
@@ -1488,11 +1487,11 @@ int hfem_destroy(hfem_ctx* c) {
     cudaStreamSynchronize(c->stream);
     void* ptrs[] = {c->shapvt, c->shapvg, c->svsv, c->shapft, c->shapfg, c->sfsf, c->perm, c->dgnodes, c->elcon,
                     c->rowstart, c->colidx, c->blk_src, c->face_src, c->rowface, c->colface, c->udg, c->uh, c->sh,
-                    c->D, c->F, c->K, c->H, c->Ru, c->DinvRu, c->Rh, c->Ro, c->ru2, c->Hg, c->Rg, c->Rr, c->rnorm, c->ws, c->DinvF,
+                    c->D, c->F, c->K, c->H, c->Ru, c->DinvRu, c->Rh, c->Ro, c->ru2, c->Hg, c->Rg, c->Rr, c->status, c->ws, c->DinvF,
                     c->info, c->Minv, c->V, c->w, c->x, c->pb, c->binfo, c->udgi,
                     c->eprob, c->fprob, c->pparam, c->palpha, c->seg_one.pstart, c->seg_one.pseg, c->seg_one.p0,
                     c->seg_one.ticket, c->seg_one.part, c->seg_map.pstart, c->seg_map.pseg, c->seg_map.p0,
-                    c->seg_map.ticket, c->seg_map.part, c->gm_sc, c->gm_h, c->gm_y, c->gm_k, c->gm_act, c->tc_err, c->rn_part, c->bf, c->bcm, c->bcs, c->Minv32,
+                    c->seg_map.ticket, c->seg_map.part, c->gm_sc, c->gm_h, c->gm_y, c->gm_k, c->gm_act, c->tc_err, c->rn_part, c->rn_ticket, c->pn_range, c->pn_ticket, c->pn_part, c->pn_out, c->bf, c->bcm, c->bcs, c->Minv32,
                     c->d_u2o, c->d_rows_lo, c->d_rows_up, c->d_fptr, c->d_fpos, c->Mg, c->bl_t, c->bl_y,
                     c->d_lvl_lo, c->d_lvl_up, c->Mg32, c->d_frec, c->d_lrec, c->d_urec, c->gm_H, c->gm_cs, c->gm_sn, c->gm_g, c->gm_nrmb, c->gm_hist,
                     c->gm_state, c->gm_its, c->gm_jc};
@@ -1923,6 +1922,21 @@ int hfem_set_problem_map(hfem_ctx* c, int nprob, const int* eprob, const int* fp
     }
     for (int p = 0; p < nprob; p++) sorted = sorted && count[p] > 0;
     if (sorted && (rc = build_segments(c, c->seg_map, count))) return rc;
+    // index range of each problem's elements and faces (per-problem norms)
+    std::vector<int> range(4 * (size_t)nprob, 0);
+    auto ranges = [&](const int* prob, int cnt, int at) {
+        for (int i = cnt - 1; i >= 0; i--) {
+            int* r = &range[4 * (size_t)prob[i] + at];
+            if (r[1] == 0) r[1] = i + 1;
+            r[0] = i;
+        }
+    };
+    ranges(eprob, d.ne, 0);
+    ranges(fprob, d.nf, 2);
+    if ((rc = upload(c, &c->pn_range, range.data(), range.size())) || (rc = dalloc(c, &c->pn_ticket, (size_t)nprob)) ||
+        (rc = dalloc(c, &c->pn_part, (size_t)nprob * NORM_SPLIT)) || (rc = dalloc(c, &c->pn_out, (size_t)nprob)))
+        return rc;
+    CK(cudaMemsetAsync(c->pn_ticket, 0, sizeof(int) * nprob, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->nprob = nprob;
     return 0;
@@ -1933,19 +1947,12 @@ int hfem_set_problem_map(hfem_ctx* c, int nprob, const int* eprob, const int* fp
 int hfem_problem_rnorms(hfem_ctx* c, double* rnorm) {
     if (!c || !rnorm) return HFEM_E_ARG;
     if (!c->nprob || !c->ru2) return fail(c, HFEM_E_STATE, "no problem map or no residual yet");
-    const hfem_dims& d = c->dims;
-    std::vector<double> ru2(d.ne), rr((size_t)d.nf * c->bsz);
-    std::vector<int> ep(d.ne), fp(d.nf);
-    CK(cudaMemcpyAsync(ru2.data(), c->ru2, sizeof(double) * ru2.size(), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(rr.data(), c->Rr, sizeof(double) * rr.size(), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(ep.data(), c->eprob, sizeof(int) * ep.size(), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(fp.data(), c->fprob, sizeof(int) * fp.size(), cudaMemcpyDeviceToHost, c->stream));
+    problem_norm_kernel<<<c->nprob * NORM_SPLIT, NORM_THREADS, 0, c->stream>>>(ProblemNormArgs{
+        c->bsz, c->ru2, c->Rr, c->eprob, c->fprob, c->pn_range, c->pn_part, c->pn_ticket, c->pn_out});
+    int rc = check_launch(c, "problem_norm");
+    if (rc) return rc;
+    CK(cudaMemcpyAsync(rnorm, c->pn_out, sizeof(double) * c->nprob, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    std::vector<double> acc(c->nprob, 0.0);
-    for (int e = 0; e < d.ne; e++) acc[ep[e]] += ru2[e];
-    for (int f = 0; f < d.nf; f++)
-        for (int k = 0; k < c->bsz; k++) acc[fp[f]] += rr[(size_t)f * c->bsz + k] * rr[(size_t)f * c->bsz + k];
-    for (int p = 0; p < c->nprob; p++) rnorm[p] = std::sqrt(acc[p]);
     return 0;
 }
 
