@@ -44,8 +44,12 @@ struct EK {
     static constexpr int KQ3 = ((S::NGV * S::ND + 3) / 4) * 4;        // volume k = (g, d)
     static constexpr int LDBK = ((KFD + 11) / 16) * 16 + 4;        // == 4 (mod 16): conflict-free B fragments
     static constexpr int LDBD = ((KV3 + 11) / 16) * 16 + 4;
+    // the FP64 volume GEMM takes k = (d', g) with g padded to whole k-steps
+    static constexpr int NGP = ((S::NGV + 3) / 4) * 4;
+    static constexpr int KVP = NGP * (S::ND + 1);
+    static constexpr int LDBP = ((KVP + 11) / 16) * 16 + 4;
     static constexpr int BKH = LDBK * (NKP + NHP);                 // one face's B operand
-    static constexpr int BDF = LDBD * (NKP + NHP);                 // the volume B operand
+    static constexpr int BDF = (LDBP > LDBD ? LDBP : LDBD) * (NKP + NHP);   // the volume B operand
     static constexpr int MTV = (S::NPV + 7) / 8;
     static constexpr int MTF = (S::NPF + 7) / 8;
     static constexpr int KV = ((S::NQ + 3) / 4) * 4;               // padded k of shapvg
@@ -71,13 +75,14 @@ struct EK {
     static constexpr int GPH = BDF > BKH + FSLP ? BDF : BKH + FSLP;
     static constexpr int UN = CME + (QPH > GPH ? QPH : GPH);
     // global workspace per CTA slot (doubles): wrl, the interior and boundary
-    // face slices, the boundary flux values, Y
+    // face slices, the boundary flux values, and Y (3xTF32 form only)
     static constexpr int W_WRL = S::NQ * S::NCU * S::NC;
     static constexpr int W_FSL = S::NFE * FSLP;
     static constexpr int W_FNB = S::NA * S::NCH;
     static constexpr int W_Y = S::NPV * S::NGV * S::NCU * S::NC;
-    static constexpr int WS = W_WRL + 2 * W_FSL + W_FNB + W_Y;
-    static_assert(CME % 2 == 0 && BKH % 2 == 0 && W_WRL % 2 == 0 && WS % 2 == 0 && W_FSL % 2 == 0,
+    static constexpr int WS = ((W_WRL + 2 * W_FSL + W_FNB + 1) / 2) * 2;    // FP64 form
+    static constexpr int WS_TF = WS + W_Y;
+    static_assert(CME % 2 == 0 && BKH % 2 == 0 && W_WRL % 2 == 0 && WS_TF % 2 == 0 && W_FSL % 2 == 0,
                   "16-byte alignment of the staged face slices");
     static_assert(O_U % 2 == 0 && O_SHU % 2 == 0, "16-byte alignment of the bulk-copied element inputs");
 };
@@ -165,7 +170,7 @@ struct ElemSmem {
     double Av[EK<S>::LDAV * EK<S>::KV];    // shapvg, zero padded: Av[i + LDAV*q]
     double Af[EK<S>::LDAF * EK<S>::KF];    // shapfg, zero padded: Af[ip + LDAF*q]
     double sfc[S::NGF * S::NPF];           // face basis values shapfc(kk, q) = shapft[q + NGF*kk]
-    double red[NT / 32];
+    double red[S::NT / 32];
     double rdg[S::NPV];                    // 1 / L(j, j) of the Cholesky factor of M
     uint64_t bar_in, bar_sl;               // bulk-copy barriers: element inputs, face slices
     alignas(16) double un[EK<S>::UN];
@@ -179,10 +184,10 @@ struct ElemSmem {
 // / Roe stabilization tensors and Sutherland's law compiled in (the default
 // instantiation holds the constant-tau, constant-viscosity physics only).
 template <class S, bool TF = false, bool GEN = false>
-__global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
+__global__ void __launch_bounds__(S::NT, 512 / S::NT) element_kernel(ElemArgs A) {
     constexpr int ND = S::ND, NPV = S::NPV, NPF = S::NPF, NGV = S::NGV, NGF = S::NGF, NFE = S::NFE;
     constexpr int NCU = S::NCU, NC = S::NC, NCH = S::NCH, NDF = S::NDF, ND1 = S::ND1, N = S::N, NB = S::NB;
-    constexpr int NA = S::NA, NQ = S::NQ;
+    constexpr int NA = S::NA, NQ = S::NQ, NT = S::NT;
     using G = EK<S>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ElemSmem<S>& sm = *reinterpret_cast<ElemSmem<S>*>(smem_raw);
@@ -190,12 +195,12 @@ __global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gr = lane >> 2, gc = lane & 3;
 
-    double* ws = A.ws + (size_t)blockIdx.x * G::WS;
+    double* ws = A.ws + (size_t)blockIdx.x * (TF ? G::WS_TF : G::WS);
     double* wrl = ws;                              // [g + NGV (r + ND1 (j + NCU c))]
     double* fsl = wrl + G::W_WRL;                  // per face: fhat Jacobian slices
     double* fslb = fsl + G::W_FSL;                 // per face: boundary-flux Jacobian slices
     double* fnb = fslb + G::W_FSL;                 // boundary flux [g' + NA j]
-    double* Ys = fnb + G::W_FNB;                   // Y(i,g,j,c) at [g + NGV (c + NC (i + NPV j))]
+    double* Ys = ws + G::WS;                       // 3xTF32 form: Y(i,g,j,c) at [g + NGV (c + NC (i + NPV j))]
 
     // shared union: M^-1 C, M^-1 E, then the phase region
     double* Cm = sm.un;                            // [b + NPV (a + NPV d)]
@@ -274,7 +279,14 @@ __global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
         __syncthreads();
         geometry<S>(T, sm.x, sm.jac, sm.Xx, sm.jacf, sm.nl);
         __syncthreads();
-        qmatrices<S>(T, A.fc_q, sm.jac, sm.Xx, sm.jacf, sm.nl, M, Cm, Em);
+        // the 3xTF32 form keeps the product tables, the dual-number columns and the
+        // dot-product Cholesky: what it rounds to TF32 stays the same bit for bit
+        if constexpr (TF)
+            qmatrices<S>(T, A.fc_q, sm.jac, sm.Xx, sm.jacf, sm.nl, M, Cm, Em);
+        else
+            qmatrices_factored<S, NT>(
+                T, A.fc_q, sm.jac, sm.Xx, sm.jacf, sm.nl, [&](int b, int q) { return sm.Av[b + G::LDAV * q]; },
+                [&](int k, int g) { return sm.Af[k + G::LDAF * g]; }, sm.sfc, sm.perm, M, Cm, Em);
         __syncthreads();
         const double* P = A.pparam ? A.pparam + 8 * A.eprob[e] : A.param;
         const int tdep = A.pparam ? (int)P[6] : A.tdep;
@@ -283,7 +295,8 @@ __global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
         // warp 0 factors M while the other warps evaluate the states at the points
         // and the pointwise fluxes, which do not depend on M
         if (warp == 0) {
-            cholesky_warp<NPV>(M, sm.rdg);
+            if constexpr (TF) cholesky_warp<NPV>(M, sm.rdg);
+            else cholesky_warp_rows<NPV>(M, sm.rdg);
         } else {
             constexpr int NT1 = NT - 32;
             const int tid1 = tid - 32;
@@ -305,8 +318,156 @@ __global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
                 }
             }
             asm volatile("bar.sync 1, %0;" ::"r"(NT1) : "memory");
-            // pointwise fluxes: one work item per (point, differentiated variable k);
-            // a one-derivative dual pass gives f and df/dw_k at that point.
+            // FP64 form: one item per (point, u column) and one per (point, gradient
+            // direction), whose ncu columns share the point's terms.  (3D p=3: 57k cycles
+            // per element with a dual-number pass per column.)
+            if constexpr (!TF) {
+                constexpr int NPT = NGV + NA;
+                const double tau = P[5];
+                for (int t = tid1; t < NPT * (NCU + ND); t += NT1) {
+                    const int p = t % NPT, k = t / NPT;
+                    const bool vol = p < NGV;
+                    const int g = vol ? p : p - NGV, fc = g / NGF, q = g % NGF;
+                    double w[NC];
+#pragma unroll
+                    for (int c = 0; c < NC; c++)
+                        w[c] = vol ? ug[g + NGV * c] : ((c < NCU) ? uhg[g + NA * c] : ugf[g + NA * c]);
+                    const NsPoint<ND> s = ns_point<ND, GEN>(P, w, A.visc_model);
+                    // the metric of the volume point, or the scaled normal of the face point
+                    double X[ND][ND];
+                    if (vol) {
+#pragma unroll
+                        for (int m = 0; m < ND; m++)
+#pragma unroll
+                            for (int d = 0; d < ND; d++) X[m][d] = sm.Xx[g + NGV * (d + ND * m)];
+                    } else {
+#pragma unroll
+                        for (int d = 0; d < ND; d++) X[0][d] = sm.nl[g + NA * d] * sm.jacf[g];
+                    }
+                    double* sl = fsl + fc * G::FSLP;
+                    double f[ND * NCU];
+                    if (k >= NCU) {
+                        const int dq = k - NCU;
+#pragma unroll
+                        for (int m = 0; m < NCU; m++) {
+                            ns_flux_qcol<ND>(P, s, dq, m, f, !A.inviscid);
+                            const int c = NCU * (1 + dq) + m;
+                            // the entries that are zero for every state are not stored for the
+                            // volume (the GEMM skips them), nor is the source row r = 0
+#pragma unroll
+                            for (int j = 0; j < NCU; j++) {
+                                const bool dep = j > 0 && (m <= ND || j == ND + 1);
+                                if (vol) {
+                                    if (!dep) continue;
+#pragma unroll
+                                    for (int r = 0; r < ND; r++) {
+                                        double tt = 0.0;
+#pragma unroll
+                                        for (int d = 0; d < ND; d++) tt = fma(f[d * NCU + j], X[r][d], tt);
+                                        wrl[g + NGV * (r + 1 + ND1 * (j + NCU * c))] = -tt;
+                                    }
+                                } else {
+                                    double dn = 0.0;
+                                    if (dep)
+#pragma unroll
+                                        for (int d = 0; d < ND; d++) dn = fma(f[d * NCU + j], X[0][d], dn);
+                                    sl[q + NGF * (j + NCH * c)] = dn;
+                                }
+                            }
+                        }
+                        continue;
+                    }
+                    if (k == 0) {
+                        ns_flux_value<ND>(P, s, f, !A.inviscid);
+                        if (vol) {
+                            const double jg = sm.jac[g];
+#pragma unroll
+                            for (int j = 0; j < NCU; j++) {
+                                double src = 0.0;
+                                if (tdep) {
+                                    double tt = 0.0;
+#pragma unroll 4
+                                    for (int a = 0; a < NPV; a++) tt = fma(T.shapvt[g + NGV * a], shu[a + NPV * j], tt);
+                                    src = tt - w[j] * fc_u;
+                                }
+                                sm.wrk[g + NGV * (0 + ND1 * j)] = src * jg;
+#pragma unroll
+                                for (int r = 0; r < ND; r++) {
+                                    double fx = 0.0;
+#pragma unroll
+                                    for (int d = 0; d < ND; d++) fx = fma(f[d * NCU + j], X[r][d], fx);
+                                    sm.wrk[g + NGV * ((r + 1) + ND1 * j)] = fx;
+                                }
+                            }
+                        } else if (!GEN || A.conv_stab == 0) {
+                            // fhat = F(uh, q).n + tau (u - uh)   (fhatDriver.cpp:54-236), times jacf
+#pragma unroll
+                            for (int j = 0; j < NCU; j++) {
+                                double tt = tau * (ugf[g + NA * j] - w[j]) * sm.jacf[g];
+#pragma unroll
+                                for (int d = 0; d < ND; d++) tt = fma(f[d * NCU + j], X[0][d], tt);
+                                sm.fn[g + NA * j] = tt;
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < NCU; j++) {
+                                double tt = 0.0;
+#pragma unroll
+                                for (int d = 0; d < ND; d++) tt = fma(f[d * NCU + j], X[0][d], tt);
+                                sm.fn[g + NA * j] = tt;      // the stabilization term is added below
+                            }
+                        }
+                    }
+                    ns_flux_ucol<ND, GEN>(P, s, w, k, f, !A.inviscid, A.visc_model);
+                    if (vol) {
+                        const double jg = sm.jac[g];
+#pragma unroll
+                        for (int j = 0; j < NCU; j++) {
+                            wrl[g + NGV * (0 + ND1 * (j + NCU * k))] = (tdep && k == j) ? fc_u * jg : 0.0;
+#pragma unroll
+                            for (int r = 0; r < ND; r++) {
+                                double tt = 0.0;
+#pragma unroll
+                                for (int d = 0; d < ND; d++) tt = fma(f[d * NCU + j], X[r][d], tt);
+                                wrl[g + NGV * ((r + 1) + ND1 * (j + NCU * k))] = -tt;
+                            }
+                        }
+                        continue;
+                    }
+                    const double jf = sm.jacf[g];
+                    double sd[NCU], tcol[NCU];
+                    if (!GEN || A.conv_stab == 0) {
+#pragma unroll
+                        for (int j = 0; j < NCU; j++) {
+                            tcol[j] = k == j ? tau : 0.0;
+                            sd[j] = -tcol[j];
+                        }
+                    } else {
+                        // the Lax-Friedrichs or Roe tensor (ns_stab_point): the uh-derivative of
+                        // the stabilization term along this column, and column k of tau
+                        double nlq[ND], uv[NCU], sv[NCU];
+#pragma unroll
+                        for (int d = 0; d < ND; d++) nlq[d] = sm.nl[g + NA * d];
+#pragma unroll
+                        for (int m = 0; m < NCU; m++) uv[m] = ugf[g + NA * m];
+                        ns_stab_point<ND>(A.conv_stab, P, nlq, w, uv, k, sv, sd, tcol);
+                        if (k == 0)
+#pragma unroll
+                            for (int j = 0; j < NCU; j++) sm.fn[g + NA * j] += sv[j] * jf;
+                    }
+#pragma unroll
+                    for (int j = 0; j < NCU; j++) {
+                        double dn = sd[j] * jf;
+#pragma unroll
+                        for (int d = 0; d < ND; d++) dn = fma(f[d * NCU + j], X[0][d], dn);
+                        sl[NGF * NCH * NC + q + NGF * (j + NCH * k)] = dn;
+                        sl[q + NGF * (j + NCH * k)] = tcol[j] * jf;
+                    }
+                }
+            }
+            // pointwise fluxes, 3xTF32 form: one work item per (point, differentiated
+            // variable k); a one-derivative dual pass gives f and df/dw_k at that point.
+            if constexpr (TF)
             for (int t = tid1; t < (NGV + NA) * NC; t += NT1) {
                 using DD = Dual<1>;
                 const int p = t % (NGV + NA), k = t / (NGV + NA);
@@ -470,8 +631,9 @@ __global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
         // One thread per (g, j, c) with g fastest: its wrl words are read once and
         // the stores of a warp are runs of consecutive words.
         // The next item's wrl words are requested before this item's products, so
-        // their latency overlaps them.
-        {
+        // their latency overlaps them.  (3xTF32 form; the FP64 form makes Y in the
+        // volume GEMM's A fragments.)
+        if constexpr (TF) {
             constexpr int NY = NGV * NCU * NC;
             auto wload = [&](int t, double* w) {
                 const int g = t % NGV, j = (t / NGV) % NCU, c = t / (NGV * NCU);
@@ -494,85 +656,133 @@ __global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
                 for (int r = 0; r < ND1; r++) w[r] = wn[r];
             }
         }
-        // volume B operands: Phi (KV3 x NKP) and Psi (KQ3 x NHP), ld LDBD.  The
-        // rows d' > 0 are shapvt (M^-1 C | M^-1 E) on the tensor cores; the d' = 0
-        // rows of Phi (the basis values) and the zero padding are written directly.
+        // volume B operands: Phi and Psi, row g + LG d' (LG = NGV, padded to whole
+        // k-steps in the FP64 form).  The rows d' > 0 are shapvt (M^-1 C | M^-1 E)
+        // on the tensor cores; the d' = 0 rows of Phi (the basis values) and the
+        // zero padding are written directly.
+        constexpr int LG = TF ? NGV : G::NGP, LDV = TF ? G::LDBD : G::LDBP, KVB = TF ? G::KV3 : G::KVP;
         {
             double* Phi = Bs;
-            double* Psi = Bs + G::LDBD * G::NKP;
-            for (int t = tid; t < G::KV3 * G::NKP; t += NT) {
-                const int k = t % G::KV3, a = t / G::KV3;
-                if (a < NPV && k >= NGV && k < NGV * ND1) continue;
-                bput<TF>(&Phi[k + G::LDBD * a], (a < NPV && k < NGV) ? T.shapvt[k + NGV * a] : 0.0);
+            double* Psi = Bs + LDV * G::NKP;
+            for (int t = tid; t < KVB * G::NKP; t += NT) {
+                const int k = t % KVB, a = t / KVB, g = k % LG, dp = k / LG;
+                if (a < NPV && dp > 0 && dp < ND1 && g < NGV) continue;
+                bput<TF>(&Phi[k + LDV * a], (a < NPV && dp == 0 && g < NGV) ? T.shapvt[g + NGV * a] : 0.0);
             }
-            for (int t = tid; t < G::KV3 * G::NHP; t += NT) {
-                const int k = t % G::KV3, f2 = t / G::KV3;
-                if (f2 < NDF && k < NGV * ND) continue;
-                bput<TF>(&Psi[k + G::LDBD * f2], 0.0);
+            for (int t = tid; t < KVB * G::NHP; t += NT) {
+                const int k = t % KVB, f2 = t / KVB;
+                if (f2 < NDF && k < LG * ND && k % LG < NGV) continue;
+                bput<TF>(&Psi[k + LDV * f2], 0.0);
             }
             basis_ce_gemm<NGV, NPV, NPV, NPV * ND + NDF * ND, NT / 32>(
                 T.shapvt, NGV, nullptr, Cm, [&](int g, int n, double v) {
                     if (n < NPV * ND) {
                         const int a = n % NPV, d = n / NPV;
-                        bput<TF>(&Phi[(g + NGV * (d + 1)) + G::LDBD * a], v);
+                        bput<TF>(&Phi[(g + LG * (d + 1)) + LDV * a], v);
                     } else {
                         const int f2 = (n - NPV * ND) % NDF, d = (n - NPV * ND) / NDF;
-                        bput<TF>(&Psi[(g + NGV * d) + G::LDBD * f2], -v);
+                        bput<TF>(&Psi[(g + LG * d) + LDV * f2], -v);
                     }
                 });
         }
         __syncthreads();
-        // ---- D_vol = Y' Phi and F_vol = Y'_q Psi (right after Y is written, while it is in L2)
+        // ---- D_vol = Y' Phi and F_vol = Y'_q Psi
         {
             const double* Phi = Bs;
-            const double* Psi = Bs + G::LDBD * G::NKP;
+            const double* Psi = Bs + LDV * G::NKP;
             // m-tiles in pairs: every B fragment read from shared memory feeds two
             // DMMAs (shared-memory bandwidth is the busiest unit of this kernel)
             constexpr int MTD = (NPV * NCU * NCU + 7) / 8;
-            // with NGV a multiple of 4 the F part's A values are the D part's
-            // shifted by NGV/4 k-steps (the q derivatives d' = d + 1)
-            constexpr bool SHIFT = NGV % 4 == 0 && G::KV3 == NGV * ND1;
             if constexpr (!TF) {
+            // A fragments made on the fly: the lane's entry (i; g, d') of row (i,j,k) is
+            // sum_r shapvg(i, (g, r)) wrl((g, r), j, (d', k)), 4 products in 3D.  Every
+            // entry is used by this warp alone, for all n-tiles of D and F, so nothing is
+            // formed twice, and Y (0.38 MB per tetrahedron p = 3) is neither written to
+            // nor read from the workspace: 3D p=3, 40k of 440k cycles per element, and a
+            // working set of all CTAs (52 MB of wrl and face slices) that stays in L2.
+            // Rows (i, pair of NsPairs): the pairs whose flux does not depend on the
+            // gradients come last; their row tiles take d' = 0 only and have F_vol = 0.
+            constexpr int SW = NGV * ND1 * NCU * NCU;      // wrl stride of d'
+            using PR = NsPairs<ND>;
+            constexpr int MDEP = (PR::DEP * NPV + 7) / 8;  // row tiles with gradient columns
             for (int mp = warp; 2 * mp < MTD; mp += NT / 32) {
-                int rr[2];
+                int ii[2], jj[2], kk[2];
                 bool rv[2];
-                const double* yrow[2];
+                const double* wr[2];
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
-                    rr[u] = 8 * (2 * mp + u) + gr;
-                    rv[u] = rr[u] < NPV * NCU * NCU;
-                    const int i = rr[u] % NPV, j = (rr[u] / NPV) % NCU, k = rr[u] / (NPV * NCU);
-                    yrow[u] = Ys + NGV * (k + NC * (i + NPV * j));
+                    const int r = 8 * (2 * mp + u) + gr;
+                    rv[u] = r < NPV * PR::ALL;
+                    const int rc = rv[u] ? r : 0;          // rows past the end: computed, not stored
+                    ii[u] = rc % NPV;
+                    PR::at(rc / NPV, jj[u], kk[u]);
+                    wr[u] = wrl + NGV * ND1 * (jj[u] + NCU * kk[u]);
                 }
-                // the A values of both m-tiles for every k-step are loaded before the
-                // first DMMA, so their latencies overlap
-                double av[2][G::KV3 / 4];
+                double acc[2][G::NTK][2], accf[2][G::NTH][2];
 #pragma unroll
-                for (int u = 0; u < 2; u++)
-#pragma unroll
-                    for (int ks = 0; ks < G::KV3 / 4; ks++) {
-                        const int kk = 4 * ks + gc, g = kk % NGV, dp = kk / NGV;
-                        av[u][ks] = (rv[u] && kk < NGV * ND1) ? yrow[u][g + NGV * NCU * dp] : 0.0;
-                    }
-                double acc[2][G::NTK][2];
-#pragma unroll
-                for (int u = 0; u < 2; u++)
+                for (int u = 0; u < 2; u++) {
 #pragma unroll
                     for (int b = 0; b < G::NTK; b++) acc[u][b][0] = acc[u][b][1] = 0.0;
 #pragma unroll
-                for (int ks = 0; ks < G::KV3 / 4; ks++) {
-                    const int kk = 4 * ks + gc;
-#pragma unroll
-                    for (int b = 0; b < G::NTK; b++) {
-                        const double bv = Phi[kk + G::LDBD * (8 * b + gr)];
-                        dmma8x8x4(acc[0][b][0], acc[0][b][1], av[0][ks], bv);
-                        dmma8x8x4(acc[1][b][0], acc[1][b][1], av[1][ks], bv);
-                    }
+                    for (int b = 0; b < G::NTH; b++) accf[u][b][0] = accf[u][b][1] = 0.0;
                 }
+                auto steps = [&](auto fullc) {
+                    constexpr int DP = decltype(fullc)::value ? ND1 : 1;
+                    bool dep[2];
+#pragma unroll
+                    for (int u = 0; u < 2; u++) dep[u] = jj[u] > 0 && (kk[u] <= ND || jj[u] == ND + 1);
+#pragma unroll 1
+                    for (int gs = 0; gs < G::NGP / 4; gs++) {
+                        const int g = 4 * gs + gc;
+                        const bool gv = g < NGV;
+                        const int gl = gv ? g : 0;
+                        double av[2][DP];
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            // d' = 0 has the source row r = 0; d' > 0 only r > 0, and only where
+                            // the pair depends on the gradients (else never written)
+                            double w[DP][ND1];
+#pragma unroll
+                            for (int dp = 0; dp < DP; dp++)
+#pragma unroll
+                                for (int r = (dp > 0); r < ND1; r++)
+                                    w[dp][r] = (dp == 0 || dep[u]) ? wr[u][gl + NGV * r + SW * dp] : 0.0;
+#pragma unroll
+                            for (int dp = 0; dp < DP; dp++) av[u][dp] = 0.0;
+#pragma unroll
+                            for (int r = 0; r < ND1; r++) {
+                                const double sv = gv ? sm.Av[ii[u] + G::LDAV * (gl + NGV * r)] : 0.0;
+#pragma unroll
+                                for (int dp = 0; dp < DP; dp++)
+                                    if (dp == 0 || r > 0) av[u][dp] = fma(sv, w[dp][r], av[u][dp]);
+                            }
+                        }
+                        const double* ph0 = Phi + g + LDV * gr;
+                        const double* ps0 = Psi + g + LDV * gr;
+#pragma unroll
+                        for (int dp = 0; dp < DP; dp++) {
+#pragma unroll
+                            for (int b = 0; b < G::NTK; b++) {
+                                const double bv = ph0[LG * dp + LDV * 8 * b];
+                                dmma8x8x4(acc[0][b][0], acc[0][b][1], av[0][dp], bv);
+                                dmma8x8x4(acc[1][b][0], acc[1][b][1], av[1][dp], bv);
+                            }
+                            if (dp == 0) continue;
+#pragma unroll
+                            for (int b = 0; b < G::NTH; b++) {
+                                const double bv = ps0[LG * (dp - 1) + LDV * 8 * b];
+                                dmma8x8x4(accf[0][b][0], accf[0][b][1], av[0][dp], bv);
+                                dmma8x8x4(accf[1][b][0], accf[1][b][1], av[1][dp], bv);
+                            }
+                        }
+                    }
+                };
+                if (2 * mp < MDEP) steps(std::true_type{});
+                else steps(std::false_type{});
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
                     if (!rv[u]) continue;
-                    const int i = rr[u] % NPV, j = (rr[u] / NPV) % NCU, k = rr[u] / (NPV * NCU);
+                    const int i = ii[u], j = jj[u], k = kk[u];
 #pragma unroll
                     for (int b = 0; b < G::NTK; b++)
 #pragma unroll
@@ -580,38 +790,6 @@ __global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
                             const int a = 8 * b + 2 * gc + h;
                             if (a < NPV) De[i + NPV * (j + NCU * (a + NPV * k))] = acc[u][b][h];
                         }
-                }
-                double aq[2][G::KQ3 / 4];
-#pragma unroll
-                for (int u = 0; u < 2; u++)
-#pragma unroll
-                    for (int ks = 0; ks < G::KQ3 / 4; ks++) {
-                        if constexpr (SHIFT) {
-                            aq[u][ks] = av[u][ks + NGV / 4];
-                        } else {
-                            const int kk = 4 * ks + gc, g = kk % NGV, d = kk / NGV;
-                            aq[u][ks] = (rv[u] && kk < NGV * ND) ? yrow[u][g + NGV * NCU * (d + 1)] : 0.0;
-                        }
-                    }
-                double accf[2][G::NTH][2];
-#pragma unroll
-                for (int u = 0; u < 2; u++)
-#pragma unroll
-                    for (int b = 0; b < G::NTH; b++) accf[u][b][0] = accf[u][b][1] = 0.0;
-#pragma unroll
-                for (int ks = 0; ks < G::KQ3 / 4; ks++) {
-                    const int kk = 4 * ks + gc;
-#pragma unroll
-                    for (int b = 0; b < G::NTH; b++) {
-                        const double bv = Psi[kk + G::LDBD * (8 * b + gr)];
-                        dmma8x8x4(accf[0][b][0], accf[0][b][1], aq[0][ks], bv);
-                        dmma8x8x4(accf[1][b][0], accf[1][b][1], aq[1][ks], bv);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    if (!rv[u]) continue;
-                    const int i = rr[u] % NPV, j = (rr[u] / NPV) % NCU, k = rr[u] / (NPV * NCU);
 #pragma unroll
                     for (int b = 0; b < G::NTH; b++)
 #pragma unroll
@@ -622,7 +800,10 @@ __global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
                 }
             }
             } else {
-            // 3xTF32: the same m-tile pairs as one m16 tile, k-steps of 8
+            // 3xTF32: the m-tile pairs as one m16 tile, k-steps of 8, Y from the workspace;
+            // with NGV a multiple of 4 the F part's A values are the D part's
+            // shifted by NGV/4 k-steps (the q derivatives d' = d + 1)
+            constexpr bool SHIFT = NGV % 4 == 0 && G::KV3 == NGV * ND1;
             const uint2* Phi2 = reinterpret_cast<const uint2*>(Phi);
             const uint2* Psi2 = reinterpret_cast<const uint2*>(Psi);
             constexpr int KS = G::KV3 / 4, KSQ = G::KQ3 / 4;
@@ -730,8 +911,18 @@ __global__ void __launch_bounds__(NT, 2) element_kernel(ElemArgs A) {
         double ru2 = 0.0;
         for (int t = tid; t < N; t += NT) {
             const int i = t % NPV, j = t / NPV;
+            // ND1 partial sums (one per derivative index), not one chain of NQ FMAs
+            double sp[ND1];
+#pragma unroll
+            for (int r = 0; r < ND1; r++) sp[r] = 0.0;
+#pragma unroll 4
+            for (int g = 0; g < NGV; g++)
+#pragma unroll
+                for (int r = 0; r < ND1; r++)
+                    sp[r] = fma(sm.Av[i + G::LDAV * (g + NGV * r)], sm.wrk[g + NGV * r + NQ * j], sp[r]);
             double s = 0.0;
-            for (int q = 0; q < NQ; q++) s += sm.Av[i + G::LDAV * q] * sm.wrk[q + NQ * j];
+#pragma unroll
+            for (int r = 0; r < ND1; r++) s += sp[r];
             for (int c2 = 0; c2 < sm.inc_n[i]; c2++) s += sm.rh[j + NCH * sm.inc_f[i * S::MAXINC + c2]];
             A.Ru[(size_t)e * N + t] = s;
             ru2 += s * s;

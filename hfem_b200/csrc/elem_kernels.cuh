@@ -11,6 +11,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "ns_flux.cuh"
+#include "schur_kernels.cuh"
 
 namespace hfem {
 
@@ -22,6 +23,14 @@ struct Shape {
     static constexpr int NA = NGF * NFE;          // face points of one element
     static constexpr int NQ = NGV * ND1;          // (volume point, derivative) pairs
     static constexpr int MAXINC = ND;             // faces meeting at a node
+    // threads per CTA of the element kernel, at 512 threads per SM: the phases of a
+    // small element have too little work for 8 warps, so more and smaller CTAs per SM
+    // overlap their barriers and latencies.  Measured (ms, 64 / 128 / 256 threads):
+    // 2D p1, 7,200 elements 0.130 / 0.173 / 0.311; 2D p2, 2,048: 0.081 / 0.108 / 0.133;
+    // 3D p1, 10,368: 0.56 / 0.60 / 0.86; 2D p3, 4,050 (Roe, Sutherland): 0.45 / 0.35 /
+    // 0.44; 2D p4, 7,938: 0.88 / 0.76 / 1.00; 3D p2, 4,374: 1.41 / 0.96 / 1.11; 3D p3,
+    // 4,374: 7.3 / 4.2 / 3.1.  (Caps of 640 to 1,024 threads per SM: slower, spills.)
+    static constexpr int NT = N <= 24 ? 64 : (N <= 60 ? 128 : 256);
 };
 
 struct Tables {                 // master element tables, reference layouts
@@ -39,7 +48,7 @@ struct ElemArgs {
     double fc_u, fc_q;
     int ne;
     double *D, *F, *K, *H, *Ru, *Rh, *Ro, *ru2;
-    double* ws;                 // gridDim.x workspace slots of EK<S>::WS doubles (element_kernel)
+    double* ws;                 // gridDim.x workspace slots of EK<S>::WS (3xTF32: WS_TF) doubles (element_kernel)
     // several problems in one mesh (NULL = the uniform values above): element ->
     // problem, and per problem [gamma, eps, Re, Pr, Mach, tau, tdep, fc_u]
     const int* eprob;
@@ -56,7 +65,7 @@ struct ElemArgs {
     int e_begin = 0;            // element range [e_begin, ne) of this launch
 };
 
-constexpr int NT = 256;         // threads per CTA for element kernels
+constexpr int QT = 256;         // threads per CTA of the q recovery
 
 // --------------------------------------------------------------- helpers
 __device__ __forceinline__ double block_sum(double v, double* red) {
@@ -169,6 +178,94 @@ __device__ void qmatrices(const Tables& T, double fc_q, const double* jac, const
             s += T.sfsf[(k + NPF * j) + NPF2 * g] * nl[g + NGF * fc + NA * d] * jacf[g + NGF * fc];
         E[T.perm[fc * NPF + k] + NPV * ((fc * NPF + j) + NDF * d)] = s;
     }
+}
+
+// The same matrices for the element kernel's FP64 form, from the factors held in
+// shared memory instead of the product tables (307 KB of svsv for the
+// tetrahedron p = 3, re-read from L2 for every element): with
+//   P_0(b, g) = fc_q shapvg(b, g) jac(g),  P_d(b, g) = sum_i shapvg(b, (g, i)) Xx(g; d, i)
+// M and C_d are the products P_d phi', npv (nd + 1) rows by npv columns, on the
+// FP64 tensor cores; E's entries are shapfg shapfc sums with shapfg and shapfc
+// from shared memory.  av(b, q) = shapvg, af(k, g) = shapfg, sfc = shapfc.
+template <class S, int NTHR, class AV, class AF>
+__device__ __forceinline__ void qmatrices_factored(const Tables& T, double fc_q, const double* jac, const double* Xx,
+                                                   const double* jacf, const double* nl, AV av, AF af,
+                                                   const double* sfc, const int* perm, double* M, double* C, double* E) {
+    constexpr int ND = S::ND, NPV = S::NPV, NGV = S::NGV, NGF = S::NGF, NPF = S::NPF, NA = S::NA, NDF = S::NDF;
+    constexpr int NR = NPV * (ND + 1), MT = (NR + 7) / 8, KS = (NGV + 3) / 4, NTN = (NPV + 7) / 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gr = lane >> 2, gc = lane & 3;
+    for (int t = threadIdx.x; t < NPV * NDF * ND; t += NTHR) E[t] = 0.0;
+    double bf[KS][NTN];
+#pragma unroll
+    for (int ks = 0; ks < KS; ks++)
+#pragma unroll
+        for (int b = 0; b < NTN; b++) {
+            const int g = 4 * ks + gc, a = 8 * b + gr;
+            bf[ks][b] = (g < NGV && a < NPV) ? __ldg(&T.shapvt[g + NGV * a]) : 0.0;
+        }
+    for (int mt = warp; mt < MT; mt += NTHR / 32) {
+        const int r = 8 * mt + gr, b = r % NPV, d = r / NPV;
+        double acc[NTN][2];
+#pragma unroll
+        for (int n = 0; n < NTN; n++) acc[n][0] = acc[n][1] = 0.0;
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++) {
+            const int g = 4 * ks + gc;
+            double a = 0.0;
+            if (g < NGV && r < NR) {
+                if (d == 0) {
+                    a = av(b, g) * (fc_q * jac[g]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < ND; i++) a += av(b, g + NGV * (i + 1)) * Xx[g + NGV * ((d - 1) + ND * i)];
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < NTN; n++) dmma8x8x4(acc[n][0], acc[n][1], a, bf[ks][n]);
+        }
+        if (r < NR)
+#pragma unroll
+            for (int n = 0; n < NTN; n++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int a = 8 * n + 2 * gc + h;
+                    if (a < NPV) (d == 0 ? M : C + NPV * NPV * (d - 1))[b + NPV * a] = acc[n][h];
+                }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < ND * NDF * NPF; t += NTHR) {
+        const int k = t % NPF, j = (t / NPF) % NPF, fc = (t / (NPF * NPF)) % S::NFE, d = t / (NPF * NPF * S::NFE);
+        double s = 0.0;
+#pragma unroll 4
+        for (int g = 0; g < NGF; g++)
+            s += af(k, g) * sfc[g + NGF * j] * (nl[g + NGF * fc + NA * d] * jacf[g + NGF * fc]);
+        E[perm[fc * NPF + k] + NPV * ((fc * NPF + j) + NDF * d)] = s;
+    }
+}
+
+// Lower Cholesky of M (npv x npv) in place by one warp, right-looking: lane i
+// holds row i in registers, so a column costs one square root, one division and
+// one shuffle per entry of its row instead of a dot product over the columns
+// before it; rdg receives the reciprocals of the diagonal.
+template <int NPV>
+__device__ __forceinline__ void cholesky_warp_rows(double* a, double* rdg) {
+    static_assert(NPV <= 32, "one row per lane");
+    const int lane = threadIdx.x & 31, row = lane < NPV ? lane : NPV - 1;
+    double r[NPV];
+#pragma unroll
+    for (int k = 0; k < NPV; k++) r[k] = a[row + NPV * k];
+#pragma unroll
+    for (int j = 0; j < NPV; j++) {
+        const double l = sqrt(__shfl_sync(0xffffffffu, r[j], j)), inv = 1.0 / l;
+        if (lane == j) rdg[j] = inv;
+        r[j] = lane == j ? l : r[j] * inv;
+#pragma unroll
+        for (int k = j + 1; k < NPV; k++) r[k] = fma(-r[j], __shfl_sync(0xffffffffu, r[j], k), r[k]);
+    }
+    if (lane < NPV)
+#pragma unroll
+        for (int k = 0; k < NPV; k++)
+            if (k <= lane) a[lane + NPV * k] = r[k];
 }
 
 // Lower Cholesky of M (npv x npv) in place, one warp; rdg (if given) receives
@@ -331,7 +428,7 @@ struct QSmem {
 
 // getQ (elementassembly.cpp:1414-1479), optionally preceded by getU (solutionupdate.cpp:6-68).
 template <class S>
-static __global__ void __launch_bounds__(NT) getq_kernel(QArgs A) {
+static __global__ void __launch_bounds__(QT) getq_kernel(QArgs A) {
     constexpr int ND = S::ND, NPV = S::NPV, NCU = S::NCU, NC = S::NC, NCH = S::NCH, NDF = S::NDF, N = S::N, NB = S::NB;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     QSmem<S>& sm = *reinterpret_cast<QSmem<S>*>(smem_raw);
@@ -339,8 +436,8 @@ static __global__ void __launch_bounds__(NT) getq_kernel(QArgs A) {
     for (int e = blockIdx.x; e < A.ne; e += gridDim.x) {
         __syncthreads();
         double* ue = A.udg + (size_t)e * NPV * NC;
-        for (int t = tid; t < NPV * ND; t += NT) sm.x[t] = A.dgnodes[(size_t)e * NPV * ND + t];
-        for (int t = tid; t < NDF * NCH; t += NT) {
+        for (int t = tid; t < NPV * ND; t += QT) sm.x[t] = A.dgnodes[(size_t)e * NPV * ND + t];
+        for (int t = tid; t < NDF * NCH; t += QT) {
             const int fn = t / NCH, c = t % NCH;
             const int gd = A.elcon[(size_t)e * NDF + fn];
             sm.uhe[fn + NDF * c] = A.uh[(size_t)gd * NCH + c];
@@ -348,7 +445,7 @@ static __global__ void __launch_bounds__(NT) getq_kernel(QArgs A) {
         }
         __syncthreads();
         const double alpha = A.palpha ? A.palpha[A.eprob[e]] : A.alpha;
-        for (int t = tid; t < N; t += NT) {
+        for (int t = tid; t < N; t += QT) {
             double v = ue[t];
             if (A.DinvF) {
                 const double* df = A.DinvF + (size_t)e * N * NB;
@@ -365,7 +462,7 @@ static __global__ void __launch_bounds__(NT) getq_kernel(QArgs A) {
         qmatrices<S>(A.T, A.fc_q, sm.jac, sm.Xx, sm.jacf, sm.nl, sm.M, sm.C, sm.E);
         __syncthreads();
         const double* she = A.sh + (size_t)e * NPV * NC;
-        for (int t = tid; t < NPV * NCU * ND; t += NT) {
+        for (int t = tid; t < NPV * NCU * ND; t += QT) {
             const int i = t % NPV, c = (t / NPV) % NCU, d = t / (NPV * NCU);
             double s = 0.0;
             for (int a = 0; a < NPV; a++) s += sm.M[i + NPV * a] * she[a + NPV * (NCU * (1 + d) + c)];
@@ -376,9 +473,9 @@ static __global__ void __launch_bounds__(NT) getq_kernel(QArgs A) {
         __syncthreads();
         cholesky_warp<NPV>(sm.M);
         __syncthreads();
-        for (int t = tid; t < NCU * ND; t += NT) chol_solve_col<NPV>(sm.M, &sm.q[NPV * t]);
+        for (int t = tid; t < NCU * ND; t += QT) chol_solve_col<NPV>(sm.M, &sm.q[NPV * t]);
         __syncthreads();
-        for (int t = tid; t < NPV * NCU * ND; t += NT) {
+        for (int t = tid; t < NPV * NCU * ND; t += QT) {
             const int i = t % NPV, c = (t / NPV) % NCU, d = t / (NPV * NCU);
             ue[i + NPV * (NCU * (1 + d) + c)] = sm.q[t];
         }

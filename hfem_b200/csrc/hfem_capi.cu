@@ -388,7 +388,7 @@ int ensure_assembly_buffers(hfem_ctx* c) {
     if ((rc = dalloc(c, &c->Ro, ne * nb))) return rc;
     if ((rc = dalloc(c, &c->ru2, ne))) return rc;
     if ((rc = dalloc(c, &c->info, ne))) return rc;
-    if ((rc = dalloc(c, &c->ws, (size_t)c->grid_elem * c->L->ws))) return rc;
+    if ((rc = dalloc(c, &c->ws, (size_t)c->grid_elem * c->L->ws_tf))) return rc;
     if ((rc = dalloc(c, &c->tc_err, 1))) return rc;
     if ((rc = dalloc(c, &c->rn_part, NORM_CTAS))) return rc;
     if ((rc = dalloc(c, &c->rn_ticket, 1))) return rc;
@@ -1443,13 +1443,13 @@ int hfem_create(const hfem_dims* dims, int device, hfem_ctx** out) {
             cudaFuncSetAttribute(L.elem_fn_v[t][g], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.elem_smem);
     cudaFuncSetAttribute(L.q_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.q_smem);
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.elem_fn, NT, L.elem_smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.elem_fn, L.elem_threads, L.elem_smem);
     c->grid_elem = std::max(1, std::min(d.ne, sms(device) * std::max(occ, 1)));
     // the workspace has grid_elem slots: no variant runs more CTAs
     for (int t = 0; t < 2; t++)
         for (int g = 0; g < 2; g++) {
             occ = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.elem_fn_v[t][g], NT, L.elem_smem);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.elem_fn_v[t][g], L.elem_threads, L.elem_smem);
             c->grid_elem_v[t][g] = std::max(1, std::min(c->grid_elem, sms(device) * std::max(occ, 1)));
         }
     cudaFuncSetAttribute(L.g1.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.g1.smem);
@@ -2390,7 +2390,7 @@ extern "C" int hfem_condense_noalloc(const hfem_dims* dims, const double* shapvt
                     cudaSuccess)
                 return HFEM_E_CUDA;
             int occ = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L->elem_fn, NT, L->elem_smem);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L->elem_fn, L->elem_threads, L->elem_smem);
             const int slots = (int)(HFEM_NOALLOC_SCRATCH_BYTES / slot_bytes);
             G.elem = std::max(1, std::min(slots, sms(dev) * std::max(occ, 1)));
             occ = 0;

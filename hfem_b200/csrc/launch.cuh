@@ -48,7 +48,8 @@ template <int MT, int WN, int NW, int BK, int ST> struct GemmParams<GemmCfg<MT, 
 
 struct Launch {
     int nd, npv, npf, ngv, ngf;
-    size_t ws;                  // workspace doubles per CTA slot (element_kernel)
+    size_t ws, ws_tf;           // workspace doubles per CTA slot of element_kernel, FP64 and 3xTF32 forms
+    int elem_threads;           // threads per CTA of the element kernels
     size_t q_smem;
     void (*getq)(dim3, size_t, cudaStream_t, const QArgs&);
     void (*inverse)(dim3, cudaStream_t, int, double*, const double*, double*, int*);

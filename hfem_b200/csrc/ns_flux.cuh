@@ -170,6 +170,200 @@ __device__ __forceinline__ void ns_flux_dual(const double* __restrict__ param, c
     }
 }
 
+// The flux and its Jacobian columns at one point without dual numbers, for the
+// element kernel's FP64 form.  (A dual pass computes every product with a zero
+// derivative, and all columns' values again.)  ns_point holds what the columns
+// share; f[d * ncu + j], fd[d * ncu + j] as ns_flux_dual's value and derivative.
+template <int ND>
+struct NsPoint {
+    double ir, v[ND], p, E, rho;
+    double G[ND][ND];       // G[d][i] = dv_i / dx_d
+    double q0[ND], qE[ND];  // gradients of rho and rho E
+    double div, mu;
+};
+
+template <int ND, bool GEN = false>
+__device__ __forceinline__ NsPoint<ND> ns_point(const double* __restrict__ param, const double* w, int visc_model) {
+    constexpr int NCU = ND + 2;
+    NsPoint<ND> s;
+    s.rho = w[0];
+    s.E = w[ND + 1];
+    s.ir = 1.0 / w[0];
+    double ke = 0.0;
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+        s.v[i] = w[1 + i] * s.ir;
+        ke = fma(s.v[i], w[1 + i], ke);
+    }
+    s.p = (param[0] - 1.0) * (s.E - 0.5 * ke);
+    s.div = 0.0;
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        const double* q = w + NCU * (1 + d);
+        s.q0[d] = q[0];
+        s.qE[d] = q[ND + 1];
+#pragma unroll
+        for (int i = 0; i < ND; i++) s.G[d][i] = (q[1 + i] - s.v[i] * q[0]) * s.ir;
+        s.div += s.G[d][d];
+    }
+    s.mu = 1.0;
+    if constexpr (GEN) {
+        if (visc_model != 0) {
+            Dual<1> wd[NCU];
+#pragma unroll
+            for (int c = 0; c < NCU; c++) wd[c] = dc<1>(w[c]);
+            s.mu = ns_sutherland<ND, 1>(param, wd).v;
+        }
+    }
+    return s;
+}
+
+// the flux
+template <int ND>
+__device__ __forceinline__ void ns_flux_value(const double* __restrict__ param, const NsPoint<ND>& s, double* f,
+                                              bool viscous) {
+    constexpr int NCU = ND + 2;
+    const double a = s.mu / param[2], kap = s.mu * (param[0] / (param[2] * param[3]));
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        f[d * NCU] = s.rho * s.v[d];
+        double fe = (s.E + s.p) * s.v[d], vg = 0.0;
+#pragma unroll
+        for (int i = 0; i < ND; i++) {
+            double t = s.G[d][i] + s.G[i][d];
+            if (i == d) t -= (2.0 / 3.0) * s.div;
+            t = viscous ? a * t : 0.0;
+            f[d * NCU + 1 + i] = fma(s.rho * s.v[i], s.v[d], t) + (i == d ? s.p : 0.0);
+            fe = fma(t, s.v[i], fe);
+            vg = fma(s.v[i], s.G[d][i], vg);
+        }
+        const double heat = s.qE[d] * s.ir - s.E * s.q0[d] * (s.ir * s.ir) - vg;
+        f[d * NCU + ND + 1] = viscous ? fma(kap, heat, fe) : fe;
+    }
+}
+
+// column k < ncu: the derivative along the conserved variable u_k
+template <int ND, bool GEN = false>
+__device__ __forceinline__ void ns_flux_ucol(const double* __restrict__ param, const NsPoint<ND>& s, const double* w,
+                                             int k, double* fd, bool viscous, int visc_model) {
+    constexpr int NCU = ND + 2;
+    const double g1 = param[0] - 1.0, iRe = 1.0 / param[2], kappa = param[0] / (param[2] * param[3]);
+    const double drho = k == 0 ? 1.0 : 0.0, dE = k == ND + 1 ? 1.0 : 0.0;
+    double dm[ND], dv[ND], dke = 0.0;
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+        dm[i] = k == 1 + i ? 1.0 : 0.0;
+        dv[i] = (dm[i] - s.v[i] * drho) * s.ir;
+        dke = fma(dv[i], w[1 + i], fma(s.v[i], dm[i], dke));
+    }
+    const double dp = g1 * (dE - 0.5 * dke);
+    double dG[ND][ND], ddiv = 0.0;
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+#pragma unroll
+        for (int i = 0; i < ND; i++) dG[d][i] = -(dv[i] * s.q0[d] + s.G[d][i] * drho) * s.ir;
+        ddiv += dG[d][d];
+    }
+    double dmu = 0.0;
+    if constexpr (GEN) {
+        if (visc_model != 0) {
+            Dual<1> wd[NCU];
+#pragma unroll
+            for (int c = 0; c < NCU; c++) {
+                wd[c].v = w[c];
+                wd[c].d[0] = c == k ? 1.0 : 0.0;
+            }
+            dmu = ns_sutherland<ND, 1>(param, wd).d[0];
+        }
+    }
+    const double ir2 = s.ir * s.ir;
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        fd[d * NCU] = dm[d];
+        double fe = fma(dE + dp, s.v[d], (s.E + s.p) * dv[d]), vg = 0.0, dvg = 0.0;
+#pragma unroll
+        for (int i = 0; i < ND; i++) {
+            double t = s.G[d][i] + s.G[i][d], dt = dG[d][i] + dG[i][d];
+            if (i == d) {
+                t -= (2.0 / 3.0) * s.div;
+                dt -= (2.0 / 3.0) * ddiv;
+            }
+            if constexpr (GEN) dt = fma(s.mu, dt, dmu * t);
+            dt = viscous ? iRe * dt : 0.0;
+            t = viscous ? iRe * (GEN ? s.mu * t : t) : 0.0;
+            fd[d * NCU + 1 + i] = fma(dm[i], s.v[d], fma(w[1 + i], dv[d], dt)) + (i == d ? dp : 0.0);
+            fe = fma(dt, s.v[i], fma(t, dv[i], fe));
+            vg = fma(s.v[i], s.G[d][i], vg);
+            dvg = fma(dv[i], s.G[d][i], fma(s.v[i], dG[d][i], dvg));
+        }
+        double dheat = -s.qE[d] * ir2 * drho - dE * s.q0[d] * ir2 + 2.0 * s.E * s.q0[d] * ir2 * s.ir * drho - dvg;
+        if constexpr (GEN) {
+            const double heat = s.qE[d] * s.ir - s.E * s.q0[d] * ir2 - vg;
+            dheat = fma(s.mu, dheat, dmu * heat);
+        }
+        fd[d * NCU + ND + 1] = viscous ? fma(kappa, dheat, fe) : fe;
+    }
+}
+
+// The derivative along q_{dq,m}, the gradient of variable m in direction dq: the
+// viscous flux is linear in q, so the column is the flux of the unit gradient,
+// g_i = dv_i/dx_dq with its stress and heat terms.  The mass flux does not depend
+// on q, and the momentum fluxes not on q_{dq,nd+1}: those entries are zero
+// (NsPairs).
+template <int ND>
+__device__ __forceinline__ void ns_flux_qcol(const double* __restrict__ param, const NsPoint<ND>& s, int dq, int m,
+                                             double* fd, bool viscous) {
+    constexpr int NCU = ND + 2;
+    const double a = viscous ? s.mu / param[2] : 0.0;
+    const double kap = viscous ? s.mu * (param[0] / (param[2] * param[3])) : 0.0;
+    double g[ND], gd = 0.0, vg = 0.0;
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+        g[i] = m == 0 ? -s.v[i] * s.ir : (m == i + 1 ? s.ir : 0.0);
+        if (i == dq) gd = g[i];
+        vg = fma(s.v[i], g[i], vg);
+    }
+    const double heat = (m == ND + 1 ? s.ir : (m == 0 ? -s.E * s.ir * s.ir : 0.0)) - vg;
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        fd[d * NCU] = 0.0;
+        double fe = 0.0;
+#pragma unroll
+        for (int i = 0; i < ND; i++) {
+            double t = (d == dq ? g[i] : 0.0) + (i == dq ? g[d] : 0.0);
+            if (i == d) t -= (2.0 / 3.0) * gd;
+            t *= a;
+            fd[d * NCU + 1 + i] = t;
+            fe = fma(t, s.v[i], fe);
+        }
+        fd[d * NCU + ND + 1] = d == dq ? fma(kap, heat, fe) : fe;
+    }
+}
+
+// The (equation j, variable m) pairs in two groups, those whose flux depends on
+// the gradient of m first: j = 1..nd+1 with m = 0..nd, and (nd+1, nd+1).  The
+// rest, mass with any variable and momentum with the energy, have zero d' > 0
+// columns in every volume, trace and boundary flux of this file (17 of 25 pairs
+// in 3D and 10 of 16 in 2D depend on gradients).
+template <int ND>
+struct NsPairs {
+    static constexpr int NCU = ND + 2, ALL = NCU * NCU, DEP = (ND + 1) * (ND + 1) + 1;
+    static __device__ __forceinline__ void at(int p, int& j, int& m) {
+        if (p < DEP - 1) {
+            j = 1 + p % (ND + 1);
+            m = p / (ND + 1);
+        } else if (p == DEP - 1) {
+            j = m = ND + 1;
+        } else if (p < DEP + NCU) {
+            j = 0;
+            m = p - DEP;
+        } else {
+            j = 1 + p - DEP - NCU;
+            m = ND + 1;
+        }
+    }
+};
+
 template <int N>
 __device__ __forceinline__ Dual<N> dsqrt(const Dual<N>& a) {
     Dual<N> r;

@@ -31,10 +31,10 @@ void launch_inverse(dim3 g, cudaStream_t st, int ne, double* D, const double* Ru
 
 template <class S, bool TF, bool GEN>
 void launch_element(dim3 g, size_t sm, cudaStream_t st, const ElemArgs& a) {
-    element_kernel<S, TF, GEN><<<g, NT, sm, st>>>(a);
+    element_kernel<S, TF, GEN><<<g, S::NT, sm, st>>>(a);
 }
 template <class S>
-void launch_getq(dim3 g, size_t sm, cudaStream_t st, const QArgs& a) { getq_kernel<S><<<g, NT, sm, st>>>(a); }
+void launch_getq(dim3 g, size_t sm, cudaStream_t st, const QArgs& a) { getq_kernel<S><<<g, QT, sm, st>>>(a); }
 template <class S>
 void launch_scatter_h(dim3 g, cudaStream_t st, const ScatterArgs& a) {
     scatter_H_block_kernel<S::NPF, S::NCH, S::NFE><<<g, 256, 0, st>>>(a);
@@ -66,6 +66,7 @@ Launch make_launch() {
     Launch L;
     L.nd = S::ND; L.npv = S::NPV; L.npf = S::NPF; L.ngv = S::NGV; L.ngf = S::NGF;
     L.ws = EK<S>::WS;
+    L.ws_tf = EK<S>::WS_TF;
     L.q_smem = sizeof(QSmem<S>);
     L.getq = launch_getq<S>;
     L.q_fn = (const void*)getq_kernel<S>;
@@ -75,6 +76,7 @@ Launch make_launch() {
     L.element_v[0][1] = launch_element<S, false, true>;
     L.element_v[1][0] = launch_element<S, true, false>;
     L.element_v[1][1] = launch_element<S, true, true>;
+    L.elem_threads = S::NT;
     L.elem_smem = sizeof(ElemSmem<S>);
     L.elem_fn = (const void*)element_kernel<S, false, false>;
     L.elem_fn_v[0][0] = (const void*)element_kernel<S, false, false>;
