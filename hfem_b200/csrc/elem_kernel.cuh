@@ -292,21 +292,15 @@ __global__ void __launch_bounds__(S::NT, 512 / S::NT) element_kernel(ElemArgs A)
         const int tdep = A.pparam ? (int)P[6] : A.tdep;
         const double fc_u = A.pparam ? P[7] : A.fc_u;
         const int* bfe = A.bf ? A.bf + (size_t)e * NFE : nullptr;
-        // warp 0 factors M while the other warps evaluate the states at the points
-        // and the pointwise fluxes, which do not depend on M
-        if (warp == 0) {
-            if constexpr (TF) cholesky_warp<NPV>(M, sm.rdg);
-            else cholesky_warp_rows<NPV>(M, sm.rdg);
-        } else {
-            constexpr int NT1 = NT - 32;
-            const int tid1 = tid - 32;
-            for (int t = tid1; t < NGV * NC; t += NT1) {
+        // the states at the points, by the threads of rank 0 <= rk < nrk
+        auto states = [&](int rk, int nrk) {
+            for (int t = rk; t < NGV * NC; t += nrk) {
                 const int g = t % NGV, c = t / NGV;
                 double s = 0.0;
                 for (int a = 0; a < NPV; a++) s += T.shapvt[g + NGV * a] * u[a + NPV * c];
                 ug[t] = s;
             }
-            for (int t = tid1; t < NA * (NC + NCH); t += NT1) {
+            for (int t = rk; t < NA * (NC + NCH); t += nrk) {
                 const int gg = t % NA, c = t / NA, fc = gg / NGF, q = gg % NGF;
                 double s = 0.0;
                 if (c < NC) {
@@ -317,157 +311,57 @@ __global__ void __launch_bounds__(S::NT, 512 / S::NT) element_kernel(ElemArgs A)
                     uhg[gg + NA * (c - NC)] = s;
                 }
             }
-            asm volatile("bar.sync 1, %0;" ::"r"(NT1) : "memory");
-            // FP64 form: one item per (point, u column) and one per (point, gradient
-            // direction), whose ncu columns share the point's terms.  (3D p=3: 57k cycles
-            // per element with a dual-number pass per column.)
-            if constexpr (!TF) {
-                constexpr int NPT = NGV + NA;
-                const double tau = P[5];
-                for (int t = tid1; t < NPT * (NCU + ND); t += NT1) {
-                    const int p = t % NPT, k = t / NPT;
-                    const bool vol = p < NGV;
-                    const int g = vol ? p : p - NGV, fc = g / NGF, q = g % NGF;
-                    double w[NC];
+        };
+        auto boundary_fluxes = [&](int rk, int nrk) {
+            // boundary faces: fb and its Jacobians at their points (one item per point and variable)
+            if (bfe) {
+                for (int t = rk; t < NFE * NGF * (NC + NCH); t += nrk) {
+                    const int fc = t / (NGF * (NC + NCH)), r = t % (NGF * (NC + NCH));
+                    if (bfe[fc] >= 0) continue;
+                    using DD = Dual<1>;
+                    const int q = r % NGF, k = r / NGF, gg = q + NGF * fc;
+                    DD w[NC], uhd[NCH], fb[NCH];
 #pragma unroll
-                    for (int c = 0; c < NC; c++)
-                        w[c] = vol ? ug[g + NGV * c] : ((c < NCU) ? uhg[g + NA * c] : ugf[g + NA * c]);
-                    const NsPoint<ND> s = ns_point<ND, GEN>(P, w, A.visc_model);
-                    // the metric of the volume point, or the scaled normal of the face point
-                    double X[ND][ND];
-                    if (vol) {
-#pragma unroll
-                        for (int m = 0; m < ND; m++)
-#pragma unroll
-                            for (int d = 0; d < ND; d++) X[m][d] = sm.Xx[g + NGV * (d + ND * m)];
-                    } else {
-#pragma unroll
-                        for (int d = 0; d < ND; d++) X[0][d] = sm.nl[g + NA * d] * sm.jacf[g];
-                    }
-                    double* sl = fsl + fc * G::FSLP;
-                    double f[ND * NCU];
-                    if (k >= NCU) {
-                        const int dq = k - NCU;
-#pragma unroll
-                        for (int m = 0; m < NCU; m++) {
-                            ns_flux_qcol<ND>(P, s, dq, m, f, !A.inviscid);
-                            const int c = NCU * (1 + dq) + m;
-                            // the entries that are zero for every state are not stored for the
-                            // volume (the GEMM skips them), nor is the source row r = 0
-#pragma unroll
-                            for (int j = 0; j < NCU; j++) {
-                                const bool dep = j > 0 && (m <= ND || j == ND + 1);
-                                if (vol) {
-                                    if (!dep) continue;
-#pragma unroll
-                                    for (int r = 0; r < ND; r++) {
-                                        double tt = 0.0;
-#pragma unroll
-                                        for (int d = 0; d < ND; d++) tt = fma(f[d * NCU + j], X[r][d], tt);
-                                        wrl[g + NGV * (r + 1 + ND1 * (j + NCU * c))] = -tt;
-                                    }
-                                } else {
-                                    double dn = 0.0;
-                                    if (dep)
-#pragma unroll
-                                        for (int d = 0; d < ND; d++) dn = fma(f[d * NCU + j], X[0][d], dn);
-                                    sl[q + NGF * (j + NCH * c)] = dn;
-                                }
-                            }
-                        }
-                        continue;
-                    }
-                    if (k == 0) {
-                        ns_flux_value<ND>(P, s, f, !A.inviscid);
-                        if (vol) {
-                            const double jg = sm.jac[g];
-#pragma unroll
-                            for (int j = 0; j < NCU; j++) {
-                                double src = 0.0;
-                                if (tdep) {
-                                    double tt = 0.0;
-#pragma unroll 4
-                                    for (int a = 0; a < NPV; a++) tt = fma(T.shapvt[g + NGV * a], shu[a + NPV * j], tt);
-                                    src = tt - w[j] * fc_u;
-                                }
-                                sm.wrk[g + NGV * (0 + ND1 * j)] = src * jg;
-#pragma unroll
-                                for (int r = 0; r < ND; r++) {
-                                    double fx = 0.0;
-#pragma unroll
-                                    for (int d = 0; d < ND; d++) fx = fma(f[d * NCU + j], X[r][d], fx);
-                                    sm.wrk[g + NGV * ((r + 1) + ND1 * j)] = fx;
-                                }
-                            }
-                        } else if (!GEN || A.conv_stab == 0) {
-                            // fhat = F(uh, q).n + tau (u - uh)   (fhatDriver.cpp:54-236), times jacf
-#pragma unroll
-                            for (int j = 0; j < NCU; j++) {
-                                double tt = tau * (ugf[g + NA * j] - w[j]) * sm.jacf[g];
-#pragma unroll
-                                for (int d = 0; d < ND; d++) tt = fma(f[d * NCU + j], X[0][d], tt);
-                                sm.fn[g + NA * j] = tt;
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < NCU; j++) {
-                                double tt = 0.0;
-#pragma unroll
-                                for (int d = 0; d < ND; d++) tt = fma(f[d * NCU + j], X[0][d], tt);
-                                sm.fn[g + NA * j] = tt;      // the stabilization term is added below
-                            }
-                        }
-                    }
-                    ns_flux_ucol<ND, GEN>(P, s, w, k, f, !A.inviscid, A.visc_model);
-                    if (vol) {
-                        const double jg = sm.jac[g];
-#pragma unroll
-                        for (int j = 0; j < NCU; j++) {
-                            wrl[g + NGV * (0 + ND1 * (j + NCU * k))] = (tdep && k == j) ? fc_u * jg : 0.0;
-#pragma unroll
-                            for (int r = 0; r < ND; r++) {
-                                double tt = 0.0;
-#pragma unroll
-                                for (int d = 0; d < ND; d++) tt = fma(f[d * NCU + j], X[r][d], tt);
-                                wrl[g + NGV * ((r + 1) + ND1 * (j + NCU * k))] = -tt;
-                            }
-                        }
-                        continue;
-                    }
-                    const double jf = sm.jacf[g];
-                    double sd[NCU], tcol[NCU];
-                    if (!GEN || A.conv_stab == 0) {
-#pragma unroll
-                        for (int j = 0; j < NCU; j++) {
-                            tcol[j] = k == j ? tau : 0.0;
-                            sd[j] = -tcol[j];
-                        }
-                    } else {
-                        // the Lax-Friedrichs or Roe tensor (ns_stab_point): the uh-derivative of
-                        // the stabilization term along this column, and column k of tau
-                        double nlq[ND], uv[NCU], sv[NCU];
-#pragma unroll
-                        for (int d = 0; d < ND; d++) nlq[d] = sm.nl[g + NA * d];
-#pragma unroll
-                        for (int m = 0; m < NCU; m++) uv[m] = ugf[g + NA * m];
-                        ns_stab_point<ND>(A.conv_stab, P, nlq, w, uv, k, sv, sd, tcol);
-                        if (k == 0)
-#pragma unroll
-                            for (int j = 0; j < NCU; j++) sm.fn[g + NA * j] += sv[j] * jf;
+                    for (int c = 0; c < NC; c++) {
+                        w[c].v = ugf[gg + NA * c];
+                        w[c].d[0] = (c == k) ? 1.0 : 0.0;
                     }
 #pragma unroll
-                    for (int j = 0; j < NCU; j++) {
-                        double dn = sd[j] * jf;
+                    for (int c = 0; c < NCH; c++) {
+                        uhd[c].v = uhg[gg + NA * c];
+                        uhd[c].d[0] = (NC + c == k) ? 1.0 : 0.0;
+                    }
+                    double nlq[ND];
 #pragma unroll
-                        for (int d = 0; d < ND; d++) dn = fma(f[d * NCU + j], X[0][d], dn);
-                        sl[NGF * NCH * NC + q + NGF * (j + NCH * k)] = dn;
-                        sl[q + NGF * (j + NCH * k)] = tcol[j] * jf;
+                    for (int d = 0; d < ND; d++) nlq[d] = sm.nl[gg + NA * d];
+                    const int ib = -bfe[fc] - 1;
+                    if (!ns_fbou_dual<ND, 1, GEN>(A.bcm[ib], P, A.bcs + (size_t)ib * NCH, nlq, w, uhd, fb,
+                                                  !A.inviscid, A.conv_stab, A.visc_model)) {
+                        for (int j = 0; j < NCH; j++) fb[j] = dc<1>(0.0);
+                    }
+                    const double jf = sm.jacf[gg];
+                    double* sl = fslb + fc * G::FSLP;
+#pragma unroll
+                    for (int j = 0; j < NCH; j++) {
+                        if (k == 0) fnb[gg + NA * j] = fb[j].v * jf;
+                        if (k < NC) sl[q + NGF * (j + NCH * k)] = fb[j].d[0] * jf;
+                        else sl[NGF * NCH * NC + q + NGF * (j + NCH * (k - NC))] = fb[j].d[0] * jf;
                     }
                 }
             }
+        };
+        if constexpr (TF) {
+        // 3xTF32 form: warp 0 factors M while the other warps evaluate the states at
+        // the points and the pointwise fluxes, which do not depend on M
+        if (warp == 0) {
+            cholesky_warp<NPV>(M, sm.rdg);
+        } else {
+            constexpr int NT1 = NT - 32;
+            const int tid1 = tid - 32;
+            states(tid1, NT1);
+            asm volatile("bar.sync 1, %0;" ::"r"(NT1) : "memory");
             // pointwise fluxes, 3xTF32 form: one work item per (point, differentiated
             // variable k); a one-derivative dual pass gives f and df/dw_k at that point.
-            if constexpr (TF)
             for (int t = tid1; t < (NGV + NA) * NC; t += NT1) {
                 using DD = Dual<1>;
                 const int p = t % (NGV + NA), k = t / (NGV + NA);
@@ -571,42 +465,139 @@ __global__ void __launch_bounds__(S::NT, 512 / S::NT) element_kernel(ElemArgs A)
                     }
                 }
             }
-            // boundary faces: fb and its Jacobians at their points (one item per point and variable)
-            if (bfe) {
-                for (int t = tid1; t < NFE * NGF * (NC + NCH); t += NT1) {
-                    const int fc = t / (NGF * (NC + NCH)), r = t % (NGF * (NC + NCH));
-                    if (bfe[fc] >= 0) continue;
-                    using DD = Dual<1>;
-                    const int q = r % NGF, k = r / NGF, gg = q + NGF * fc;
-                    DD w[NC], uhd[NCH], fb[NCH];
+            boundary_fluxes(tid1, NT1);
+        }
+        } else {
+        // FP64 form: warp 0 factors M while the other warps evaluate the states, then
+        // all threads the fluxes: a directional point is a (volume point, metric row)
+        // or a face point with its scaled normal; one item for its flux and u columns,
+        // one for its gradient columns.  (3D p=3: 46k cycles per element when each of
+        // the point's columns was an item of its own; bound by FP64 issue.)
+        if (warp == 0) cholesky_warp_rows<NPV>(M, sm.rdg);
+        else states(tid - 32, NT - 32);
+        __syncthreads();
+        const double gam = P[0], iRe = A.inviscid ? 0.0 : 1.0 / P[2], kappa = A.inviscid ? 0.0 : gam * iRe / P[3];
+        constexpr int NVD = NGV * ND, NDP = NVD + NA;
+        for (int t = tid; t < 2 * NDP; t += NT) {
+            const int p = t < NDP ? t : t - NDP;
+            const bool vol = p < NVD, upart = t < NDP;
+            const int g = vol ? p % NGV : p - NVD, r = p / NGV, fc = g / NGF, q = g % NGF;
+            double w[NC], X[ND];
 #pragma unroll
-                    for (int c = 0; c < NC; c++) {
-                        w[c].v = ugf[gg + NA * c];
-                        w[c].d[0] = (c == k) ? 1.0 : 0.0;
-                    }
+            for (int c = 0; c < NC; c++)
+                w[c] = vol ? ug[g + NGV * c] : ((c < NCU) ? uhg[g + NA * c] : ugf[g + NA * c]);
 #pragma unroll
-                    for (int c = 0; c < NCH; c++) {
-                        uhd[c].v = uhg[gg + NA * c];
-                        uhd[c].d[0] = (NC + c == k) ? 1.0 : 0.0;
-                    }
-                    double nlq[ND];
+            for (int d = 0; d < ND; d++) X[d] = vol ? sm.Xx[g + NGV * (d + ND * r)] : sm.nl[g + NA * d] * sm.jacf[g];
+            double mu = 1.0, dmu[NCU];
+            if constexpr (GEN) {
+                if (A.visc_model != 0 && !A.inviscid) {
+                    Dual<NCU> wd[NCU];
 #pragma unroll
-                    for (int d = 0; d < ND; d++) nlq[d] = sm.nl[gg + NA * d];
-                    const int ib = -bfe[fc] - 1;
-                    if (!ns_fbou_dual<ND, 1, GEN>(A.bcm[ib], P, A.bcs + (size_t)ib * NCH, nlq, w, uhd, fb,
-                                                  !A.inviscid, A.conv_stab, A.visc_model)) {
-                        for (int j = 0; j < NCH; j++) fb[j] = dc<1>(0.0);
+                    for (int c = 0; c < NCU; c++) {
+                        wd[c] = dc<NCU>(w[c]);
+                        wd[c].d[c] = 1.0;
                     }
-                    const double jf = sm.jacf[gg];
-                    double* sl = fslb + fc * G::FSLP;
+                    const Dual<NCU> m = ns_sutherland<ND, NCU>(P, wd);
+                    mu = m.v;
 #pragma unroll
-                    for (int j = 0; j < NCH; j++) {
-                        if (k == 0) fnb[gg + NA * j] = fb[j].v * jf;
-                        if (k < NC) sl[q + NGF * (j + NCH * k)] = fb[j].d[0] * jf;
-                        else sl[NGF * NCH * NC + q + NGF * (j + NCH * (k - NC))] = fb[j].d[0] * jf;
-                    }
+                    for (int c = 0; c < NCU; c++) dmu[c] = m.d[c];
                 }
             }
+            NsDir<ND> s;
+            ns_dir<ND>(gam, iRe, kappa, mu, w, X, s);
+            double* wv = wrl + g + NGV * (r + 1);
+            double* sl = fsl + fc * G::FSLP + q;
+            if (!upart) {
+                if (vol) {
+                    ns_dir_q<ND>(s, [&](int dq, int m, int j, double v) {
+                        wv[NGV * ND1 * (j + NCU * (NCU * (1 + dq) + m))] = -v;
+                    });
+                } else {
+                    ns_dir_q<ND>(s, [&](int dq, int m, int j, double v) {
+                        sl[NGF * (j + NCH * (NCU * (1 + dq) + m))] = v;
+                    });
+                    // the pairs that do not depend on the gradients
+#pragma unroll
+                    for (int dq = 0; dq < ND; dq++)
+#pragma unroll
+                        for (int z = NsPairs<ND>::DEP; z < NsPairs<ND>::ALL; z++) {
+                            int j, m;
+                            NsPairs<ND>::at(z, j, m);
+                            sl[NGF * (j + NCH * (NCU * (1 + dq) + m))] = 0.0;
+                        }
+                }
+                continue;
+            }
+            const double* dm = (GEN && A.visc_model != 0 && !A.inviscid) ? dmu : nullptr;
+            if (vol) {
+                ns_dir_u<ND>(
+                    gam, iRe, kappa, dm, s, [&](int j, double v) { sm.wrk[g + NGV * (r + 1 + ND1 * j)] = v; },
+                    [&](int k, int j, double v) { wv[NGV * ND1 * (j + NCU * k)] = -v; });
+                if (r == 0) {
+                    // the source and its derivative (row r = 0 of the pulled-back flux)
+                    const double jg = sm.jac[g];
+#pragma unroll
+                    for (int j = 0; j < NCU; j++) {
+                        double src = 0.0;
+                        if (tdep) {
+                            double tt = 0.0;
+#pragma unroll 4
+                            for (int a = 0; a < NPV; a++) tt = fma(T.shapvt[g + NGV * a], shu[a + NPV * j], tt);
+                            src = tt - w[j] * fc_u;
+                        }
+                        sm.wrk[g + NGV * ND1 * j] = src * jg;
+#pragma unroll
+                        for (int k = 0; k < NCU; k++)
+                            wrl[g + NGV * ND1 * (j + NCU * k)] = (tdep && k == j) ? fc_u * jg : 0.0;
+                    }
+                }
+                continue;
+            }
+            // fhat = F(uh, q).n + tau (u - uh)   (fhatDriver.cpp:54-236), times jacf, with
+            // the constant tensor here, Lax-Friedrichs or Roe below
+            const double jf = sm.jacf[g], tau = P[5];
+            double* slu = sl + NGF * NCH * NC;
+            if (!GEN || A.conv_stab == 0) {
+                ns_dir_u<ND>(
+                    gam, iRe, kappa, dm, s,
+                    [&](int j, double v) { sm.fn[g + NA * j] = fma(tau * jf, ugf[g + NA * j] - w[j], v); },
+                    [&](int k, int j, double v) { slu[NGF * (j + NCH * k)] = j == k ? v - tau * jf : v; });
+#pragma unroll
+                for (int k = 0; k < NCU; k++)
+#pragma unroll
+                    for (int j = 0; j < NCU; j++) sl[NGF * (j + NCH * k)] = j == k ? tau * jf : 0.0;
+            } else {
+                ns_dir_u<ND>(
+                    gam, iRe, kappa, dm, s, [&](int j, double v) { sm.fn[g + NA * j] = v; },
+                    [&](int k, int j, double v) { slu[NGF * (j + NCH * k)] = v; });
+            }
+        }
+        if (GEN && A.conv_stab != 0) {
+            // the stabilization term's derivative along uh_k and column k of the tensor,
+            // one item per (face point, k), added to what the items above wrote
+            __syncthreads();
+            for (int t = tid; t < NA * NCU; t += NT) {
+                const int g = t % NA, k = t / NA, fc = g / NGF, q = g % NGF;
+                const double jf = sm.jacf[g];
+                double nlq[ND], uhv[NCU], uv[NCU], sv[NCU], sd[NCU], tcol[NCU];
+#pragma unroll
+                for (int d = 0; d < ND; d++) nlq[d] = sm.nl[g + NA * d];
+#pragma unroll
+                for (int m = 0; m < NCU; m++) {
+                    uhv[m] = uhg[g + NA * m];
+                    uv[m] = ugf[g + NA * m];
+                }
+                ns_stab_point<ND>(A.conv_stab, P, nlq, uhv, uv, k, sv, sd, tcol);
+                double* sl = fsl + fc * G::FSLP + q;
+#pragma unroll
+                for (int j = 0; j < NCU; j++) {
+                    if (k == 0) sm.fn[g + NA * j] += sv[j] * jf;
+                    sl[NGF * NCH * NC + NGF * (j + NCH * k)] += sd[j] * jf;
+                    sl[NGF * (j + NCH * k)] = tcol[j] * jf;
+                }
+            }
+        }
+        boundary_fluxes(tid, NT);
         }
         __syncthreads();
         // M^-1 C and M^-1 E in place, one column per thread
@@ -1031,7 +1022,7 @@ __global__ void __launch_bounds__(S::NT, 512 / S::NT) element_kernel(ElemArgs A)
                             if (rv[u] && a < NPV) {
                                 const int j = jj[u], ip = ipp[u], m = mm[u];
                                 if (store) Ke[j + NCH * (fc * NPF + ip) + (size_t)NB * (a + NPV * m)] = acc[u][b][h];
-                                if (liftD) atomicAdd(&De[inode[u] + NPV * (j + NCU * (a + NPV * m))], acc[u][b][h]);
+                                if (liftD && acc[u][b][h] != 0.0) atomicAdd(&De[inode[u] + NPV * (j + NCU * (a + NPV * m))], acc[u][b][h]);
                             }
                         }
                 // H in two column halves: half the accumulators live at a time

@@ -244,9 +244,9 @@ __device__ __forceinline__ void qmatrices_factored(const Tables& T, double fc_q,
 }
 
 // Lower Cholesky of M (npv x npv) in place by one warp, right-looking: lane i
-// holds row i in registers, so a column costs one square root, one division and
-// one shuffle per entry of its row instead of a dot product over the columns
-// before it; rdg receives the reciprocals of the diagonal.
+// holds row i in registers, so a column costs one reciprocal square root and one
+// shuffle per entry of its row instead of a dot product over the columns before
+// it; rdg receives the reciprocals of the diagonal.
 template <int NPV>
 __device__ __forceinline__ void cholesky_warp_rows(double* a, double* rdg) {
     static_assert(NPV <= 32, "one row per lane");
@@ -256,9 +256,9 @@ __device__ __forceinline__ void cholesky_warp_rows(double* a, double* rdg) {
     for (int k = 0; k < NPV; k++) r[k] = a[row + NPV * k];
 #pragma unroll
     for (int j = 0; j < NPV; j++) {
-        const double l = sqrt(__shfl_sync(0xffffffffu, r[j], j)), inv = 1.0 / l;
+        const double inv = rsqrt(__shfl_sync(0xffffffffu, r[j], j));
         if (lane == j) rdg[j] = inv;
-        r[j] = lane == j ? l : r[j] * inv;
+        r[j] *= inv;
 #pragma unroll
         for (int k = j + 1; k < NPV; k++) r[k] = fma(-r[j], __shfl_sync(0xffffffffu, r[j], k), r[k]);
     }

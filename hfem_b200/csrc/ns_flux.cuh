@@ -170,173 +170,157 @@ __device__ __forceinline__ void ns_flux_dual(const double* __restrict__ param, c
     }
 }
 
-// The flux and its Jacobian columns at one point without dual numbers, for the
-// element kernel's FP64 form.  (A dual pass computes every product with a zero
-// derivative, and all columns' values again.)  ns_point holds what the columns
-// share; f[d * ncu + j], fd[d * ncu + j] as ns_flux_dual's value and derivative.
+// The flux through one direction X, F(w).X = sum_d f_d X_d, and its Jacobian
+// columns without dual numbers, for the element kernel's FP64 form: X is a row of
+// the volume point's metric or the face point's scaled normal, so what is formed
+// is what the element integrals need, and no product with a zero derivative.
+// NsDir holds the terms that the columns share.
 template <int ND>
-struct NsPoint {
-    double ir, v[ND], p, E, rho;
-    double G[ND][ND];       // G[d][i] = dv_i / dx_d
-    double q0[ND], qE[ND];  // gradients of rho and rho E
-    double div, mu;
+struct NsDir {
+    double ir, rho, E, p, v[ND], v2;
+    double X[ND], q0[ND];
+    double Vn, Q0n, qEn, div;   // v.X, grad(rho).X, grad(rho E).X, div v
+    double Gn[ND], Hn[ND];      // sum_d dv_i/dx_d X_d,  sum_d dv_d/dx_i X_d
+    double a, kap;              // mu / Re, mu gamma / (Re Pr); 0 for the Euler flux
 };
 
-template <int ND, bool GEN = false>
-__device__ __forceinline__ NsPoint<ND> ns_point(const double* __restrict__ param, const double* w, int visc_model) {
+// iRe = 1/Re and kappa = gamma/(Re Pr), both 0 for the Euler flux
+template <int ND>
+__device__ __forceinline__ void ns_dir(double gam, double iRe, double kappa, double mu, const double* w,
+                                       const double* X, NsDir<ND>& s) {
     constexpr int NCU = ND + 2;
-    NsPoint<ND> s;
     s.rho = w[0];
     s.E = w[ND + 1];
     s.ir = 1.0 / w[0];
-    double ke = 0.0;
+    s.v2 = s.Vn = s.Q0n = s.qEn = s.div = 0.0;
 #pragma unroll
     for (int i = 0; i < ND; i++) {
+        s.X[i] = X[i];
         s.v[i] = w[1 + i] * s.ir;
-        ke = fma(s.v[i], w[1 + i], ke);
+        s.v2 = fma(s.v[i], s.v[i], s.v2);
+        s.Vn = fma(s.v[i], X[i], s.Vn);
+        s.q0[i] = w[NCU * (1 + i)];
+        s.Q0n = fma(s.q0[i], X[i], s.Q0n);
+        s.qEn = fma(w[NCU * (1 + i) + ND + 1], X[i], s.qEn);
+        s.Gn[i] = s.Hn[i] = 0.0;
     }
-    s.p = (param[0] - 1.0) * (s.E - 0.5 * ke);
-    s.div = 0.0;
+    s.p = (gam - 1.0) * fma(-0.5 * s.rho, s.v2, s.E);
 #pragma unroll
-    for (int d = 0; d < ND; d++) {
-        const double* q = w + NCU * (1 + d);
-        s.q0[d] = q[0];
-        s.qE[d] = q[ND + 1];
-#pragma unroll
-        for (int i = 0; i < ND; i++) s.G[d][i] = (q[1 + i] - s.v[i] * q[0]) * s.ir;
-        s.div += s.G[d][d];
-    }
-    s.mu = 1.0;
-    if constexpr (GEN) {
-        if (visc_model != 0) {
-            Dual<1> wd[NCU];
-#pragma unroll
-            for (int c = 0; c < NCU; c++) wd[c] = dc<1>(w[c]);
-            s.mu = ns_sutherland<ND, 1>(param, wd).v;
-        }
-    }
-    return s;
-}
-
-// the flux
-template <int ND>
-__device__ __forceinline__ void ns_flux_value(const double* __restrict__ param, const NsPoint<ND>& s, double* f,
-                                              bool viscous) {
-    constexpr int NCU = ND + 2;
-    const double a = s.mu / param[2], kap = s.mu * (param[0] / (param[2] * param[3]));
-#pragma unroll
-    for (int d = 0; d < ND; d++) {
-        f[d * NCU] = s.rho * s.v[d];
-        double fe = (s.E + s.p) * s.v[d], vg = 0.0;
+    for (int d = 0; d < ND; d++)
 #pragma unroll
         for (int i = 0; i < ND; i++) {
-            double t = s.G[d][i] + s.G[i][d];
-            if (i == d) t -= (2.0 / 3.0) * s.div;
-            t = viscous ? a * t : 0.0;
-            f[d * NCU + 1 + i] = fma(s.rho * s.v[i], s.v[d], t) + (i == d ? s.p : 0.0);
-            fe = fma(t, s.v[i], fe);
-            vg = fma(s.v[i], s.G[d][i], vg);
+            const double g = fma(-s.v[i], s.q0[d], w[NCU * (1 + d) + 1 + i]) * s.ir;   // dv_i/dx_d
+            s.Gn[i] = fma(g, X[d], s.Gn[i]);
+            s.Hn[d] = fma(g, X[i], s.Hn[d]);
+            if (i == d) s.div += g;
         }
-        const double heat = s.qE[d] * s.ir - s.E * s.q0[d] * (s.ir * s.ir) - vg;
-        f[d * NCU + ND + 1] = viscous ? fma(kap, heat, fe) : fe;
-    }
+    s.a = iRe * mu;
+    s.kap = kappa * mu;
 }
 
-// column k < ncu: the derivative along the conserved variable u_k
-template <int ND, bool GEN = false>
-__device__ __forceinline__ void ns_flux_ucol(const double* __restrict__ param, const NsPoint<ND>& s, const double* w,
-                                             int k, double* fd, bool viscous, int visc_model) {
-    constexpr int NCU = ND + 2;
-    const double g1 = param[0] - 1.0, iRe = 1.0 / param[2], kappa = param[0] / (param[2] * param[3]);
-    const double drho = k == 0 ? 1.0 : 0.0, dE = k == ND + 1 ? 1.0 : 0.0;
-    double dm[ND], dv[ND], dke = 0.0;
+// The flux F.X and its columns along the conserved variables: val(j, F_j) and
+// col(k, j, dF_j/du_k).  dmu[k] = dmu/du_k (GEN; NULL: constant viscosity).
+template <int ND, class Val, class Col>
+__device__ __forceinline__ void ns_dir_u(double gam, double iRe, double kappa, const double* dmu, const NsDir<ND>& s,
+                                         Val val, Col col) {
+    const double g1 = gam - 1.0, ir2 = s.ir * s.ir, c23 = 2.0 / 3.0;
+    double sh[ND], tn[ND], vt = 0.0, vG = 0.0;       // stress without mu/Re, stress, v.stress, v.Gn
 #pragma unroll
     for (int i = 0; i < ND; i++) {
-        dm[i] = k == 1 + i ? 1.0 : 0.0;
-        dv[i] = (dm[i] - s.v[i] * drho) * s.ir;
-        dke = fma(dv[i], w[1 + i], fma(s.v[i], dm[i], dke));
+        sh[i] = s.Gn[i] + s.Hn[i] - c23 * s.div * s.X[i];
+        tn[i] = s.a * sh[i];
+        vt = fma(s.v[i], tn[i], vt);
+        vG = fma(s.v[i], s.Gn[i], vG);
     }
-    const double dp = g1 * (dE - 0.5 * dke);
-    double dG[ND][ND], ddiv = 0.0;
+    const double heat = s.qEn * s.ir - s.E * s.Q0n * ir2 - vG, EP = s.E + s.p;
+    val(0, s.rho * s.Vn);
 #pragma unroll
-    for (int d = 0; d < ND; d++) {
+    for (int i = 0; i < ND; i++) val(1 + i, fma(s.rho * s.v[i], s.Vn, fma(s.p, s.X[i], tn[i])));
+    val(ND + 1, fma(EP, s.Vn, fma(s.kap, heat, vt)));
+    // what a viscosity derivative adds to column k
+    auto visc = [&](int k, int i) { return dmu ? iRe * dmu[k] * sh[i] : 0.0; };
+    auto visc_e = [&](int k) {
+        if (!dmu) return 0.0;
+        double t = kappa * dmu[k] * heat;
 #pragma unroll
-        for (int i = 0; i < ND; i++) dG[d][i] = -(dv[i] * s.q0[d] + s.G[d][i] * drho) * s.ir;
-        ddiv += dG[d][d];
-    }
-    double dmu = 0.0;
-    if constexpr (GEN) {
-        if (visc_model != 0) {
-            Dual<1> wd[NCU];
+        for (int i = 0; i < ND; i++) t = fma(iRe * dmu[k] * s.v[i], sh[i], t);
+        return t;
+    };
+    // along rho: dv = -v/rho
+    {
+        double vq = 0.0;
 #pragma unroll
-            for (int c = 0; c < NCU; c++) {
-                wd[c].v = w[c];
-                wd[c].d[0] = c == k ? 1.0 : 0.0;
-            }
-            dmu = ns_sutherland<ND, 1>(param, wd).d[0];
-        }
-    }
-    const double ir2 = s.ir * s.ir;
-#pragma unroll
-    for (int d = 0; d < ND; d++) {
-        fd[d * NCU] = dm[d];
-        double fe = fma(dE + dp, s.v[d], (s.E + s.p) * dv[d]), vg = 0.0, dvg = 0.0;
+        for (int i = 0; i < ND; i++) vq = fma(s.v[i], s.q0[i], vq);
+        const double dVn = -s.Vn * s.ir, dp = 0.5 * g1 * s.v2, ddiv = fma(vq, s.ir, -s.div) * s.ir;
+        double et = 0.0, vdG = 0.0;
+        col(0, 0, 0.0);
 #pragma unroll
         for (int i = 0; i < ND; i++) {
-            double t = s.G[d][i] + s.G[i][d], dt = dG[d][i] + dG[i][d];
-            if (i == d) {
-                t -= (2.0 / 3.0) * s.div;
-                dt -= (2.0 / 3.0) * ddiv;
-            }
-            if constexpr (GEN) dt = fma(s.mu, dt, dmu * t);
-            dt = viscous ? iRe * dt : 0.0;
-            t = viscous ? iRe * (GEN ? s.mu * t : t) : 0.0;
-            fd[d * NCU + 1 + i] = fma(dm[i], s.v[d], fma(w[1 + i], dv[d], dt)) + (i == d ? dp : 0.0);
-            fe = fma(dt, s.v[i], fma(t, dv[i], fe));
-            vg = fma(s.v[i], s.G[d][i], vg);
-            dvg = fma(dv[i], s.G[d][i], fma(s.v[i], dG[d][i], dvg));
+            const double dG = fma(s.v[i] * s.ir, s.Q0n, -s.Gn[i]) * s.ir;
+            const double dH = fma(s.q0[i], s.Vn * s.ir, -s.Hn[i]) * s.ir;
+            const double dt = fma(s.a, dG + dH - c23 * ddiv * s.X[i], visc(0, i));
+            // stress: v.dt + dv.t; heat: -(dv.Gn + v.dGn)
+            et = fma(s.v[i], fma(-tn[i], s.ir, dt), et);
+            vdG = fma(s.v[i], fma(-s.Gn[i], s.ir, dG), vdG);
+            col(0, 1 + i, fma(s.rho * s.v[i], dVn, fma(dp, s.X[i], dt)));
         }
-        double dheat = -s.qE[d] * ir2 * drho - dE * s.q0[d] * ir2 + 2.0 * s.E * s.q0[d] * ir2 * s.ir * drho - dvg;
-        if constexpr (GEN) {
-            const double heat = s.qE[d] * s.ir - s.E * s.q0[d] * ir2 - vg;
-            dheat = fma(s.mu, dheat, dmu * heat);
-        }
-        fd[d * NCU + ND + 1] = viscous ? fma(kappa, dheat, fe) : fe;
+        const double dheat = fma(-s.qEn, ir2, 2.0 * s.E * s.Q0n * ir2 * s.ir) - vdG;
+        double mu_e = dmu ? kappa * dmu[0] * heat : 0.0;
+        col(0, ND + 1, fma(dp, s.Vn, fma(EP, dVn, fma(s.kap, dheat, et + mu_e))));
     }
+    // along the momentum: dv_l = 1/rho
+#pragma unroll
+    for (int l = 0; l < ND; l++) {
+        const double dVn = s.X[l] * s.ir, dp = -g1 * s.v[l], ddiv = -s.q0[l] * ir2, dGl = -s.Q0n * ir2;
+        double et = tn[l] * s.ir;
+        col(1 + l, 0, s.X[l]);
+#pragma unroll
+        for (int i = 0; i < ND; i++) {
+            const double dt = fma(s.a, (i == l ? dGl : 0.0) - s.q0[i] * dVn * s.ir - c23 * ddiv * s.X[i], visc(1 + l, i));
+            et = fma(s.v[i], dt, et);
+            col(1 + l, 1 + i, fma(s.rho * s.v[i], dVn, fma(dp, s.X[i], dt)) + (i == l ? s.Vn : 0.0));
+        }
+        const double dheat = -fma(s.Gn[l], s.ir, s.v[l] * dGl);
+        double mu_e = dmu ? kappa * dmu[1 + l] * heat : 0.0;
+        col(1 + l, ND + 1, fma(dp, s.Vn, fma(EP, dVn, fma(s.kap, dheat, et + mu_e))));
+    }
+    // along the energy
+    col(ND + 1, 0, 0.0);
+#pragma unroll
+    for (int i = 0; i < ND; i++) col(ND + 1, 1 + i, fma(g1, s.X[i], visc(ND + 1, i)));
+    col(ND + 1, ND + 1, fma(gam, s.Vn, fma(-s.kap, s.Q0n * ir2, visc_e(ND + 1))));
 }
 
-// The derivative along q_{dq,m}, the gradient of variable m in direction dq: the
-// viscous flux is linear in q, so the column is the flux of the unit gradient,
-// g_i = dv_i/dx_dq with its stress and heat terms.  The mass flux does not depend
-// on q, and the momentum fluxes not on q_{dq,nd+1}: those entries are zero
-// (NsPairs).
-template <int ND>
-__device__ __forceinline__ void ns_flux_qcol(const double* __restrict__ param, const NsPoint<ND>& s, int dq, int m,
-                                             double* fd, bool viscous) {
-    constexpr int NCU = ND + 2;
-    const double a = viscous ? s.mu / param[2] : 0.0;
-    const double kap = viscous ? s.mu * (param[0] / (param[2] * param[3])) : 0.0;
-    double g[ND], gd = 0.0, vg = 0.0;
+// The columns along the gradients: col(dq, m, j, dF_j/dq_{dq,m}) for the pairs
+// (j, m) that depend on them (NsPairs); the flux is linear in q, so a column is
+// the flux of the unit gradient.
+template <int ND, class Col>
+__device__ __forceinline__ void ns_dir_q(const NsDir<ND>& s, Col col) {
+    const double ai = s.a * s.ir, ki = s.kap * s.ir, c23 = 2.0 / 3.0;
 #pragma unroll
-    for (int i = 0; i < ND; i++) {
-        g[i] = m == 0 ? -s.v[i] * s.ir : (m == i + 1 ? s.ir : 0.0);
-        if (i == dq) gd = g[i];
-        vg = fma(s.v[i], g[i], vg);
-    }
-    const double heat = (m == ND + 1 ? s.ir : (m == 0 ? -s.E * s.ir * s.ir : 0.0)) - vg;
+    for (int dq = 0; dq < ND; dq++) {
+        const double X = s.X[dq];
+        // m = 0: g_i = -v_i/rho
 #pragma unroll
-    for (int d = 0; d < ND; d++) {
-        fd[d * NCU] = 0.0;
-        double fe = 0.0;
+        for (int i = 0; i < ND; i++)
+            col(dq, 0, 1 + i, -ai * (fma(s.v[i], X, -c23 * s.v[dq] * s.X[i]) + (i == dq ? s.Vn : 0.0)));
+        col(dq, 0, ND + 1, fma(-ai, fma(s.v2, X, (1.0 - c23) * s.v[dq] * s.Vn), ki * fma(-s.E, s.ir, s.v2) * X));
+        // m = 1 + l: g_l = 1/rho
 #pragma unroll
-        for (int i = 0; i < ND; i++) {
-            double t = (d == dq ? g[i] : 0.0) + (i == dq ? g[d] : 0.0);
-            if (i == d) t -= (2.0 / 3.0) * gd;
-            t *= a;
-            fd[d * NCU + 1 + i] = t;
-            fe = fma(t, s.v[i], fe);
+        for (int l = 0; l < ND; l++) {
+#pragma unroll
+            for (int i = 0; i < ND; i++) {
+                double t = 0.0;
+                if (i == l) t = X;
+                if (i == dq) t += s.X[l];
+                if (l == dq) t -= c23 * s.X[i];
+                col(dq, 1 + l, 1 + i, ai * t);
+            }
+            double e = fma(s.v[l], X, s.v[dq] * s.X[l]);
+            if (l == dq) e = fma(-c23, s.Vn, e);
+            col(dq, 1 + l, ND + 1, fma(ai, e, -ki * s.v[l] * X));
         }
-        fd[d * NCU + ND + 1] = d == dq ? fma(kap, heat, fe) : fe;
+        col(dq, ND + 1, ND + 1, ki * X);
     }
 }
 
