@@ -435,8 +435,8 @@ ScatterArgs scatter_args(hfem_ctx* c) {
     return s;
 }
 
-// The interior-face lift D += P K (src = K, n columns) or F += P H (src = H,
-// nb columns) applied by the condensation kernels (lift.cuh).
+// The interior-face lift F += P H (src = H, nb columns), applied as F is loaded by
+// the fused condensation, or by lift_F ahead of the others (lift.cuh).
 LiftArgs lift_args(hfem_ctx* c, const double* src, int cols) {
     LiftArgs L;
     L.src = src;
@@ -450,7 +450,12 @@ LiftArgs lift_args(hfem_ctx* c, const double* src, int cols) {
     return L;
 }
 
-// F += P H (interior faces) in place, ahead of the condensation kernels.
+FusedArgs fused_args(hfem_ctx* c) {
+    return FusedArgs{c->dims.ne, c->D, c->F, c->K, c->H, c->DinvF, c->DinvRu, c->Rh, lift_args(c, nullptr, c->nb)};
+}
+
+// F += P H (interior faces) in place, ahead of the batched GEMMs and the
+// tensor-core condensation.
 int lift_F(hfem_ctx* c) {
     Timed t(c, "lift_F");
     const long long cols = (long long)c->dims.ne * c->nb;
@@ -503,12 +508,12 @@ int enqueue_assembly(hfem_ctx* c, bool matrix) {
             c->L->inverse(dim3(c->grid_inv), c->stream, ne, c->D, c->Ru, c->DinvRu, c->info);
             if ((rc = check_launch(c, "inverse"))) return rc;
         }
-        if (c->precision != 1 && c->g1_sel < 0 && c->g2_sel < 0) {
-            // both products in one kernel (tilings chosen by hfem_set_gemm_tiles
+        const bool fused = c->precision != 1 && c->g1_sel < 0 && c->g2_sel < 0;
+        if (fused) {
+            // both products and Rh in one kernel (tilings chosen by hfem_set_gemm_tiles
             // or hfem_autotune run the two batched GEMMs instead)
-            if ((rc = lift_F(c))) return rc;
             Timed t(c, "schur_fused");
-            c->L->schur_fused(c->stream, ne, c->D, c->F, c->K, c->H, c->DinvF);
+            c->L->schur_fused(c->stream, fused_args(c));
             if ((rc = check_launch(c, "schur_fused"))) return rc;
         } else if (c->precision != 1) {
             const GemmLaunch& g1 = c->g1_sel >= 0 ? gemm_candidates()[c->g1_sel] : c->L->g1;
@@ -527,13 +532,16 @@ int enqueue_assembly(hfem_ctx* c, bool matrix) {
                 if ((rc = check_launch(c, "gemm_schur"))) return rc;
             }
         } else {
+            // (lifting while F is staged, as the fused kernel does, was slower here: one CTA
+            // per SM waits on the gathers of H; 2.43 against 1.51 + 0.58 ms, 4,374
+            // tetrahedra p = 3)
             if ((rc = lift_F(c))) return rc;
             Timed t(c, "schur_tc");
             SchurTcArgs ta{ne, c->D, c->F, c->K, c->H, c->DinvF, c->tc_err};
             c->L->schur_tc(dim3(c->grid_tc), c->L->tc_smem, c->stream, ta);
             if ((rc = check_launch(c, "schur_tc"))) return rc;
         }
-        {
+        if (!fused) {
             Timed t(c, "gemv_Rh");
             batched_dgemv_kernel<<<sms(c->device) * 8, 256, 0, c->stream>>>(ne, nb, n, -1.0, c->K, (long long)nb * n,
                                                                            c->DinvRu, n, c->Rh, nb);
@@ -2040,17 +2048,30 @@ int hfem_autotune(hfem_ctx* c, int reps, int* best, double* ms) {
             if (ms) ms[which * cand.size() + k] = per;
             if (per < bt[which]) bt[which] = per, bi[which] = (int)k;
         }
-    // the fused kernel does both products: kept when it beats the best pair
+    // the pair needs the lift pass in front of it
+    double lift = 0.0;
     {
-        c->L->schur_fused(c->stream, ne, c->D, c->F, c->K, c->H, c->DinvF);   // warm-up
-        if ((rc = check_launch(c, "autotune"))) return rc;
+        if ((rc = lift_F(c))) return rc;                   // warm-up
         CK(cudaEventRecord(e0, c->stream));
-        for (int r = 0; r < reps; r++) c->L->schur_fused(c->stream, ne, c->D, c->F, c->K, c->H, c->DinvF);
+        for (int r = 0; r < reps; r++)
+            if ((rc = lift_F(c))) return rc;
         CK(cudaEventRecord(e1, c->stream));
         CK(cudaEventSynchronize(e1));
         float t = 0.f;
         CK(cudaEventElapsedTime(&t, e0, e1));
-        if ((double)t / reps <= bt[0] + bt[1]) bi[0] = bi[1] = -1;
+        lift = (double)t / reps;
+    }
+    // the fused kernel does both products and the lift: kept when it beats them
+    {
+        c->L->schur_fused(c->stream, fused_args(c));       // warm-up
+        if ((rc = check_launch(c, "autotune"))) return rc;
+        CK(cudaEventRecord(e0, c->stream));
+        for (int r = 0; r < reps; r++) c->L->schur_fused(c->stream, fused_args(c));
+        CK(cudaEventRecord(e1, c->stream));
+        CK(cudaEventSynchronize(e1));
+        float t = 0.f;
+        CK(cudaEventElapsedTime(&t, e0, e1));
+        if ((double)t / reps <= bt[0] + bt[1] + lift) bi[0] = bi[1] = -1;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -2402,7 +2423,6 @@ extern "C" int hfem_condense_noalloc(const hfem_dims* dims, const double* shapvt
         gi = std::min(d.ne, G.inv);
     }
     cudaStream_t st = (cudaStream_t)stream;
-    const int n = L->npv * (d.nd + 2), nb = (d.nd + 2) * d.npf * (d.nd + 1);
 
     ElemArgs a;
     a.T = Tables{shapvt, shapvg, shapvgdotshapvl, shapft, shapfg, shapfgdotshapfc, perm};
@@ -2431,20 +2451,14 @@ extern "C" int hfem_condense_noalloc(const hfem_dims* dims, const double* shapvt
     L->inverse(dim3(gi), st, d.ne, D, DinvRu, DinvRu, info);
     if (cudaGetLastError() != cudaSuccess) return HFEM_E_CUDA;
     LiftArgs lh;
-    lh.src = H;
     lh.perm = perm;
     lh.bf = bf;
     lh.npv = d.npv;
     lh.npf = d.npf;
     lh.nfe = d.nfe;
     lh.nch = d.nd + 2;
-    lh.cols = nb;
-    // F (formed in the DinvF buffer) += P H, then the condensation in place
-    lift_inplace_kernel<<<sms(dev) * 8, 32 * LIFT_WARPS, 0, st>>>(d.ne, n, lh, DinvF);
-    if (cudaGetLastError() != cudaSuccess) return HFEM_E_CUDA;
-    L->schur_fused(st, d.ne, D, DinvF, K, H, DinvF);
-    if (cudaGetLastError() != cudaSuccess) return HFEM_E_CUDA;
-    batched_dgemv_kernel<<<sms(dev) * 8, 256, 0, st>>>(d.ne, nb, n, -1.0, K, (long long)nb * n, DinvRu, n, Rh, nb);
+    // the lift, the condensation (in place: F was formed in the DinvF buffer) and Rh
+    L->schur_fused(st, FusedArgs{d.ne, D, DinvF, K, H, DinvF, DinvRu, Rh, lh});
     if (cudaGetLastError() != cudaSuccess) return HFEM_E_CUDA;
     return 0;
 }

@@ -8,6 +8,7 @@
 #include "elem_kernels.cuh"
 #include "schur_kernels.cuh"
 #include "schur_tc.cuh"
+#include "schur_fused.cuh"
 
 namespace hfem {
 
@@ -68,7 +69,7 @@ struct Launch {
     int tc_tmem;                // tensor-memory columns of one tensor-core Schur CTA
     const void* tc_fn;
     void (*scatter_h)(dim3, cudaStream_t, const ScatterArgs&);
-    void (*schur_fused)(cudaStream_t, int, const double*, const double*, const double*, double*, double*);
+    void (*schur_fused)(cudaStream_t, const FusedArgs&);
     size_t fused_smem;
     const void* fused_fn;
 };

@@ -5,11 +5,15 @@
 // to the element node that carries the face dof, so
 //   D = D_vol + P K,   F = F_vol + P H,
 // with P the node <- face-dof incidence given by perm.  The element kernel
-// writes D (lifted), F_vol and the trace rows K, H; lift_inplace_kernel adds
-// P H to F between the element kernel and the condensation, one coalesced pass
-// instead of reductions in L2 from the element kernel.  Boundary faces are
-// lifted by the element kernel itself (their trace rows take the boundary flux
-// while their element rows keep fhat), so the lift here skips them.
+// writes D (lifted), F_vol and the trace rows K, H.  The fused FP64
+// condensation adds P H when it loads F: a thread keeps one row of F for all
+// columns, so its (at most nd) source rows of H are found once (lift_row), and the
+// entries of H it gathers are the columns the same CTA reads again as the
+// product's accumulators.  lift_inplace_kernel is the pass on its own, ahead of
+// the batched GEMMs and the tensor-core condensation (3D p=3: 640 KB per element
+// through HBM, 6.4 of 89 ms per pass over 48,000 elements when every path took it).  Boundary faces
+// are lifted by the element kernel itself (their trace rows take the boundary
+// flux while their element rows keep fhat), so the lift here skips them.
 //
 // Row r = i + npv j of D (or F) with column c receives, for every interior face
 // dof fdof of node i in increasing order (the order of the reference's face
@@ -43,6 +47,35 @@ __device__ __forceinline__ void lift_table(const LiftArgs& L, LiftTable& t) {
             if (L.perm[f] == i && c < LIFT_MAXINC) t.f[i * LIFT_MAXINC + c++] = f;
         t.n[i] = c;
     }
+}
+
+// The rows of H (or K) whose entries row `row` of element e receives, ascending
+// (the order of the reference's face loop); -1: none.
+struct LiftRow {
+    int s[LIFT_MAXINC];
+};
+__device__ __forceinline__ LiftRow lift_row(const LiftArgs& L, int e, int row) {
+    LiftRow r;
+#pragma unroll
+    for (int q = 0; q < LIFT_MAXINC; q++) r.s[q] = -1;
+    const int i = row % L.npv, j = row / L.npv;
+    int c = 0;
+#pragma unroll 8
+    for (int f = 0; f < L.npf * L.nfe; f++) {
+        if (L.perm[f] != i || (L.bf && L.bf[(size_t)e * L.nfe + f / L.npf] < 0)) continue;
+#pragma unroll
+        for (int q = 0; q < LIFT_MAXINC; q++)
+            if (q == c) r.s[q] = j + L.nch * f;
+        c++;
+    }
+    return r;
+}
+// v plus those entries of one column of H
+__device__ __forceinline__ double lift_add_row(const LiftRow& r, const double* hcol, double v) {
+#pragma unroll
+    for (int q = 0; q < LIFT_MAXINC; q++)
+        if (r.s[q] >= 0) v += hcol[r.s[q]];
+    return v;
 }
 
 // v plus the lifted trace entries of row `row` of element e, one column; hs is

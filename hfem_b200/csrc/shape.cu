@@ -5,8 +5,6 @@
 #include "launch.cuh"
 #include "elem_kernel.cuh"
 #include "inverse_blocked.cuh"
-#include "lift.cuh"
-#include "schur_fused.cuh"
 
 namespace hfem {
 
@@ -53,12 +51,11 @@ struct FusedPick {
     using Cfg = FusedCfg<S::N, S::NB, BN, NW>;
 };
 template <class S>
-void launch_schur_fused(cudaStream_t st, int ne, const double* Dinv, const double* F, const double* K, double* H,
-                        double* DinvF) {
-    static_assert(S::NB <= LIFT_MAXNB, "the lift stages one column of H per warp");
+void launch_schur_fused(cudaStream_t st, const FusedArgs& a) {
+    static_assert(S::NB <= LIFT_MAXNB, "lift_inplace_kernel stages one column of H per warp");
     using P = FusedPick<S>;
     schur_fused_kernel<S::N, S::NB, P::BN, P::NW>
-        <<<(unsigned)(ne * P::Cfg::STRIPS), P::Cfg::THREADS, P::Cfg::SMEM, st>>>(ne, Dinv, F, K, H, DinvF);
+        <<<(unsigned)(a.ne * P::Cfg::STRIPS), P::Cfg::THREADS, P::Cfg::SMEM, st>>>(a);
 }
 
 template <class S>
