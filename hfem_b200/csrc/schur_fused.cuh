@@ -2,19 +2,22 @@
 //   X = D^-1 (F + P H)  (n x nb, written out as DinvF),  H <- H - K X  and
 //   Rh <- Rh - K (D^-1 Ru),
 // on the FP64 tensor cores (mma.sync m8n8k4 f64).  One CTA per (element, strip
-// of BN columns of F / DinvF / H): the strip of X never leaves shared memory
-// between the two products.  A operands (D^-1, then K in row chunks) stream
-// through a 2-stage cp.async ring in k tiles of 20; the B operand (the F strip,
-// then the X strip) sits in shared memory whole.  Warp w owns m-tiles w, w+NW,
-// ... of every job and all BN/8 n-tiles.  H's accumulators start from H.
-// P H is the interior-face lift (lift.cuh), added as the F strip is loaded; the
-// CTA of strip 0 also forms K (D^-1 Ru) from the K tiles in its ring (as kernels
-// of their own these took 1.76 and 0.41 ms beside this one's 7.07 on 13,182
-// tetrahedra p = 3).
+// of BN columns of F / DinvF / H): the strip of F, then of -X, is the B operand in
+// shared memory.  A warp owns row tiles (8 rows, all BN/8 column tiles) and reads
+// its A fragments (D^-1, then K: no other warp needs them) straight from global
+// memory, PD k-steps ahead, so the products run without staging, barriers or a
+// scaling of A; the strips of an element share A in L2.
+// P H is the interior-face lift (lift.cuh), added as the F strip is loaded; strip 0
+// also forms K (D^-1 Ru) from its A fragments.
 // DinvF may be F itself: a CTA has its whole F strip in shared memory before it
 // writes the X strip over it, and strips are disjoint.
+// Bound by the FP64 tensor pipe (3D p=3: 24.4k DMMAs per element, 16.4 ms for
+// 48,000 at the measured 37 TFLOP/s).  13,182 tetrahedra p = 3: 8.27 -> 6.19 ms
+// (21.9 TFLOP/s algorithmic) against A tiles staged through a cp.async ring with a
+// barrier per 20 columns and alpha A formed for every fragment.
 #pragma once
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "lift.cuh"
 #include "schur_kernels.cuh"
 
@@ -22,21 +25,26 @@ namespace hfem {
 
 template <int N, int NB, int BN, int NW>
 struct FusedCfg {
-    static constexpr int BK = 20;
-    static constexpr int MT = (N + 7) / 8;                 // m-tiles per job (rows of D^-1, or a chunk of K)
-    static constexpr int BM = 8 * MT;
-    static constexpr int NTN = BN / 8;                     // n-tiles
-    static constexpr int KT = (N + BK - 1) / BK;           // k tiles
-    static constexpr int KP = KT * BK;                     // padded k extent (rows of the B strip)
-    static constexpr int LDA = ((BM + 11) / 16) * 16 + 4;  // == 4 (mod 16)
-    static constexpr int LDB = ((KP + 11) / 16) * 16 + 4;  // == 4 (mod 16)
-    static constexpr int MPW = (MT + NW - 1) / NW;         // m-tiles per warp
-    static constexpr int CHUNKS = (NB + BM - 1) / BM;      // row chunks of K / H
+    static constexpr int MT = (N + 7) / 8;                 // row tiles of X
+    static constexpr int MTH = (NB + 7) / 8;               // row tiles of H
+    static constexpr int NTN = BN / 8;                     // column tiles
+    static constexpr int KS = (N + 3) / 4;                 // k-steps
+    static constexpr int KP = 4 * KS;                      // padded k extent (rows of the B strip)
+    static constexpr int LDB = ((KP + 11) / 16) * 16 + 4;  // == 4 (mod 16): conflict-free B fragments
     static constexpr int STRIPS = (NB + BN - 1) / BN;
     static constexpr int THREADS = 32 * NW;
-    static constexpr size_t SMEM = sizeof(double) * ((size_t)LDB * BN + 2 * (size_t)LDA * BK);
-    static_assert(BM <= THREADS, "one thread per row of a chunk (Rh)");
-    static_assert(BN % 8 == 0 && N % 2 == 0 && NB % 2 == 0, "tile and 16-byte copy granularity");
+    static constexpr size_t SMEM = sizeof(double) * ((size_t)LDB * BN + KP);
+    static constexpr int XW = (MT + NW - 1) / NW;          // most row tiles of one warp, X and H
+    static constexpr int HW = (MTH + NW - 1) / NW;
+    // Row tiles of H at a time, k-steps that A is read ahead, and CTAs per SM.  Large
+    // elements: two tiles share every B fragment, 128 registers.  Small ones are
+    // bound by the latency of loading F, H and A of many short CTAs: one tile at a
+    // time in 64 registers.  Measured (ms; 2, 6, 4 | 1, 4, 8): 13,182 3D p3 6.19 |
+    // 11.7; 4,374 3D p2 0.536 | 0.493; 10,368 3D p1 0.304 | 0.218; 7,938 2D p4 0.419 |
+    // 0.360; 4,050 2D p3 0.119 | 0.109; 2,048 2D p2 0.038 | 0.029.
+    static constexpr bool LARGE = N >= 64;
+    static constexpr int PASS = LARGE ? 2 : 1, PD = (LARGE ? 6 : 4) < KS ? (LARGE ? 6 : 4) : KS, CTAS = LARGE ? 4 : 8;
+    static_assert(BN % 8 == 0, "whole column tiles");
 };
 
 struct FusedArgs {
@@ -48,12 +56,56 @@ struct FusedArgs {
     LiftArgs lift;              // perm, bf and sizes; src and cols unused
 };
 
+// acc[a] += A(rows of tile t[a], :) Bs for T row tiles of one warp: A column-major,
+// rows past m_end repeat the last row (their results are not stored); RHS: also
+// y[a] = this lane's share of A (row 8 t[a] + gr) . dru.
+template <class C, int T, bool RHS>
+__device__ __forceinline__ void fused_product(const double* __restrict__ A, int lda, int m_end, int n,
+                                              const int (&t)[T], const double* Bs, const double* dru,
+                                              double (&acc)[T][C::NTN][2], double (&y)[T]) {
+    constexpr int PD = C::PD;
+    const int lane = threadIdx.x & 31, gr = lane >> 2, gc = lane & 3;
+    const double* ap[T];
+#pragma unroll
+    for (int a = 0; a < T; a++) {
+        const int row = 8 * t[a] + gr;
+        ap[a] = A + (row < m_end ? row : m_end - 1) + (size_t)lda * gc;
+    }
+    auto fetch = [&](int ks, double (&f)[T]) {
+#pragma unroll
+        for (int a = 0; a < T; a++)
+            f[a] = (4 * C::KS == n || 4 * ks + gc < n) ? __ldg(ap[a] + (size_t)lda * 4 * ks) : 0.0;
+    };
+    double f[PD][T];
+#pragma unroll
+    for (int p = 0; p < PD; p++) fetch(p, f[p]);
+    const double* bp = Bs + gc + C::LDB * gr;
+#pragma unroll
+    for (int ks = 0; ks < C::KS; ks++) {
+        double af[T], bf[C::NTN];
+#pragma unroll
+        for (int a = 0; a < T; a++) af[a] = f[ks % PD][a];
+        if (ks + PD < C::KS) fetch(ks + PD, f[ks % PD]);
+#pragma unroll
+        for (int b = 0; b < C::NTN; b++) bf[b] = bp[4 * ks + C::LDB * 8 * b];
+#pragma unroll
+        for (int b = 0; b < C::NTN; b++)
+#pragma unroll
+            for (int a = 0; a < T; a++) dmma8x8x4(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
+        if constexpr (RHS) {
+            const double d = dru[4 * ks + gc];
+#pragma unroll
+            for (int a = 0; a < T; a++) y[a] = fma(af[a], d, y[a]);
+        }
+    }
+}
+
 template <int N, int NB, int BN, int NW>
-__global__ void __launch_bounds__(32 * NW) schur_fused_kernel(FusedArgs A) {
+__global__ void __launch_bounds__(32 * NW, (FusedCfg<N, NB, BN, NW>::CTAS)) schur_fused_kernel(FusedArgs A) {
     using C = FusedCfg<N, NB, BN, NW>;
     extern __shared__ __align__(16) double fsm[];
-    double* Bs = fsm;                                  // LDB x BN: the F strip, then the X strip
-    double* As = fsm + (size_t)C::LDB * BN;            // 2 stages of LDA x BK
+    double* Bs = fsm;                                  // LDB x BN: the F strip, then the -X strip
+    double* dru = fsm + (size_t)C::LDB * BN;           // D^-1 Ru, zero padded
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gr = lane >> 2, gc = lane & 3;
     const int e = blockIdx.x / C::STRIPS, c0 = (blockIdx.x % C::STRIPS) * BN;
@@ -63,61 +115,16 @@ __global__ void __launch_bounds__(32 * NW) schur_fused_kernel(FusedArgs A) {
     const double* Ke = A.K + (size_t)e * NB * N;
     double* He = A.H + (size_t)e * NB * NB;
     double* Xe = A.DinvF + (size_t)e * N * NB;
-
-    // A tile loader: rows [m0, m0 + BM) of A (lda rows, m_end valid), k columns [k0, k0 + BK)
-    auto load_a = [&](int st, const double* A, int lda, int m0, int m_end, int k0) {
-        double* as = As + (size_t)st * C::LDA * C::BK;
-        for (int t = tid; t < (C::BM / 2) * C::BK; t += C::THREADS) {
-            const int m = 2 * (t % (C::BM / 2)), k = t / (C::BM / 2);
-            const bool ok = m0 + m < m_end && k0 + k < N;
-            cp_async16z(&as[m + C::LDA * k], A + (ok ? (m0 + m) + (size_t)lda * (k0 + k) : 0), ok);
-        }
-    };
-
-    double acc[C::MPW][C::NTN][2];
-    double yrow = 0.0;         // strip 0: row tid of K (D^-1 Ru), this chunk
     const bool rhs = c0 == 0;
-    const double* dru = A.DinvRu + (size_t)e * N;
-    // one product: acc (+)= alpha A[m0.., :] Bs, k tiles through the ring (the
-    // first one already requested)
-    auto run = [&](const double* A, int lda, int m0, int m_end, double alpha, bool gemv) {
-        for (int kt = 0; kt < C::KT; kt++) {
-            cp_async_wait<0>();
-            __syncthreads();
-            if (kt + 1 < C::KT) load_a((kt + 1) & 1, A, lda, m0, m_end, (kt + 1) * C::BK);
-            cp_async_commit();
-            const double* as = As + (size_t)(kt & 1) * C::LDA * C::BK;
-            if (gemv && tid < C::BM) {
-#pragma unroll 4
-                for (int k = 0; k < C::BK; k++)
-                    if (kt * C::BK + k < N) yrow = fma(as[tid + C::LDA * k], __ldg(&dru[kt * C::BK + k]), yrow);
-            }
-#pragma unroll
-            for (int ks = 0; ks < C::BK; ks += 4) {
-                double bf[C::NTN];
-#pragma unroll
-                for (int b = 0; b < C::NTN; b++) bf[b] = Bs[(kt * C::BK + ks + gc) + C::LDB * (8 * b + gr)];
-#pragma unroll
-                for (int a = 0; a < C::MPW; a++) {
-                    const int mt = warp + NW * a;
-                    if (mt < C::MT) {
-                        const double af = alpha * as[(8 * mt + gr) + C::LDA * (ks + gc)];
-#pragma unroll
-                        for (int b = 0; b < C::NTN; b++) dmma8x8x4(acc[a][b][0], acc[a][b][1], af, bf[b]);
-                    }
-                }
-            }
-        }
-        __syncthreads();   // every warp is done with the ring and with Bs
-    };
+    // the warps' shares rotate from CTA to CTA, so that the longer shares of the
+    // CTAs of an SM do not meet on one scheduler
+    const int w = (warp + (int)((blockIdx.x * 2654435761u) >> 16)) % NW;
 
-    // ---- X = D^-1 (F + P H)_strip; the strip's rows >= N and columns past NB are
-    // zero.  A thread keeps one row of F for all columns.
-    load_a(0, De, N, 0, N, 0);
-    cp_async_commit();
+    // the strip of F + P H; rows >= N and columns past NB are zero.  A thread keeps
+    // one row of F for all columns.
     {
-        constexpr int CG = C::THREADS / N > 0 ? C::THREADS / N : 1;
-        static_assert(N <= C::THREADS, "one thread per row of F");
+        constexpr int CG = C::THREADS / N;
+        static_assert(CG > 0, "one thread per row of F");
         const int row = tid % N, cg = tid / N;
         if (cg < CG) {
             const LiftRow lr = lift_row(A.lift, e, row);
@@ -131,59 +138,92 @@ __global__ void __launch_bounds__(32 * NW) schur_fused_kernel(FusedArgs A) {
         if constexpr (C::KP > N)
             for (int t = tid; t < (C::KP - N) * BN; t += C::THREADS)
                 Bs[N + t % (C::KP - N) + C::LDB * (t / (C::KP - N))] = 0.0;
+        for (int t = tid; t < C::KP; t += C::THREADS) dru[t] = t < N ? A.DinvRu[(size_t)e * N + t] : 0.0;
     }
+    __syncthreads();
+
+    // ---- X = D^-1 (F + P H)_strip: row tiles w, w + NW, ...
+    double x[C::XW][C::NTN][2];
+    {
+        int t[C::XW];
+        double none[C::XW];
 #pragma unroll
-    for (int a = 0; a < C::MPW; a++)
+        for (int a = 0; a < C::XW; a++) {
+            t[a] = w + NW * a;
 #pragma unroll
-        for (int b = 0; b < C::NTN; b++) acc[a][b][0] = acc[a][b][1] = 0.0;
-    run(De, N, 0, N, 1.0, false);
-    // X to global and into Bs (the B operand of the second product)
+            for (int b = 0; b < C::NTN; b++) x[a][b][0] = x[a][b][1] = 0.0;
+        }
+        // the last tile of a warp with fewer tiles than the others: nothing to do
+        if (w + NW * (C::XW - 1) < C::MT) {
+            fused_product<C, C::XW, false>(De, N, N, N, t, Bs, dru, x, none);
+        } else if constexpr (C::XW > 1) {
+            fused_product<C, C::XW - 1, false>(De, N, N, N, reinterpret_cast<const int(&)[C::XW - 1]>(t), Bs, dru,
+                                               reinterpret_cast<double(&)[C::XW - 1][C::NTN][2]>(x),
+                                               reinterpret_cast<double(&)[C::XW - 1]>(none));
+        }
+    }
+    __syncthreads();
+    // X to global memory, -X into Bs (the B operand of the second product)
 #pragma unroll
-    for (int a = 0; a < C::MPW; a++) {
-        const int mt = warp + NW * a;
+    for (int a = 0; a < C::XW; a++) {
+        const int mt = w + NW * a;
 #pragma unroll
         for (int b = 0; b < C::NTN; b++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int row = 8 * mt + gr, col = 8 * b + 2 * gc + h;
                 if (mt < C::MT && row < N) {
-                    Bs[row + C::LDB * col] = acc[a][b][h];
-                    if (c0 + col < NB) Xe[row + (size_t)N * (c0 + col)] = acc[a][b][h];
+                    Bs[row + C::LDB * col] = -x[a][b][h];
+                    if (c0 + col < NB) Xe[row + (size_t)N * (c0 + col)] = x[a][b][h];
                 }
             }
     }
     __syncthreads();
 
-    // ---- H_strip -= K X, in row chunks of BM
-    for (int ch = 0; ch < C::CHUNKS; ch++) {
-        const int m0 = ch * C::BM;
-        load_a(0, Ke, NB, m0, NB, 0);
-        cp_async_commit();
+    // ---- H_strip += K (-X): row tiles from the other end (w = NW - 1 first), so
+    // that the warps with one tile of X more have one of H less; PASS at a time
+    const int wh = NW - 1 - w;
+    auto hpass = [&](auto tc, int a0) {
+        constexpr int T = decltype(tc)::value;
+        int t[T];
+        double acc[T][C::NTN][2], y[T];
 #pragma unroll
-        for (int a = 0; a < C::MPW; a++)
-#pragma unroll
-            for (int b = 0; b < C::NTN; b++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int mt = warp + NW * a;
-                    const int row = m0 + 8 * mt + gr, col = c0 + 8 * b + 2 * gc + h;
-                    acc[a][b][h] = (mt < C::MT && row < NB && col < NB) ? He[row + (size_t)NB * col] : 0.0;
-                }
-        yrow = 0.0;
-        run(Ke, NB, m0, NB, -1.0, rhs);
-        if (rhs && tid < C::BM && m0 + tid < NB) A.Rh[(size_t)e * NB + m0 + tid] -= yrow;
-#pragma unroll
-        for (int a = 0; a < C::MPW; a++) {
-            const int mt = warp + NW * a;
+        for (int a = 0; a < T; a++) {
+            t[a] = wh + NW * (a0 + a);
+            y[a] = 0.0;
 #pragma unroll
             for (int b = 0; b < C::NTN; b++)
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const int row = m0 + 8 * mt + gr, col = c0 + 8 * b + 2 * gc + h;
-                    if (mt < C::MT && row < NB && col < NB) He[row + (size_t)NB * col] = acc[a][b][h];
+                    const int row = 8 * t[a] + gr, col = c0 + 8 * b + 2 * gc + h;
+                    acc[a][b][h] = (row < NB && col < NB) ? He[row + (size_t)NB * col] : 0.0;
                 }
         }
-    }
+        if (rhs) fused_product<C, T, true>(Ke, NB, NB, N, t, Bs, dru, acc, y);
+        else fused_product<C, T, false>(Ke, NB, NB, N, t, Bs, dru, acc, y);
+#pragma unroll
+        for (int a = 0; a < T; a++) {
+            const int row = 8 * t[a] + gr;
+#pragma unroll
+            for (int b = 0; b < C::NTN; b++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int col = c0 + 8 * b + 2 * gc + h;
+                    if (row < NB && col < NB) He[row + (size_t)NB * col] = acc[a][b][h];
+                }
+            if (rhs) {
+                y[a] += __shfl_xor_sync(0xffffffffu, y[a], 1);
+                y[a] += __shfl_xor_sync(0xffffffffu, y[a], 2);
+                if (gc == 0 && row < NB) A.Rh[(size_t)e * NB + row] -= y[a];
+            }
+        }
+    };
+    const int cnt = wh < C::MTH ? (C::MTH - wh + NW - 1) / NW : 0;      // this warp's row tiles of H
+    int a0 = 0;
+#pragma unroll 1
+    for (; a0 + C::PASS <= cnt; a0 += C::PASS) hpass(std::integral_constant<int, C::PASS>{}, a0);
+    if constexpr (C::PASS > 1)
+        if (a0 < cnt) hpass(std::integral_constant<int, 1>{}, a0);
 }
 
 }  // namespace hfem
