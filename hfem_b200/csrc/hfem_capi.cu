@@ -21,6 +21,7 @@
 #include "elem_kernels.cuh"
 #include "krylov_kernels.cuh"
 #include "krylov_seg.cuh"
+#include "krylov_cycle.cuh"
 #include "schur_kernels.cuh"
 #include "launch.cuh"
 #include "norms.cuh"
@@ -72,6 +73,12 @@ struct SegTab {
     int *pseg = nullptr, *p0 = nullptr, *ticket = nullptr;
     double* part = nullptr;
     size_t part_n = 0;
+    // the one-kernel cycle (krylov_cycle.cuh): grid, pieces by rows, entries of the
+    // largest slice; grid 0: the system is not one for it
+    int cyc_grid = 0, cyc_npieces = 0, cyc_lmax = 0;
+    int *cyc_cp0 = nullptr, *cyc_prow = nullptr, *cyc_pseg = nullptr, *cyc_p0 = nullptr;
+    double* cyc_part = nullptr;
+    size_t cyc_part_n = 0;
 };
 
 struct hfem_ctx {
@@ -148,6 +155,7 @@ struct hfem_ctx {
     double *gm_sc = nullptr, *gm_h = nullptr, *gm_y = nullptr;
     int *gm_state = nullptr, *gm_its = nullptr, *gm_jc = nullptr, *gm_k = nullptr;
     unsigned char* gm_act = nullptr;
+    unsigned* gm_bar = nullptr;             // barrier counter and error flag of the one-kernel cycle
     size_t gm_hist_n = 0;
     int gm_restart = 0, gm_P = 0;
     // BILU0: ordering (computed once, from the first system), level schedule, factors
@@ -1138,6 +1146,61 @@ int matvec(hfem_ctx* c, const double* x, double* z, bool prec, const double* xsc
     return check_launch(c, "matvec");
 }
 
+// Block sizes with an instance of the one-kernel cycle; returns its kernel.
+template <typename MT>
+const void* cycle_kernel(int bsz) {
+    switch (bsz) {
+        case 8: return (const void*)gmres_cycle_kernel<8, MT>;
+        case 12: return (const void*)gmres_cycle_kernel<12, MT>;
+        case 15: return (const void*)gmres_cycle_kernel<15, MT>;
+        case 16: return (const void*)gmres_cycle_kernel<16, MT>;
+        case 20: return (const void*)gmres_cycle_kernel<20, MT>;
+        case 30: return (const void*)gmres_cycle_kernel<30, MT>;
+        default: return nullptr;
+    }
+}
+
+// Rows of the one-kernel cycle: one CTA per SM, each a contiguous range of block
+// rows, cut at the problems' boundaries into pieces.  cyc_grid stays 0 for systems
+// that the cycle does not take: block size 50 (its rows are streamed by a whole
+// CTA), slices above CYC_MAXL entries (their steps are bound by the basis traffic,
+// not by latency), or CTAs whose rows span too many problems.
+int build_cycle(hfem_ctx* c, SegTab& T, const std::vector<long long>& count) {
+    T.cyc_grid = 0;
+    const int b = c->bsz, nf = c->dims.nf, G = std::min(sms(c->device), nf);
+    if (!cycle_kernel<double>(b) || (long long)((nf + G - 1) / G) * b > CYC_MAXL) return 0;
+    std::vector<int> cp0, prow, pseg, p0(count.size() + 1, 0);
+    std::vector<int> send(count.size());                    // first row after segment p
+    int r = 0, lmax = 0;
+    for (size_t p = 0; p < count.size(); p++) send[p] = r += (int)(count[p] / b);
+    size_t p = 0;
+    int row = 0;
+    for (int g = 0; g < G; g++) {
+        cp0.push_back((int)prow.size());
+        const int end = (int)((long long)nf * (g + 1) / G);
+        lmax = std::max(lmax, (end - row) * b);
+        while (row < end) {
+            prow.push_back(row);
+            pseg.push_back((int)p);
+            row = std::min(end, send[p]);
+            if (row == send[p]) p++;
+        }
+        if ((int)prow.size() - cp0.back() > CYC_MAXP) return 0;
+    }
+    cp0.push_back((int)prow.size());
+    prow.push_back(nf);
+    for (size_t q = 0; q < pseg.size(); q++) p0[pseg[q] + 1] = (int)q + 1;
+    int rc;
+    if ((rc = upload(c, &T.cyc_cp0, cp0.data(), cp0.size())) || (rc = upload(c, &T.cyc_prow, prow.data(), prow.size())) ||
+        (rc = upload(c, &T.cyc_pseg, pseg.data(), pseg.size())) || (rc = upload(c, &T.cyc_p0, p0.data(), p0.size())))
+        return rc;
+    CK(cudaStreamSynchronize(c->stream));       // the host tables above are read until here
+    T.cyc_npieces = (int)pseg.size();
+    T.cyc_lmax = lmax;
+    T.cyc_grid = G;
+    return 0;
+}
+
 // The pieces of `count[p]` consecutive entries per segment p: a power of two of
 // SEG_THREADS up to SEG_PIECE entries each, about one CTA per SM.
 int build_segments(hfem_ctx* c, SegTab& T, const std::vector<long long>& count) {
@@ -1168,7 +1231,7 @@ int build_segments(hfem_ctx* c, SegTab& T, const std::vector<long long>& count) 
     T.npieces = (int)pseg.size();
     T.nseg = (int)count.size();
     T.rows = (int)(piece / SEG_THREADS);
-    return 0;
+    return build_cycle(c, T, count);
 }
 
 // The preconditioner of one GMRES: factors of the current Hg, and pb = M^-1 Rg.
@@ -1294,6 +1357,33 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
     const GmState GS{P, restart, maxit, tol, c->gm_H, c->gm_cs, c->gm_sn, c->gm_g, c->gm_nrmb, c->gm_sc, c->gm_state,
                      c->gm_its, c->gm_jc, c->gm_act, want_hist ? c->gm_hist : nullptr, want_hist ? hist_len : 0};
     const SegLaunch run = seg_launch(T.rows);
+    // one kernel per cycle, when the system is one for it (build_cycle)
+    const void* cyc = nullptr;
+    size_t cyc_smem = 0;
+    CycleArgs CA{};
+    if (T.cyc_grid && precond != 0 && restart <= CYC_MAXR) {
+        cyc = prec && c->precision >= 1 ? cycle_kernel<float>(c->bsz) : cycle_kernel<double>(c->bsz);
+        const size_t most = 200 * 1024;
+        const bool vcache = 8 * cyc_smem_doubles(T.cyc_lmax, restart, true) <= most;
+        cyc_smem = 8 * cyc_smem_doubles(T.cyc_lmax, restart, vcache);
+        const size_t rows = (size_t)T.cyc_npieces * (restart + 1);
+        if (T.cyc_part_n < 2 * rows + T.cyc_npieces) {
+            T.cyc_part_n = 0;
+            if ((rc = dalloc(c, &T.cyc_part, 2 * rows + T.cyc_npieces))) return rc;
+            T.cyc_part_n = 2 * rows + T.cyc_npieces;
+        }
+        if (!c->gm_bar) {
+            if ((rc = dalloc(c, &c->gm_bar, 2))) return rc;
+            CK(cudaMemsetAsync(c->gm_bar, 0, 2 * sizeof(unsigned), c->stream));
+        }
+        CK(cudaFuncSetAttribute(cyc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        const size_t ld = (size_t)(restart + 1) * P;
+        CA = CycleArgs{c->rowstart, c->colidx, c->Hg,
+                       !prec ? nullptr : (c->precision >= 1 ? (const void*)c->Minv32 : (const void*)c->Minv), c->V, n,
+                       T.cyc_cp0, T.cyc_prow, T.cyc_pseg, T.cyc_p0, T.cyc_npieces, T.cyc_part, T.cyc_part + rows,
+                       T.cyc_part + 2 * rows, c->gm_h, c->gm_h + ld, c->gm_bar, (int*)(c->gm_bar + 1), T.cyc_lmax,
+                       vcache ? 1 : 0};
+    }
     // out = xsc M^-1 Hg x
     auto op = [&](const double* x, double* out, const double* xsc) -> int {
         if (precond != 0) return matvec(c, x, out, prec, xsc, mv_act);
@@ -1317,7 +1407,13 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
         // V_0 = M^-1 b - M^-1 A x (x = 0 in the first cycle), beta = |V_0|
         if (!first && (rc = op(c->x, c->V, nullptr))) return rc;
         run.start(c, SP, GS, first);
-        for (int j = 0; j < restart && live; j++) {
+        if (cyc) {
+            Timed t(c, "arnoldi_cycle");
+            CK(cudaMemsetAsync(c->gm_bar, 0, sizeof(unsigned), c->stream));
+            void* args[] = {(void*)&CA, (void*)&GS};
+            CK(cudaLaunchCooperativeKernel(cyc, dim3(T.cyc_grid), dim3(CYC_THREADS), args, cyc_smem, c->stream));
+        }
+        for (int j = 0; j < restart && live && !cyc; j++) {
             if ((rc = op(c->V + (size_t)j * n, c->V + (size_t)(j + 1) * n, c->gm_sc + (size_t)j * P))) return rc;
             {
                 Timed t(c, "orthogonalise");
@@ -1329,6 +1425,15 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
         // x += V y for every problem that took part in this cycle
         run.end(c, SP, GS, n);
         if ((rc = check_launch(c, "combine"))) return rc;
+        if (cyc) {
+            int expired = 0;
+            CK(cudaMemcpyAsync(&expired, c->gm_bar + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+            if ((rc = any_running(live))) return rc;
+            if (expired) {
+                CK(cudaMemsetAsync(c->gm_bar + 1, 0, sizeof(int), c->stream));
+                return fail(c, HFEM_E_CUDA, "GMRES cycle kernel: a barrier wait expired");
+            }
+        }
     }
     std::vector<int> its(P);
     CK(cudaMemcpyAsync(its.data(), c->gm_its, sizeof(int) * P, cudaMemcpyDeviceToHost, c->stream));
@@ -1499,7 +1604,9 @@ int hfem_destroy(hfem_ctx* c) {
                     c->info, c->Minv, c->V, c->w, c->x, c->pb, c->binfo, c->udgi,
                     c->eprob, c->fprob, c->pparam, c->palpha, c->seg_one.pstart, c->seg_one.pseg, c->seg_one.p0,
                     c->seg_one.ticket, c->seg_one.part, c->seg_map.pstart, c->seg_map.pseg, c->seg_map.p0,
-                    c->seg_map.ticket, c->seg_map.part, c->gm_sc, c->gm_h, c->gm_y, c->gm_k, c->gm_act, c->tc_err, c->rn_part, c->rn_ticket, c->pn_range, c->pn_ticket, c->pn_part, c->pn_out, c->bf, c->bcm, c->bcs, c->Minv32,
+                    c->seg_map.ticket, c->seg_map.part, c->seg_one.cyc_cp0, c->seg_one.cyc_prow, c->seg_one.cyc_pseg,
+                    c->seg_one.cyc_p0, c->seg_one.cyc_part, c->seg_map.cyc_cp0, c->seg_map.cyc_prow, c->seg_map.cyc_pseg,
+                    c->seg_map.cyc_p0, c->seg_map.cyc_part, c->gm_bar, c->gm_sc, c->gm_h, c->gm_y, c->gm_k, c->gm_act, c->tc_err, c->rn_part, c->rn_ticket, c->pn_range, c->pn_ticket, c->pn_part, c->pn_out, c->bf, c->bcm, c->bcs, c->Minv32,
                     c->d_u2o, c->d_rows_lo, c->d_rows_up, c->d_fptr, c->d_fpos, c->Mg, c->bl_t, c->bl_y,
                     c->d_lvl_lo, c->d_lvl_up, c->Mg32, c->d_frec, c->d_lrec, c->d_urec, c->gm_H, c->gm_cs, c->gm_sn, c->gm_g, c->gm_nrmb, c->gm_hist,
                     c->gm_state, c->gm_its, c->gm_jc};
