@@ -155,7 +155,7 @@ struct hfem_ctx {
     double *gm_sc = nullptr, *gm_h = nullptr, *gm_y = nullptr;
     int *gm_state = nullptr, *gm_its = nullptr, *gm_jc = nullptr, *gm_k = nullptr;
     unsigned char* gm_act = nullptr;
-    unsigned* gm_bar = nullptr;             // barrier counter and error flag of the one-kernel cycle
+    unsigned* gm_bar = nullptr;             // barrier counters and error flag of the one-kernel cycle
     size_t gm_hist_n = 0;
     int gm_restart = 0, gm_P = 0;
     // BILU0: ordering (computed once, from the first system), level schedule, factors
@@ -1108,13 +1108,14 @@ int bj_factor(hfem_ctx* c) {
 }
 
 // z = xsc M^-1 Hg x (M^-1 omitted when !prec), rows of problems with
-// act[p] == 0 skipped; xsc: a factor per segment (NULL: 1).
-int matvec(hfem_ctx* c, const double* x, double* z, bool prec, const double* xsc, const unsigned char* act) {
+// act[p] == 0 skipped (act NULL: none); xsc: a factor per problem (NULL: 1); map:
+// rows to problems by the problem map, else all rows are problem 0.
+int matvec(hfem_ctx* c, const double* x, double* z, bool prec, const double* xsc, const unsigned char* act, bool map) {
     Timed t(c, "matvec");
     const int nf = c->dims.nf;
     const double* M = prec ? c->Minv : nullptr;
     const bool f32 = prec && c->precision >= 1;
-    const int* rseg = act ? c->fprob : nullptr;
+    const int* rseg = map ? c->fprob : nullptr;
     const int grid = std::max(1, std::min((nf + 7) / 8, sms(c->device) * 8));
     switch (c->bsz) {
         // small or odd block sizes: a warp per block row
@@ -1156,15 +1157,15 @@ const void* cycle_kernel(int bsz) {
         case 16: return (const void*)gmres_cycle_kernel<16, MT>;
         case 20: return (const void*)gmres_cycle_kernel<20, MT>;
         case 30: return (const void*)gmres_cycle_kernel<30, MT>;
+        case 50: return (const void*)gmres_cycle_kernel<50, double, true>;     // the product apart
         default: return nullptr;
     }
 }
 
 // Rows of the one-kernel cycle: one CTA per SM, each a contiguous range of block
 // rows, cut at the problems' boundaries into pieces.  cyc_grid stays 0 for systems
-// that the cycle does not take: block size 50 (its rows are streamed by a whole
-// CTA), slices above CYC_MAXL entries (their steps are bound by the basis traffic,
-// not by latency), or CTAs whose rows span too many problems.
+// that the cycle does not take: slices above CYC_MAXL entries (their steps are bound
+// by the basis traffic, not by latency), or CTAs whose rows span too many problems.
 int build_cycle(hfem_ctx* c, SegTab& T, const std::vector<long long>& count) {
     T.cyc_grid = 0;
     const int b = c->bsz, nf = c->dims.nf, G = std::min(sms(c->device), nf);
@@ -1325,7 +1326,6 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
     if (!map && !T.npieces && (rc = build_segments(c, T, {n}))) return rc;
     if ((rc = ensure_krylov(c, restart))) return rc;
     const int P = T.nseg;
-    const unsigned char* mv_act = map ? c->gm_act : nullptr;   // row -> problem only with a problem map
     if (c->gm_restart < restart || c->gm_P < P) {
         const size_t r1 = (size_t)std::max(restart, c->gm_restart) + 1, PP = (size_t)std::max(P, c->gm_P);
         if ((rc = dalloc(c, &c->gm_h, 4 * r1 * PP)) || (rc = dalloc(c, &c->gm_y, r1 * PP)) ||
@@ -1337,7 +1337,6 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
             return rc;
         c->gm_restart = (int)r1 - 1;
         c->gm_P = (int)PP;
-        mv_act = map ? c->gm_act : nullptr;
     }
     if (T.part_n < (size_t)T.npieces * (restart + 1)) {
         T.part_n = 0;
@@ -1360,11 +1359,13 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
     // one kernel per cycle, when the system is one for it (build_cycle)
     const void* cyc = nullptr;
     size_t cyc_smem = 0;
+    bool ext = false;               // ... per step, after the product's own launch
     CycleArgs CA{};
     if (T.cyc_grid && precond != 0 && restart <= CYC_MAXR) {
         cyc = prec && c->precision >= 1 ? cycle_kernel<float>(c->bsz) : cycle_kernel<double>(c->bsz);
         const size_t most = 200 * 1024;
-        const bool vcache = 8 * cyc_smem_doubles(T.cyc_lmax, restart, true) <= most;
+        ext = c->bsz > 32;
+        const bool vcache = !ext && 8 * cyc_smem_doubles(T.cyc_lmax, restart, true) <= most;
         cyc_smem = 8 * cyc_smem_doubles(T.cyc_lmax, restart, vcache);
         const size_t rows = (size_t)T.cyc_npieces * (restart + 1);
         if (T.cyc_part_n < 2 * rows + T.cyc_npieces) {
@@ -1373,21 +1374,21 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
             T.cyc_part_n = 2 * rows + T.cyc_npieces;
         }
         if (!c->gm_bar) {
-            if ((rc = dalloc(c, &c->gm_bar, 2))) return rc;
-            CK(cudaMemsetAsync(c->gm_bar, 0, 2 * sizeof(unsigned), c->stream));
+            if ((rc = dalloc(c, &c->gm_bar, 4))) return rc;
+            CK(cudaMemsetAsync(c->gm_bar, 0, 4 * sizeof(unsigned), c->stream));
         }
         CK(cudaFuncSetAttribute(cyc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         const size_t ld = (size_t)(restart + 1) * P;
         CA = CycleArgs{c->rowstart, c->colidx, c->Hg,
                        !prec ? nullptr : (c->precision >= 1 ? (const void*)c->Minv32 : (const void*)c->Minv), c->V, n,
                        T.cyc_cp0, T.cyc_prow, T.cyc_pseg, T.cyc_p0, T.cyc_npieces, T.cyc_part, T.cyc_part + rows,
-                       T.cyc_part + 2 * rows, c->gm_h, c->gm_h + ld, c->gm_bar, (int*)(c->gm_bar + 1), T.cyc_lmax,
-                       vcache ? 1 : 0};
+                       T.cyc_part + 2 * rows, c->gm_h, c->gm_h + ld, c->gm_bar, (int*)(c->gm_bar + 3), 0, restart,
+                       T.cyc_lmax, vcache ? 1 : 0};
     }
     // out = xsc M^-1 Hg x
     auto op = [&](const double* x, double* out, const double* xsc) -> int {
-        if (precond != 0) return matvec(c, x, out, prec, xsc, mv_act);
-        int r = matvec(c, x, c->bl_t, false, xsc, mv_act);
+        if (precond != 0) return matvec(c, x, out, prec, xsc, c->gm_act, map);
+        int r = matvec(c, x, c->bl_t, false, xsc, c->gm_act, map);
         return r ? r : bilu0_apply(c, c->bl_t, out);
     };
     // the Givens rotations, residual estimates and stopping tests run on the
@@ -1407,17 +1408,25 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
         // V_0 = M^-1 b - M^-1 A x (x = 0 in the first cycle), beta = |V_0|
         if (!first && (rc = op(c->x, c->V, nullptr))) return rc;
         run.start(c, SP, GS, first);
-        if (cyc) {
-            Timed t(c, "arnoldi_cycle");
-            CK(cudaMemsetAsync(c->gm_bar, 0, sizeof(unsigned), c->stream));
+        auto cycle = [&](int j0, int j1) -> int {
+            CA.j0 = j0;
+            CA.j1 = j1;
             void* args[] = {(void*)&CA, (void*)&GS};
             CK(cudaLaunchCooperativeKernel(cyc, dim3(T.cyc_grid), dim3(CYC_THREADS), args, cyc_smem, c->stream));
+            return 0;
+        };
+        if (cyc) CK(cudaMemsetAsync(c->gm_bar, 0, 3 * sizeof(unsigned), c->stream));
+        if (cyc && !ext) {
+            Timed t(c, "arnoldi_cycle");
+            if ((rc = cycle(0, restart))) return rc;
         }
-        for (int j = 0; j < restart && live && !cyc; j++) {
-            if ((rc = op(c->V + (size_t)j * n, c->V + (size_t)(j + 1) * n, c->gm_sc + (size_t)j * P))) return rc;
+        for (int j = 0; j < restart && live && (!cyc || ext); j++) {
+            if ((rc = op(c->V + (size_t)j * n, c->V + (size_t)(j + 1) * n, ext ? nullptr : c->gm_sc + (size_t)j * P))) return rc;
             {
                 Timed t(c, "orthogonalise");
-                run.step(c, SP, GS, n, j);
+                if (ext) rc = cycle(j, j + 1);
+                else run.step(c, SP, GS, n, j);
+                if (rc) return rc;
             }
             if ((rc = check_launch(c, "arnoldi"))) return rc;
             if (((j + 1) % GM_CHECK == 0 || j + 1 == restart) && (rc = any_running(live))) return rc;
@@ -1427,10 +1436,10 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
         if ((rc = check_launch(c, "combine"))) return rc;
         if (cyc) {
             int expired = 0;
-            CK(cudaMemcpyAsync(&expired, c->gm_bar + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+            CK(cudaMemcpyAsync(&expired, c->gm_bar + 3, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
             if ((rc = any_running(live))) return rc;
             if (expired) {
-                CK(cudaMemsetAsync(c->gm_bar + 1, 0, sizeof(int), c->stream));
+                CK(cudaMemsetAsync(c->gm_bar + 3, 0, sizeof(int), c->stream));
                 return fail(c, HFEM_E_CUDA, "GMRES cycle kernel: a barrier wait expired");
             }
         }
@@ -2272,7 +2281,7 @@ int hfem_matvec(hfem_ctx* c, const double* x, double* y) {
     if (!c || !x || !y) return HFEM_E_ARG;
     if (!c->assembled) return fail(c, HFEM_E_STATE, "assemble before a matvec");
     CK(cudaSetDevice(c->device));
-    int rc = matvec(c, x, y, false, nullptr, nullptr);
+    int rc = matvec(c, x, y, false, nullptr, nullptr, false);
     if (rc) return rc;
     CK(cudaStreamSynchronize(c->stream));
     return 0;

@@ -3,8 +3,8 @@
 //
 // One CTA per SM owns a contiguous range of block rows and its slice of every
 // basis vector (in shared memory when it fits, else in L2).  An Arnoldi step is
-//   product  w = M^-1 Hg V_j on the CTA's rows, a warp per row; meanwhile warp 0
-//            sums |V_j| and, in the CTA that owns the problem's first piece, runs
+//   product  w = M^-1 Hg V_j on the CTA's rows, a warp per row; meanwhile
+//            warp 0 sums |V_j| and, in the CTA that owns the problem's first piece, runs
 //            step j-1's Givens rotation and stopping test
 //   BAR 1    h1 = V^T w from all pieces' partial sums; w -= V h1; V^T w again
 //   BAR 2    h2 likewise; V_{j+1} = w - V h2 to global memory, its norm's partial
@@ -15,16 +15,21 @@
 // all CTAs see the same values.  The stopping tests of step j-1 are read after
 // BAR 1 of step j, so a cycle ends without the host.
 //
-// Measured (B200): 36,864 unknowns of 2D p = 2, 62 steps, 1.19 ms against 2.9 ms
+// Measured (B200): 36,864 unknowns of 2D p = 2, 62 steps, 1.15 ms against 2.9 ms
 // with the four launches per step of krylov_seg.cuh; eight problems of 104k unknowns
-// together, 74 steps, 2.7 against 4.2 ms.  For block size 50 (129,600 unknowns of 3D
-// p = 3) a step is bound by streaming Hg, and the launches per step stay.
+// together, 74 steps, 2.2 against 4.2 ms.
+//
+// EXT (block size 50): the product stays a launch of its own, one CTA per row (rows
+// of 140 KB streamed by the cycle's CTAs took 105 us a step against 74), and the
+// kernel is one step's orthogonalisation, the unscaled w read from V_{j+1}: 129,600 unknowns of
+// 3D p = 3, 32 us a step against 41 us with the three launches of krylov_seg.cuh.
 //
 // Barriers spin on a counter in global memory; the launch is cooperative, so all
 // CTAs are resident, and every spin is bounded: on expiry the kernel sets err and
 // returns.
 #pragma once
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "krylov_seg.cuh"
 
 namespace hfem {
@@ -49,8 +54,9 @@ struct CycleArgs {
     int npieces;
     double *part1, *part2, *partn;      // partial sums: (restart + 1) x npieces twice, npieces
     double *h1, *h2;                    // this step's projections, entry (i, seg) at i * P + seg
-    unsigned* bar;                      // zero at launch
+    unsigned* bar;                      // 3 counters, zero before a cycle
     int* err;
+    int j0, j1;                         // steps of this launch (EXT: one; else 0, restart)
     int lmax;                           // entries of the largest slice
     int vcache;                         // the slices of V fit in shared memory
 };
@@ -63,22 +69,26 @@ inline size_t cyc_smem_doubles(int lmax, int restart, bool vcache) {
            (vcache ? (size_t)lmax * (restart + 1) : 0);
 }
 
-__device__ __forceinline__ bool cyc_barrier(unsigned* bar, unsigned target, int* err) {
+// Barrier `which` (0, 1, 2 in turn) of the CTAs.  Each has its own counter, zero
+// when the first CTA arrives; past barrier b every CTA has left barrier b - 1, so
+// CTA 0 zeroes that counter for its next use.
+__device__ __forceinline__ bool cyc_barrier(unsigned* bar, int which, int* err) {
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        atomicAdd(bar, 1u);
+        atomicAdd(&bar[which], 1u);
         unsigned v = 0;
         int good = 0;
         for (int it = 0; it < (1 << 21); it++) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-            if ((int)(v - target) >= 0) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&bar[which]) : "memory");
+            if (v >= gridDim.x) {
                 good = 1;
                 break;
             }
         }
         if (!good) atomicExch(err, 3);
+        else if (blockIdx.x == 0) bar[(which + 2) % 3] = 0;
         ok = good;
     }
     __syncthreads();
@@ -178,7 +188,7 @@ __device__ __forceinline__ void cyc_row(int i, const int* __restrict__ rowstart,
     if (lane < BSZ) out(lane, z);
 }
 
-template <int BSZ, typename MT>
+template <int BSZ, typename MT, bool EXT = false>
 __global__ void __launch_bounds__(CYC_THREADS, 1) gmres_cycle_kernel(CycleArgs A, GmState S) {
     extern __shared__ __align__(16) double cyc_sm[];
     __shared__ int run[CYC_MAXP], pseg[CYC_MAXP], pofs[CYC_MAXP + 1], s_any;
@@ -202,13 +212,19 @@ __global__ void __launch_bounds__(CYC_THREADS, 1) gmres_cycle_kernel(CycleArgs A
     if (tid < npc) {
         pseg[tid] = A.pseg[pc0 + tid];
         run[tid] = S.act[pseg[tid]];
-        scs[tid * R2] = S.sc[pseg[tid]];
+        for (int i = 0; i <= A.j0; i++) scs[tid * R2 + i] = S.sc[(size_t)i * P + pseg[tid]];
+    }
+    if (tid == 0) s_any = 0;
+    __syncthreads();
+    if constexpr (EXT) {
+        for (int p = tid; p < P; p += CYC_THREADS)
+            if (S.act[p]) s_any = 1;
+        __syncthreads();
+        if (!s_any) return;
     }
     if (A.vcache)
         for (int t = tid; t < len; t += CYC_THREADS) vsm[t] = Vg[t];
     __syncthreads();
-    unsigned nbar = 0;
-    const unsigned G = gridDim.x;
     auto owner = [&](int c) { return A.seg_p0[pseg[c]] == pc0 + c; };
 
     // sum over the pieces of own piece c's segment of `cnt` rows of partials, into
@@ -230,25 +246,54 @@ __global__ void __launch_bounds__(CYC_THREADS, 1) gmres_cycle_kernel(CycleArgs A
             }
         }
     };
-    // <V_i, w> for i < k over own piece c
-    auto dots = [&](int c, int k, double* part) {
+    // <V_i, w> for i < k over own piece c: a warp per column (NC columns at a time
+    // when there are more columns than warps), or SP warps per column when there are
+    // few, their sums added through shared memory
+    auto columns = [&](int c, int k, double* part, auto ncc) {
+        constexpr int NC = decltype(ncc)::value;
         const int o0 = pofs[c], o1 = pofs[c + 1];
-        for (int base = warp; base < k; base += 4 * CYC_WARPS) {
-            double t[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int base = warp; base < k; base += NC * CYC_WARPS) {
+            double t[NC];
+#pragma unroll
+            for (int u = 0; u < NC; u++) t[u] = 0.0;
             const double* vp = vb + (size_t)base * ldv;
-#pragma unroll 4
+#pragma unroll(NC == 1 ? 16 : 8)
             for (int i = o0 + lane; i < o1; i += 32) {
                 const double x = ws[i];
 #pragma unroll
-                for (int u = 0; u < 4; u++)
+                for (int u = 0; u < NC; u++)
                     if (base + CYC_WARPS * u < k) t[u] = fma(vp[(size_t)CYC_WARPS * u * ldv + i], x, t[u]);
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < NC; u++) {
                 if (base + CYC_WARPS * u >= k) continue;
                 t[u] = seg_warp_sum(t[u]);
                 if (lane == 0) part[(size_t)(base + CYC_WARPS * u) * A.npieces + pc0 + c] = t[u];
             }
+        }
+    };
+    auto dots = [&](int c, int k, double* part) {
+        const int SP = k <= CYC_WARPS / 8 ? 8 : (k <= CYC_WARPS / 4 ? 4 : (k <= CYC_WARPS / 2 ? 2 : 1));
+        if (SP == 1) {
+            if (k <= CYC_WARPS) columns(c, k, part, std::integral_constant<int, 1>{});
+            else columns(c, k, part, std::integral_constant<int, 2>{});
+            return;
+        }
+        const int o0 = pofs[c], o1 = pofs[c + 1], i = warp / SP;
+        double t = 0.0;
+        if (i < k) {
+            const double* vp = vb + (size_t)i * ldv;
+#pragma unroll 8
+            for (int q = o0 + 32 * (warp % SP) + lane; q < o1; q += 32 * SP) t = fma(vp[q], ws[q], t);
+        }
+        t = seg_warp_sum(t);
+        __syncthreads();
+        if (lane == 0) red[warp] = t;
+        __syncthreads();
+        if (tid < k) {
+            double s = 0.0;
+            for (int q = 0; q < SP; q++) s += red[tid * SP + q];
+            part[(size_t)tid * A.npieces + pc0 + c] = s;
         }
     };
     // v[r] = scale(c) ws - sum_{i<k} cf_i V_i at this thread's entries
@@ -288,8 +333,11 @@ __global__ void __launch_bounds__(CYC_THREADS, 1) gmres_cycle_kernel(CycleArgs A
         __syncwarp();
     };
 
-    for (int j = 0; j < R; j++) {
+    for (int j = A.j0; j < A.j1; j++) {
         // ---- product on the rows of running problems
+        if constexpr (EXT) {
+            for (int i = tid; i < len; i += CYC_THREADS) ws[i] = Vg[(size_t)(j + 1) * A.n + i];
+        } else {
         if (warp == 0 && j > 0) finish(j);
         const double* x = A.V + (size_t)j * A.n;
         // warp 0 takes a row last: it has the norms to sum
@@ -300,20 +348,22 @@ __global__ void __launch_bounds__(CYC_THREADS, 1) gmres_cycle_kernel(CycleArgs A
             cyc_row<BSZ, MT>(row0 + r, A.rowstart, A.colidx, A.Hg, Minv, x, ys,
                              [&](int q, double z) { ws[r * BSZ + q] = z; });
         }
+        }
         __syncthreads();
-        if (j > 0 && tid < npc && run[tid]) scs[tid * R2 + j] = s_nn[tid] == 0.0 ? 1.0 : 1.0 / s_nn[tid];
+        if (!EXT && j > 0 && tid < npc && run[tid]) scs[tid * R2 + j] = s_nn[tid] == 0.0 ? 1.0 : 1.0 / s_nn[tid];
         for (int c = 0; c < npc; c++)
             if (run[c]) dots(c, j + 1, A.part1);
-        nbar += G;
-        if (!cyc_barrier(A.bar, nbar, A.err)) return;
+        if (!cyc_barrier(A.bar, 0, A.err)) return;
         // ---- step j - 1's stopping tests
-        if (tid == 0) s_any = 0;
-        __syncthreads();
-        for (int p = tid; p < P; p += CYC_THREADS)
-            if (__ldcg(&S.act[p])) s_any = 1;
-        if (tid < npc) run[tid] = __ldcg(&S.act[pseg[tid]]);
-        __syncthreads();
-        if (!s_any) return;
+        if constexpr (!EXT) {
+            if (tid == 0) s_any = 0;
+            __syncthreads();
+            for (int p = tid; p < P; p += CYC_THREADS)
+                if (__ldcg(&S.act[p])) s_any = 1;
+            if (tid < npc) run[tid] = __ldcg(&S.act[pseg[tid]]);
+            __syncthreads();
+            if (!s_any) return;
+        }
         // ---- first projection: h1_i = sc_i sc_j <V_i, z>
         for (int c = 0; c < npc; c++)
             if (run[c])
@@ -332,8 +382,7 @@ __global__ void __launch_bounds__(CYC_THREADS, 1) gmres_cycle_kernel(CycleArgs A
         __syncthreads();
         for (int c = 0; c < npc; c++)
             if (run[c]) dots(c, j + 1, A.part2);
-        nbar += G;
-        if (!cyc_barrier(A.bar, nbar, A.err)) return;
+        if (!cyc_barrier(A.bar, 1, A.err)) return;
         // ---- second projection
         for (int c = 0; c < npc; c++)
             if (run[c])
@@ -369,10 +418,9 @@ __global__ void __launch_bounds__(CYC_THREADS, 1) gmres_cycle_kernel(CycleArgs A
                 if (lane == 0) A.partn[pc0 + c] = t;
             }
         }
-        nbar += G;
-        if (!cyc_barrier(A.bar, nbar, A.err)) return;
+        if (!cyc_barrier(A.bar, 2, A.err)) return;
     }
-    if (warp == 0) finish(R);
+    if (warp == 0) finish(A.j1);
 }
 
 }  // namespace hfem

@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(SEG_THREADS) seg_combine_kernel(SegPieces P, l
 // in Hg, so the row is one column-major BSZ x (nblk * BSZ) matrix; the warp's
 // lanes form G = 32 / BSZ column groups of BSZ rows (R = 2 rows per lane when
 // BSZ > 32), and the groups' partial sums are added in group order.  Rows of
-// inactive segments (act[rseg[i]] == 0) are skipped.
+// inactive segments (act[rseg[i]] == 0; rseg NULL: one segment) are skipped.
 template <int BSZ, typename MT>
 __global__ void __launch_bounds__(256) bsr_matvec_warp_kernel(int nrows, const int* __restrict__ rowstart,
                                                               const int* __restrict__ colidx,
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(256) bsr_matvec_warp_kernel(int nrows, const i
     const bool on = g < G;
     const int nwarps = gridDim.x * 8;
     for (int i = blockIdx.x * 8 + wib; i < nrows; i += nwarps) {
-        if (act && !act[rseg[i]]) continue;
+        if (act && !act[rseg ? rseg[i] : 0]) continue;
         const int k0 = rowstart[i], k1 = rowstart[i + 1];
         const int ncol = (k1 - k0) * BSZ;
         const double* A = Hg + (size_t)k0 * BSZ * BSZ;
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(RowMv<BSZ>::THREADS) bsr_matvec_row_kernel(int
     __shared__ double y[BSZ];
     const int tid = threadIdx.x, g = tid / C::L2, q = tid - g * C::L2;
     const int i = blockIdx.x;
-    if (act && !act[rseg[i]]) return;
+    if (act && !act[rseg ? rseg[i] : 0]) return;
     const int k0 = rowstart[i], ncol = (rowstart[i + 1] - k0) * BSZ;
     const bool on = tid < C::USED;
     double a0 = 0.0, a1 = 0.0;
