@@ -388,7 +388,7 @@ static __global__ void scatter_R_kernel(ScatterArgs A) {
             const int a = A.face_src[(i * 2 + c) * 2 + 1];
             const int ind = A.elcon[(size_t)e * ndf + a * A.npf + m1] - i * A.npf;
             const size_t idx = (size_t)e * A.nb + a * bsz + ind * A.nch + n1;
-            s += A.Rh[idx];
+            if (A.Rg) s += A.Rh[idx];
             if (A.Ro) so += A.Ro[idx];
         }
         if (A.Rg) A.Rg[t] = s;

@@ -91,6 +91,8 @@ struct hfem_ctx {
     bool have_master = false, have_mesh = false, have_phys = false, have_sol = false, assembled = false;
     int grid_elem = 0, grid_inv = 0, grid_tc = 0;
     int grid_elem_v[2][2] = {};         // per element-kernel variant [tf][gen], at most grid_elem
+    int grid_res[2] = {};               // residual-only pass [gen]
+    bool res_blocks = false;            // D, K, H, Rh of the last residual-only pass not formed yet (form_blocks)
     // element-wise state arriving in pieces (hfem_assemble_host): the element
     // kernel of piece k waits for chunk_ev[k]
     cudaStream_t copy_stream = nullptr;
@@ -488,7 +490,11 @@ int enqueue_assembly(hfem_ctx* c, bool matrix) {
     const int gen = (c->conv_stab != 0 || c->visc_model != 0) ? 1 : 0;
     const dim3 ge(c->grid_elem_v[tf][gen]);
     auto element = c->L->element_v[tf][gen];
-    {
+    if (!matrix) {
+        Timed t(c, "residual");
+        c->L->residual[gen](dim3(c->grid_res[gen]), c->L->res_smem, c->stream, elem_args(c));
+        if ((rc = check_launch(c, "residual"))) return rc;
+    } else {
         Timed t(c, "element");
         if (c->pending_chunks > 0) {
             // one launch per piece of the state, each after that piece's copy
@@ -587,6 +593,7 @@ int finish_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
     if (st.wait_err == 1) return fail(c, HFEM_E_CUDA, "tensor-core Schur kernel: an MMA completion wait expired");
     if (st.wait_err == 2) return fail(c, HFEM_E_CUDA, "element kernel: a bulk-copy completion wait expired");
     if (matrix) c->assembled = true;
+    c->res_blocks = !matrix;
     flush_timer(c);
     if (rnorm_out) *rnorm_out = st.rnorm;
     return 0;
@@ -600,7 +607,21 @@ int run_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
     return finish_assembly(c, matrix, rnorm_out);
 }
 
+// After a residual-only pass the element blocks are D, K, H and Rh at its state
+// (hfem_download); they are formed when one of them is asked for.
+int form_blocks(hfem_ctx* c) {
+    const int tf = (c->precision == 1 || c->precision == 3) ? 1 : 0;
+    const int gen = (c->conv_stab != 0 || c->visc_model != 0) ? 1 : 0;
+    c->L->element_v[tf][gen](dim3(c->grid_elem_v[tf][gen]), c->L->elem_smem, c->stream, elem_args(c));
+    int rc = check_launch(c, "element");
+    if (rc) return rc;
+    c->res_blocks = false;
+    CK(cudaStreamSynchronize(c->stream));
+    return 0;
+}
+
 int launch_getq(hfem_ctx* c, const double* duh, double alpha) {
+    c->res_blocks = false;
     QArgs q;
     q.T = Tables{c->shapvt, c->shapvg, c->svsv, c->shapft, c->shapfg, c->sfsf, c->perm};
     q.dgnodes = c->dgnodes;
@@ -1563,6 +1584,12 @@ int hfem_create(const hfem_dims* dims, int device, hfem_ctx** out) {
     for (int t = 0; t < 2; t++)
         for (int g = 0; g < 2; g++)
             cudaFuncSetAttribute(L.elem_fn_v[t][g], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.elem_smem);
+    for (int g = 0; g < 2; g++) {
+        cudaFuncSetAttribute(L.res_fn[g], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.res_smem);
+        int occ = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.res_fn[g], L.res_threads, L.res_smem);
+        c->grid_res[g] = std::max(1, std::min(d.ne, sms(device) * std::max(occ, 1)));
+    }
     cudaFuncSetAttribute(L.q_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.q_smem);
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.elem_fn, L.elem_threads, L.elem_smem);
@@ -1722,6 +1749,7 @@ int hfem_set_mesh(hfem_ctx* c, const double* dgnodes, const int* elcon, const in
     c->h_rowstart.assign(rowstart, rowstart + nf + 1);
     c->h_colidx.assign(colidx, colidx + nblk);
     c->have_order = false;
+    c->res_blocks = false;
     if (c->bf) { pool_free(c->bf); c->bf = nullptr; }      // boundary flags belong to the old mesh
     c->have_mesh = true;
     return 0;
@@ -1764,6 +1792,7 @@ int hfem_set_boundary(hfem_ctx* c, const int* bf, int nbnd, const int* bcm, cons
         return rc;
     CK(cudaStreamSynchronize(c->stream));
     c->nbnd = nbnd;
+    c->res_blocks = false;
     c->assembled = false;
     return 0;
 }
@@ -1773,6 +1802,7 @@ int hfem_set_app(hfem_ctx* c, int appname) {
     if (appname != 0 && appname != 1)
         return fail(c, HFEM_E_UNSUPPORTED, "appname %d (supported: 0 Euler, 1 Navier-Stokes)", appname);
     c->appname = appname;
+    c->res_blocks = false;
     c->assembled = false;
     return 0;
 }
@@ -1786,12 +1816,14 @@ int hfem_set_models(hfem_ctx* c, int conv_stab, int viscosity_model) {
         return fail(c, HFEM_E_UNSUPPORTED, "viscosityModel %d (supported: 0 constant, 1 Sutherland)", viscosity_model);
     c->conv_stab = conv_stab;
     c->visc_model = viscosity_model;
+    c->res_blocks = false;
     c->assembled = false;
     return 0;
 }
 
 int hfem_set_physics(hfem_ctx* c, const double* param, int tdep, double fc_u, double fc_q, double time) {
     if (!c || !param) return HFEM_E_ARG;
+    c->res_blocks = false;
     if (!(param[0] > 1.0) || !(param[2] > 0.0) || !(param[3] > 0.0))
         return fail(c, HFEM_E_ARG, "physicsparam needs gamma > 1, Re > 0, Pr > 0");
     for (int i = 0; i < 6; i++) c->param[i] = param[i];
@@ -1818,6 +1850,7 @@ static int set_solution_common(hfem_ctx* c, const double* udg, const double* uh,
     else CK(cudaMemsetAsync(c->sh, 0, sizeof(double) * nudg, c->stream));
     c->have_sol = true;
     c->assembled = false;
+    c->res_blocks = false;
     return 0;
 }
 
@@ -2325,6 +2358,7 @@ int hfem_set_precision(hfem_ctx* c, int mode) {
                                    "FP32 preconditioner), 2 (FP32 preconditioner) or 3 (3xTF32 element "
                                    "contractions, FP32 preconditioner)");
     c->precision = mode;
+    c->res_blocks = false;
     c->assembled = false;
     return 0;
 }
@@ -2336,6 +2370,10 @@ int hfem_gmres_problems(hfem_ctx* c, int precond, int restart, double tol, int m
 
 int device_buffer(hfem_ctx* c, int what, const double** src, size_t* need) {
     const hfem_dims& d = c->dims;
+    if (c->res_blocks && (what == 5 || what == 6 || what == 10 || what == 13)) {
+        int rc = form_blocks(c);
+        if (rc) return rc;
+    }
     switch (what) {
         case 0: *src = c->Hg; *need = (size_t)d.nblocks * c->bsz * c->bsz; break;
         case 1: *src = c->Rg; *need = (size_t)d.nf * c->bsz; break;

@@ -58,6 +58,11 @@ struct Launch {
     // [tf][gen]: 3xTF32 contractions; Lax-Friedrichs / Roe tensor or Sutherland's law compiled in
     void (*element_v[2][2])(dim3, size_t, cudaStream_t, const ElemArgs&);
     size_t elem_smem;
+    // residual-only pass [gen]
+    void (*residual[2])(dim3, size_t, cudaStream_t, const ElemArgs&);
+    const void* res_fn[2];
+    size_t res_smem;
+    int res_threads;
     const void* elem_fn;
     const void* elem_fn_v[2][2];
     int inv_threads;

@@ -218,25 +218,37 @@ __device__ __forceinline__ void ns_dir(double gam, double iRe, double kappa, dou
     s.kap = kappa * mu;
 }
 
+// The flux F.X alone: val(j, F_j).
+template <int ND, class Val>
+__device__ __forceinline__ void ns_dir_value(const NsDir<ND>& s, Val val) {
+    double vt = 0.0, vG = 0.0;
+    val(0, s.rho * s.Vn);
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+        const double tn = s.a * (s.Gn[i] + s.Hn[i] - (2.0 / 3.0) * s.div * s.X[i]);
+        vt = fma(s.v[i], tn, vt);
+        vG = fma(s.v[i], s.Gn[i], vG);
+        val(1 + i, fma(s.rho * s.v[i], s.Vn, fma(s.p, s.X[i], tn)));
+    }
+    const double heat = s.qEn * s.ir - s.E * s.Q0n * (s.ir * s.ir) - vG;
+    val(ND + 1, fma(s.E + s.p, s.Vn, fma(s.kap, heat, vt)));
+}
+
 // The flux F.X and its columns along the conserved variables: val(j, F_j) and
 // col(k, j, dF_j/du_k).  dmu[k] = dmu/du_k (GEN; NULL: constant viscosity).
 template <int ND, class Val, class Col>
 __device__ __forceinline__ void ns_dir_u(double gam, double iRe, double kappa, const double* dmu, const NsDir<ND>& s,
                                          Val val, Col col) {
     const double g1 = gam - 1.0, ir2 = s.ir * s.ir, c23 = 2.0 / 3.0;
-    double sh[ND], tn[ND], vt = 0.0, vG = 0.0;       // stress without mu/Re, stress, v.stress, v.Gn
+    double sh[ND], tn[ND], vG = 0.0;                 // stress without mu/Re, stress, v.Gn
 #pragma unroll
     for (int i = 0; i < ND; i++) {
         sh[i] = s.Gn[i] + s.Hn[i] - c23 * s.div * s.X[i];
         tn[i] = s.a * sh[i];
-        vt = fma(s.v[i], tn[i], vt);
         vG = fma(s.v[i], s.Gn[i], vG);
     }
     const double heat = s.qEn * s.ir - s.E * s.Q0n * ir2 - vG, EP = s.E + s.p;
-    val(0, s.rho * s.Vn);
-#pragma unroll
-    for (int i = 0; i < ND; i++) val(1 + i, fma(s.rho * s.v[i], s.Vn, fma(s.p, s.X[i], tn[i])));
-    val(ND + 1, fma(EP, s.Vn, fma(s.kap, heat, vt)));
+    ns_dir_value<ND>(s, val);
     // what a viscosity derivative adds to column k
     auto visc = [&](int k, int i) { return dmu ? iRe * dmu[k] * sh[i] : 0.0; };
     auto visc_e = [&](int k) {

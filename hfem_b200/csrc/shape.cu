@@ -5,6 +5,7 @@
 #include "launch.cuh"
 #include "elem_kernel.cuh"
 #include "inverse_blocked.cuh"
+#include "residual.cuh"
 
 namespace hfem {
 
@@ -30,6 +31,10 @@ void launch_inverse(dim3 g, cudaStream_t st, int ne, double* D, const double* Ru
 template <class S, bool TF, bool GEN>
 void launch_element(dim3 g, size_t sm, cudaStream_t st, const ElemArgs& a) {
     element_kernel<S, TF, GEN><<<g, S::NT, sm, st>>>(a);
+}
+template <class S, bool GEN>
+void launch_residual(dim3 g, size_t sm, cudaStream_t st, const ElemArgs& a) {
+    residual_kernel<S, GEN><<<g, RES_THREADS, sm, st>>>(a);
 }
 template <class S>
 void launch_getq(dim3 g, size_t sm, cudaStream_t st, const QArgs& a) { getq_kernel<S><<<g, QT, sm, st>>>(a); }
@@ -78,6 +83,12 @@ Launch make_launch() {
     L.element_v[1][0] = launch_element<S, true, false>;
     L.element_v[1][1] = launch_element<S, true, true>;
     L.elem_threads = S::NT;
+    L.residual[0] = launch_residual<S, false>;
+    L.residual[1] = launch_residual<S, true>;
+    L.res_fn[0] = (const void*)residual_kernel<S, false>;
+    L.res_fn[1] = (const void*)residual_kernel<S, true>;
+    L.res_smem = sizeof(ResSmem<S>);
+    L.res_threads = RES_THREADS;
     L.elem_smem = sizeof(ElemSmem<S>);
     L.elem_fn = (const void*)element_kernel<S, false, false>;
     L.elem_fn_v[0][0] = (const void*)element_kernel<S, false, false>;

@@ -267,7 +267,10 @@ int hfem_gmres_problems(hfem_ctx* ctx, int precond, int restart, double tol, int
  * 10 element K (nb*n*ne), 12 element Rh before condensation (nb*ne),
  * 13 element D^-1 after an
  * assembly (n*n*ne; D itself after a residual-only pass), 14 ||Ru_e||^2 before
- * condensation (ne). */
+ * condensation (ne).  hfem_residual forms no element blocks; 5, 6, 10 and 13
+ * asked for after it are H, Rh and K before condensation and D, formed then, as
+ * long as the state it was taken at is unchanged (after a change: the blocks of
+ * the last assembly). */
 int hfem_download(hfem_ctx* ctx, int what, double* host, size_t count);
 
 /* Per-kernel device time (ms) accumulated since the last reset, when timing

@@ -10,7 +10,8 @@ import pytest
 
 from hfem_b200.batch import BatchSolver
 from hfem_b200.core import HDGSolver, HfemError
-from hfem_b200.gen.problem import ns2d_vortex, ns3d_fourier
+from hfem_b200.gen.problem import as_euler, ns2d_channel, ns2d_vortex, ns3d_box, ns3d_fourier, with_models
+from oracle import Oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -27,6 +28,38 @@ def test_residual_norm(prob):
         rr, ru2 = s.download("Rr"), s.download("ru2")
         ref = np.sqrt(np.sum(ru2) + np.sum(rr ** 2))
         assert abs(rn - ref) <= (rr.size + ru2.size) * EPS * ref
+    s.close()
+
+
+RESIDUALS = {"2d_p1": lambda: ns2d_vortex(n=5, porder=1), "2d_p2": lambda: ns2d_vortex(n=4, porder=2),
+             "2d_p3_walls_roe": lambda: with_models(ns2d_channel(n=3, porder=3), 2, 1),
+             "2d_p4_euler": lambda: as_euler(ns2d_vortex(n=3, porder=4)), "3d_p1": lambda: ns3d_fourier(n=3, porder=1),
+             "3d_p2_walls_lf": lambda: with_models(ns3d_box(n=2, porder=2), 1, 0),
+             "3d_p3": lambda: ns3d_fourier(n=3, porder=3)}
+
+
+@pytest.mark.parametrize("name", list(RESIDUALS))
+def test_residual_only_pass(name):
+    """Against the element kernel's residual (1e-13 of its largest entry: the same
+    sums of at most a few hundred terms in another order), and the element blocks
+    asked for after it against the oracle's (1e-12, as in the parity tests)."""
+    prob = RESIDUALS[name]()
+    s = HDGSolver(prob)
+    s.getQ()
+    rn = s.assembleLinearSystem()
+    ref = {k: s.download(k) for k in ("Rr", "Ro", "ru2", "Rg", "DinvRu")}
+    assert abs(s.computeResidualNorm() - rn) <= 1e-13 * rn
+    for k in ("Rr", "Ro", "ru2"):
+        assert np.max(np.abs(s.download(k) - ref[k])) <= 1e-13 * np.max(np.abs(ref[k]))
+    for k in ("Rg", "DinvRu"):
+        assert np.array_equal(s.download(k), ref[k])
+    udg, uh = s.get_solution()
+    o = Oracle(prob)
+    for e in (0, prob.mesh.ne - 1):
+        b = o.element(udg, uh, e)
+        for k, r in (("Dinv", "D"), ("K", "K"), ("H", "H"), ("Rh", "Rh")):
+            got = s.download(k).reshape(prob.mesh.ne, -1)[e]
+            assert np.max(np.abs(got - b[r])) <= 1e-12 * max(np.max(np.abs(b[r])), np.max(np.abs(ref["Ro"])))
     s.close()
 
 
