@@ -87,31 +87,6 @@ struct EK {
     static_assert(O_U % 2 == 0 && O_SHU % 2 == 0, "16-byte alignment of the bulk-copied element inputs");
 };
 
-// Cholesky solves L L' x = b for one column held in registers, in the axpy
-// (column) form: after x_j is final every later entry takes its update, so each
-// step has up to npv - 1 independent FMAs; rdg holds 1 / L(j, j).
-template <int NPV>
-__device__ __forceinline__ void chol_solve_col_axpy(const double* lm, const double* rdg, double* col) {
-    const volatile double* l = lm;
-    double x[NPV];
-#pragma unroll
-    for (int i = 0; i < NPV; i++) x[i] = col[i];
-#pragma unroll
-    for (int j = 0; j < NPV; j++) {
-        x[j] *= rdg[j];
-#pragma unroll
-        for (int i = j + 1; i < NPV; i++) x[i] = fma(-l[i + NPV * j], x[j], x[i]);
-    }
-#pragma unroll
-    for (int j = NPV - 1; j >= 0; j--) {
-        x[j] *= rdg[j];
-#pragma unroll
-        for (int i = 0; i < j; i++) x[i] = fma(-l[j + NPV * i], x[j], x[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < NPV; i++) col[i] = x[i];
-}
-
 // Basis-by-(M^-1 C | M^-1 E) products on the FP64 tensor cores, one n-tile per
 // warp at a time:
 //   OUT(r, n) = sum_kk A(r, kk) CE(row(kk), n),  r < MR, kk < KD, n < NPV ND + NDF ND

@@ -65,7 +65,6 @@ struct ElemArgs {
     int e_begin = 0;            // element range [e_begin, ne) of this launch
 };
 
-constexpr int QT = 256;         // threads per CTA of the q recovery
 
 // --------------------------------------------------------------- helpers
 __device__ __forceinline__ double block_sum(double v, double* red) {
@@ -292,20 +291,6 @@ __device__ void cholesky_warp(double* a, double* rdg = nullptr) {
     }
 }
 
-template <int NPV>
-__device__ __forceinline__ void chol_solve_col(const double* l, double* x) {
-    for (int i = 0; i < NPV; i++) {
-        double t = x[i];
-        for (int k = 0; k < i; k++) t -= l[i + NPV * k] * x[k];
-        x[i] = t / l[i + NPV * i];
-    }
-    for (int i = NPV - 1; i >= 0; i--) {
-        double t = x[i];
-        for (int k = i + 1; k < NPV; k++) t -= l[k + NPV * i] * x[k];
-        x[i] = t / l[i + NPV * i];
-    }
-}
-
 // --------------------------------------------------------------- scatter
 // Owner-gather into the face-block system (globalassembly.cpp:40-89): every
 // Hg entry sums its (at most two) element contributions in ascending element
@@ -412,27 +397,71 @@ struct QArgs {
     const double* palpha;
 };
 
+constexpr int QT = 128;         // threads per CTA of the q recovery
+
 template <class S>
 struct QSmem {
     double x[S::NPV * S::ND];
     double jac[S::NGV], Xx[S::NGV * S::ND * S::ND];
     double jacf[S::NA], nl[S::NA * S::ND];
-    double M[S::NPV * S::NPV];
-    double C[S::NPV * S::NPV * S::ND];
-    double E[S::NPV * S::NDF * S::ND];
-    double u[S::NPV * S::NCU];
-    double uhe[S::NDF * S::NCH];
-    double de[S::NB];
+    double M[S::NPV * S::NPV], rdg[S::NPV];
+    double u[S::NPV * S::NCU], ug[S::NGV * S::NCU];
+    double uhe[S::NDF * S::NCH], uhq[S::NA * S::NCH];
+    double de[S::NB], part[QT > S::N ? QT / S::N * S::N : S::N];
     double q[S::NPV * S::NCU * S::ND];
+    int perm[S::NDF];
+    int inc_n[S::NPV];
+    int inc_f[S::NPV * S::MAXINC];
 };
 
-// getQ (elementassembly.cpp:1414-1479), optionally preceded by getU (solutionupdate.cpp:6-68).
+// Cholesky solves L L' x = b for one column held in registers, in the axpy
+// (column) form: after x_j is final every later entry takes its update, so each
+// step has up to npv - 1 independent FMAs; rdg holds 1 / L(j, j).
+template <int NPV>
+__device__ __forceinline__ void chol_solve_col_axpy(const double* lm, const double* rdg, double* col) {
+    const volatile double* l = lm;
+    double x[NPV];
+#pragma unroll
+    for (int i = 0; i < NPV; i++) x[i] = col[i];
+#pragma unroll
+    for (int j = 0; j < NPV; j++) {
+        x[j] *= rdg[j];
+#pragma unroll
+        for (int i = j + 1; i < NPV; i++) x[i] = fma(-l[i + NPV * j], x[j], x[i]);
+    }
+#pragma unroll
+    for (int j = NPV - 1; j >= 0; j--) {
+        x[j] *= rdg[j];
+#pragma unroll
+        for (int i = 0; i < j; i++) x[i] = fma(-l[j + NPV * i], x[j], x[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < NPV; i++) col[i] = x[i];
+}
+
+// getQ (elementassembly.cpp:1414-1479), optionally preceded by getU
+// (solutionupdate.cpp:6-68).  The right-hand side C u - E uhat is summed from u and
+// uhat at the quadrature points (C and E themselves, 72 products for each of 1,200
+// entries of the tetrahedron p = 3, are not formed), the source's part of q is added
+// after the solve, D^-1 F duh is read by all threads, several columns each, and the
+// factorisation runs under the sums.  Bound by HBM in the update (D^-1 F once).
+// 1,296 tetrahedra p = 3: getQ 205 -> 70 us, with the update 242 -> 123 us.
 template <class S>
 static __global__ void __launch_bounds__(QT) getq_kernel(QArgs A) {
-    constexpr int ND = S::ND, NPV = S::NPV, NCU = S::NCU, NC = S::NC, NCH = S::NCH, NDF = S::NDF, N = S::N, NB = S::NB;
+    constexpr int ND = S::ND, NPV = S::NPV, NPF = S::NPF, NGV = S::NGV, NGF = S::NGF, NA = S::NA;
+    constexpr int NCU = S::NCU, NC = S::NC, NCH = S::NCH, NDF = S::NDF, N = S::N, NB = S::NB;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     QSmem<S>& sm = *reinterpret_cast<QSmem<S>*>(smem_raw);
+    const Tables& T = A.T;
     const int tid = threadIdx.x;
+    for (int t = tid; t < NDF; t += QT) sm.perm[t] = T.perm[t];
+    __syncthreads();
+    for (int i = tid; i < NPV; i += QT) {
+        int c = 0;
+        for (int f = 0; f < NDF; f++)
+            if (sm.perm[f] == i && c < S::MAXINC) sm.inc_f[i * S::MAXINC + c++] = f;
+        sm.inc_n[i] = c;
+    }
     for (int e = blockIdx.x; e < A.ne; e += gridDim.x) {
         __syncthreads();
         double* ue = A.udg + (size_t)e * NPV * NC;
@@ -444,40 +473,104 @@ static __global__ void __launch_bounds__(QT) getq_kernel(QArgs A) {
             if (A.DinvF) sm.de[fn * NCH + c] = A.duh[(size_t)gd * NCH + c];
         }
         __syncthreads();
-        const double alpha = A.palpha ? A.palpha[A.eprob[e]] : A.alpha;
-        for (int t = tid; t < N; t += QT) {
-            double v = ue[t];
-            if (A.DinvF) {
-                const double* df = A.DinvF + (size_t)e * N * NB;
+        if (A.DinvF) {
+            // u += alpha (D^-1 Ru - D^-1 F duh): thread (row, group), groups of columns
+            constexpr int G = QT / N > 0 ? QT / N : 1;
+            const double alpha = A.palpha ? A.palpha[A.eprob[e]] : A.alpha;
+            const double* df = A.DinvF + (size_t)e * N * NB;
+            for (int t = tid; t < N * G; t += QT) {
+                const int row = t % N, g = t / N;
+                double s[4] = {0.0, 0.0, 0.0, 0.0};
+                int c = g;
+#pragma unroll 4
+                for (; c + 3 * G < NB; c += 4 * G)
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        s[k] = fma(__ldg(&df[row + (size_t)N * (c + k * G)]), sm.de[c + k * G], s[k]);
+                for (; c < NB; c += G) s[0] = fma(__ldg(&df[row + (size_t)N * c]), sm.de[c], s[0]);
+                sm.part[t] = (s[0] + s[1]) + (s[2] + s[3]);
+            }
+            __syncthreads();
+            for (int t = tid; t < N; t += QT) {
                 double s = 0.0;
-                for (int c = 0; c < NB; c++) s += df[t + (size_t)N * c] * sm.de[c];
+#pragma unroll
+                for (int g = 0; g < G; g++) s += sm.part[t + N * g];
+                double v = ue[t];
                 v += -alpha * s;
                 v += alpha * A.DinvRu[(size_t)e * N + t];
                 ue[t] = v;
+                sm.u[t] = v;
             }
-            sm.u[t] = v;
+        } else {
+            for (int t = tid; t < N; t += QT) sm.u[t] = ue[t];
         }
-        geometry<S>(A.T, sm.x, sm.jac, sm.Xx, sm.jacf, sm.nl);
+        geometry<S>(T, sm.x, sm.jac, sm.Xx, sm.jacf, sm.nl);
         __syncthreads();
-        qmatrices<S>(A.T, A.fc_q, sm.jac, sm.Xx, sm.jacf, sm.nl, sm.M, sm.C, sm.E);
+        // M, and u and uhat at the points
+        for (int t = tid; t < NPV * NPV; t += QT) {
+            const int i = t % NPV, a = t / NPV;
+            double s = 0.0;
+#pragma unroll 4
+            for (int g = 0; g < NGV; g++)
+                s = fma(__ldg(&T.shapvg[i + NPV * g]) * sm.jac[g], __ldg(&T.shapvt[g + NGV * a]), s);
+            sm.M[t] = A.fc_q * s;
+        }
+        for (int t = tid; t < NGV * NCU; t += QT) {
+            const int g = t % NGV, c = t / NGV;
+            double s = 0.0;
+#pragma unroll 4
+            for (int a = 0; a < NPV; a++) s = fma(__ldg(&T.shapvt[g + NGV * a]), sm.u[a + NPV * c], s);
+            sm.ug[t] = s;
+        }
+        for (int t = tid; t < NA * NCH; t += QT) {
+            const int gg = t % NA, c = t / NA, fc = gg / NGF, q = gg % NGF;
+            double s = 0.0;
+#pragma unroll 4
+            for (int m = 0; m < NPF; m++) s = fma(__ldg(&T.shapft[q + NGF * m]), sm.uhe[fc * NPF + m + NDF * c], s);
+            sm.uhq[t] = s * sm.jacf[gg];
+        }
+        __syncthreads();
+        // the last warp factors M while the others form the right-hand sides
+        if (tid >= QT - 32) {
+            cholesky_warp_rows<NPV>(sm.M, sm.rdg);
+        } else {
+            for (int t = tid; t < NPV * NCU * ND; t += QT - 32) {
+                const int i = t % NPV, c = (t / NPV) % NCU, d = t / (NPV * NCU);
+                double sp[ND];
+#pragma unroll
+                for (int r = 0; r < ND; r++) sp[r] = 0.0;
+#pragma unroll 4
+                for (int g = 0; g < NGV; g++) {
+                    const double v = sm.ug[g + NGV * c];
+#pragma unroll
+                    for (int r = 0; r < ND; r++)
+                        sp[r] = fma(__ldg(&T.shapvg[i + NPV * (g + NGV * (r + 1))]) * sm.Xx[g + NGV * (d + ND * r)], v,
+                                    sp[r]);
+                }
+                double s = 0.0;
+#pragma unroll
+                for (int r = 0; r < ND; r++) s += sp[r];
+                for (int k = 0; k < sm.inc_n[i]; k++) {
+                    const int f = sm.inc_f[i * S::MAXINC + k], fc = f / NPF, ip = f % NPF;
+                    double b = 0.0;
+#pragma unroll 4
+                    for (int q = 0; q < NGF; q++) {
+                        const int gg = q + NGF * fc;
+                        b = fma(__ldg(&T.shapfg[ip + NPF * q]) * sm.nl[gg + NA * d], sm.uhq[gg + NA * c], b);
+                    }
+                    s -= b;
+                }
+                sm.q[t] = s;
+            }
+        }
+        __syncthreads();
+        for (int t = tid; t < NCU * ND; t += QT) chol_solve_col_axpy<NPV>(sm.M, sm.rdg, &sm.q[NPV * t]);
         __syncthreads();
         const double* she = A.sh + (size_t)e * NPV * NC;
         for (int t = tid; t < NPV * NCU * ND; t += QT) {
             const int i = t % NPV, c = (t / NPV) % NCU, d = t / (NPV * NCU);
-            double s = 0.0;
-            for (int a = 0; a < NPV; a++) s += sm.M[i + NPV * a] * she[a + NPV * (NCU * (1 + d) + c)];
-            for (int a = 0; a < NPV; a++) s += sm.C[i + NPV * (a + NPV * d)] * sm.u[a + NPV * c];
-            for (int fn = 0; fn < NDF; fn++) s -= sm.E[i + NPV * (fn + NDF * d)] * sm.uhe[fn + NDF * c];
-            sm.q[t] = s;
-        }
-        __syncthreads();
-        cholesky_warp<NPV>(sm.M);
-        __syncthreads();
-        for (int t = tid; t < NCU * ND; t += QT) chol_solve_col<NPV>(sm.M, &sm.q[NPV * t]);
-        __syncthreads();
-        for (int t = tid; t < NPV * NCU * ND; t += QT) {
-            const int i = t % NPV, c = (t / NPV) % NCU, d = t / (NPV * NCU);
-            ue[i + NPV * (NCU * (1 + d) + c)] = sm.q[t];
+            const int at = i + NPV * (NCU * (1 + d) + c);
+            ue[at] = sm.q[t] + she[at];
         }
     }
 }

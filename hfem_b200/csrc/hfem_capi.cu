@@ -91,7 +91,7 @@ struct hfem_ctx {
     bool have_master = false, have_mesh = false, have_phys = false, have_sol = false, assembled = false;
     int grid_elem = 0, grid_inv = 0, grid_tc = 0;
     int grid_elem_v[2][2] = {};         // per element-kernel variant [tf][gen], at most grid_elem
-    int grid_res[2] = {};               // residual-only pass [gen]
+    int grid_res[2] = {}, grid_q = 0;   // residual-only pass [gen]; q recovery
     bool res_blocks = false;            // D, K, H, Rh of the last residual-only pass not formed yet (form_blocks)
     // element-wise state arriving in pieces (hfem_assemble_host): the element
     // kernel of piece k waits for chunk_ev[k]
@@ -638,7 +638,7 @@ int launch_getq(hfem_ctx* c, const double* duh, double alpha) {
     q.eprob = c->eprob;
     q.palpha = (duh && c->nprob && c->palpha_on) ? c->palpha : nullptr;
     Timed t(c, duh ? "update" : "getq");
-    c->L->getq(dim3(c->grid_elem), c->L->q_smem, c->stream, q);
+    c->L->getq(dim3(c->grid_q), c->L->q_smem, c->stream, q);
     return check_launch(c, "getq");
 }
 
@@ -1592,6 +1592,9 @@ int hfem_create(const hfem_dims* dims, int device, hfem_ctx** out) {
     }
     cudaFuncSetAttribute(L.q_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.q_smem);
     int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.q_fn, L.q_threads, L.q_smem);
+    c->grid_q = std::max(1, std::min(d.ne, sms(device) * std::max(occ, 1)));
+    occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.elem_fn, L.elem_threads, L.elem_smem);
     c->grid_elem = std::max(1, std::min(d.ne, sms(device) * std::max(occ, 1)));
     // the workspace has grid_elem slots: no variant runs more CTAs

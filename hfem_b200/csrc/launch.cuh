@@ -52,6 +52,7 @@ struct Launch {
     size_t ws, ws_tf;           // workspace doubles per CTA slot of element_kernel, FP64 and 3xTF32 forms
     int elem_threads;           // threads per CTA of the element kernels
     size_t q_smem;
+    int q_threads;
     void (*getq)(dim3, size_t, cudaStream_t, const QArgs&);
     void (*inverse)(dim3, cudaStream_t, int, double*, const double*, double*, int*);
     void (*element)(dim3, size_t, cudaStream_t, const ElemArgs&);

@@ -74,6 +74,7 @@ Launch make_launch() {
     L.ws = EK<S>::WS;
     L.ws_tf = EK<S>::WS_TF;
     L.q_smem = sizeof(QSmem<S>);
+    L.q_threads = QT;
     L.getq = launch_getq<S>;
     L.q_fn = (const void*)getq_kernel<S>;
     L.inverse = launch_inverse<S::N>;
