@@ -1093,6 +1093,17 @@ __global__ void gather_diag_kernel(int nrows, int b2, const int* __restrict__ ro
         out[t] = Hg[(size_t)rowstart[t / b2] * b2 + t % b2];
 }
 
+// Orders up to 32 by warps (inverse_warp_kernel), the others by CTAs.  Both kernels
+// also solve with a right-hand side: c->w is free here and its result is ignored.
+template <int B>
+int bj_warp(hfem_ctx* c) {
+    const int nf = c->dims.nf;
+    gather_diag_kernel<<<sms(c->device) * 8, 256, 0, c->stream>>>(nf, B * B, c->rowstart, c->Hg, c->Minv);
+    const int grid = std::min((nf + WINV_WARPS - 1) / WINV_WARPS, sms(c->device) * 16);
+    inverse_warp_kernel<B><<<grid, 32 * WINV_WARPS, 0, c->stream>>>(nf, c->Minv, c->w, c->w, c->binfo);
+    return check_launch(c, "bj_inverse");
+}
+
 template <int B>
 int bj_blocked(hfem_ctx* c) {
     cudaFuncSetAttribute(inverse_blocked_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InvBlk<B>::SMEM);
@@ -1101,31 +1112,25 @@ int bj_blocked(hfem_ctx* c) {
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, inverse_blocked_kernel<B>, InvBlk<B>::THREADS, InvBlk<B>::SMEM);
     const int grid = std::max(1, std::min(nf, sms(c->device) * std::max(occ, 1)));
-    // the kernel also solves with a right-hand side: c->w is free here and its
-    // result is ignored
     inverse_blocked_kernel<B><<<grid, InvBlk<B>::THREADS, InvBlk<B>::SMEM, c->stream>>>(nf, c->Minv, c->w, c->w,
                                                                                      c->binfo);
     return check_launch(c, "bj_inverse");
 }
 
 // Block-Jacobi factor: Minv_i = inv(Hg_ii) for every face row (binfo[i] = 1 +
-// pivot step of a singular block).  Block sizes with a blocked Gauss-Jordan
-// instance take it (diagonal blocks gathered first); the others the one-CTA-
-// per-block kernel.
+// pivot step of a singular block), the diagonal blocks gathered first.
 int bj_factor(hfem_ctx* c) {
     Timed t(c, "bj_inverse");
     switch (c->bsz) {
-        case 12: return bj_blocked<12>(c);
-        case 16: return bj_blocked<16>(c);
-        case 20: return bj_blocked<20>(c);
-        case 30: return bj_blocked<30>(c);
+        case 8: return bj_warp<8>(c);
+        case 12: return bj_warp<12>(c);
+        case 15: return bj_warp<15>(c);
+        case 16: return bj_warp<16>(c);
+        case 20: return bj_warp<20>(c);
+        case 30: return bj_warp<30>(c);
         case 50: return bj_blocked<50>(c);
-        default: break;
+        default: return fail(c, HFEM_E_UNSUPPORTED, "no block Jacobi for block size %d", c->bsz);
     }
-    const size_t smem = sizeof(double) * ((size_t)c->bsz * c->bsz + c->bsz) + sizeof(int) * c->bsz;
-    bj_inverse_kernel<<<std::min(c->dims.nf, sms(c->device) * 8), 64, smem, c->stream>>>(
-        c->dims.nf, c->bsz, c->rowstart, c->Hg, c->Minv, c->binfo);
-    return check_launch(c, "bj_inverse");
 }
 
 // z = xsc M^-1 Hg x (M^-1 omitted when !prec), rows of problems with
@@ -1617,7 +1622,7 @@ int hfem_create(const hfem_dims* dims, int device, hfem_ctx** out) {
     occ = 0;
     cudaFuncSetAttribute(L.inv_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.inv_smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, L.inv_fn, L.inv_threads, L.inv_smem);
-    c->grid_inv = std::max(1, std::min(d.ne, sms(device) * std::max(occ, 1)));
+    c->grid_inv = std::max(1, std::min((d.ne + L.inv_per_cta - 1) / L.inv_per_cta, sms(device) * std::max(occ, 1)));
     if (pool_alloc(device, (void**)&c->status, sizeof(PassStatus)) != cudaSuccess) {
         cudaStreamDestroy(c->own);
         delete c;
@@ -2577,7 +2582,7 @@ extern "C" int hfem_condense_noalloc(const hfem_dims* dims, const double* shapvt
             G.ready = true;
         }
         ge = std::min(d.ne, G.elem);
-        gi = std::min(d.ne, G.inv);
+        gi = std::min((d.ne + L->inv_per_cta - 1) / L->inv_per_cta, G.inv);
     }
     cudaStream_t st = (cudaStream_t)stream;
 

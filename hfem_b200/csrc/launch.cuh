@@ -66,7 +66,7 @@ struct Launch {
     int res_threads;
     const void* elem_fn;
     const void* elem_fn_v[2][2];
-    int inv_threads;
+    int inv_threads, inv_per_cta;
     size_t inv_smem;
     const void *q_fn, *inv_fn;
     GemmLaunch g1, g2;

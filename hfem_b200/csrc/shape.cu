@@ -25,7 +25,25 @@ template <> struct SchurCfg<Shape<3, 20, 10, 24, 12>> { using g1 = GemmCfg<5, 3,
 
 template <int N>
 void launch_inverse(dim3 g, cudaStream_t st, int ne, double* D, const double* Ru, double* RuOut, int* info) {
-    inverse_blocked_kernel<N><<<g, InvBlk<N>::THREADS, InvBlk<N>::SMEM, st>>>(ne, D, Ru, RuOut, info);
+    if constexpr (N <= 32)
+        inverse_warp_kernel<N><<<g, 32 * WINV_WARPS, 0, st>>>(ne, D, Ru, RuOut, info);
+    else
+        inverse_blocked_kernel<N><<<g, InvBlk<N>::THREADS, InvBlk<N>::SMEM, st>>>(ne, D, Ru, RuOut, info);
+}
+// threads, dynamic shared memory, matrices per CTA and the kernel itself
+template <int N>
+void inverse_launch(Launch& L) {
+    if constexpr (N <= 32) {
+        L.inv_threads = 32 * WINV_WARPS;
+        L.inv_smem = 0;
+        L.inv_per_cta = WINV_WARPS;
+        L.inv_fn = (const void*)inverse_warp_kernel<N>;
+    } else {
+        L.inv_threads = InvBlk<N>::THREADS;
+        L.inv_smem = InvBlk<N>::SMEM;
+        L.inv_per_cta = 1;
+        L.inv_fn = (const void*)inverse_blocked_kernel<N>;
+    }
 }
 
 template <class S, bool TF, bool GEN>
@@ -96,9 +114,7 @@ Launch make_launch() {
     L.elem_fn_v[0][1] = (const void*)element_kernel<S, false, true>;
     L.elem_fn_v[1][0] = (const void*)element_kernel<S, true, false>;
     L.elem_fn_v[1][1] = (const void*)element_kernel<S, true, true>;
-    L.inv_threads = InvBlk<S::N>::THREADS;
-    L.inv_smem = InvBlk<S::N>::SMEM;
-    L.inv_fn = (const void*)inverse_blocked_kernel<S::N>;
+    inverse_launch<S::N>(L);
     L.g1 = GemmParams<typename SchurCfg<S>::g1>::make();
     L.g2 = GemmParams<typename SchurCfg<S>::g2>::make();
     L.schur_tc = launch_schur_tc<S>;
