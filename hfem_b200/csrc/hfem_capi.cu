@@ -562,14 +562,12 @@ int enqueue_assembly(hfem_ctx* c, bool matrix) {
             if ((rc = check_launch(c, "gemv_Rh"))) return rc;
         }
         {
-            Timed t(c, "scatter_H");
+            Timed t(c, "scatter");
             c->L->scatter_h(dim3(std::max(1, std::min((c->dims.nblocks + 7) / 8, sms(c->device) * 8))), c->stream, sa);
             if ((rc = check_launch(c, "scatter_H"))) return rc;
         }
     } else {
         sa.Rg = nullptr;
-    }
-    {
         Timed t(c, "scatter_R");
         scatter_R_kernel<<<sms(c->device) * 4, 256, 0, c->stream>>>(sa);
         if ((rc = check_launch(c, "scatter_R"))) return rc;
