@@ -93,6 +93,7 @@ struct hfem_ctx {
     int grid_elem_v[2][2] = {};         // per element-kernel variant [tf][gen], at most grid_elem
     int grid_res[2] = {}, grid_q = 0;   // residual-only pass [gen]; q recovery
     bool res_blocks = false;            // D, K, H, Rh of the last residual-only pass not formed yet (form_blocks)
+    bool res_eager = false;             // a caller may see or change them unnoticed: formed after each call
     // element-wise state arriving in pieces (hfem_assemble_host): the element
     // kernel of piece k waits for chunk_ev[k]
     cudaStream_t copy_stream = nullptr;
@@ -495,6 +496,7 @@ int enqueue_assembly(hfem_ctx* c, bool matrix) {
         c->L->residual[gen](dim3(c->grid_res[gen]), c->L->res_smem, c->stream, elem_args(c));
         if ((rc = check_launch(c, "residual"))) return rc;
     } else {
+        c->res_blocks = false;
         Timed t(c, "element");
         if (c->pending_chunks > 0) {
             // one launch per piece of the state, each after that piece's copy
@@ -591,7 +593,7 @@ int finish_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
     if (st.wait_err == 1) return fail(c, HFEM_E_CUDA, "tensor-core Schur kernel: an MMA completion wait expired");
     if (st.wait_err == 2) return fail(c, HFEM_E_CUDA, "element kernel: a bulk-copy completion wait expired");
     if (matrix) c->assembled = true;
-    c->res_blocks = !matrix;
+    if (!matrix) c->res_blocks = true;
     flush_timer(c);
     if (rnorm_out) *rnorm_out = st.rnorm;
     return 0;
@@ -606,8 +608,12 @@ int run_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
 }
 
 // After a residual-only pass the element blocks are D, K, H and Rh at its state
-// (hfem_download); they are formed when one of them is asked for.
+// (hfem_download).  They are formed when one of them is asked for, before a call
+// that changes what they depend on (keep_blocks), and at the end of each call once
+// the caller holds a device pointer to them or to the state, or has captured the
+// context's assembly (res_eager).
 int form_blocks(hfem_ctx* c) {
+    CK(cudaSetDevice(c->device));
     const int tf = (c->precision == 1 || c->precision == 3) ? 1 : 0;
     const int gen = (c->conv_stab != 0 || c->visc_model != 0) ? 1 : 0;
     c->L->element_v[tf][gen](dim3(c->grid_elem_v[tf][gen]), c->L->elem_smem, c->stream, elem_args(c));
@@ -619,7 +625,6 @@ int form_blocks(hfem_ctx* c) {
 }
 
 int launch_getq(hfem_ctx* c, const double* duh, double alpha) {
-    c->res_blocks = false;
     QArgs q;
     q.T = Tables{c->shapvt, c->shapvg, c->svsv, c->shapft, c->shapfg, c->sfsf, c->perm};
     q.dgnodes = c->dgnodes;
@@ -639,6 +644,9 @@ int launch_getq(hfem_ctx* c, const double* duh, double alpha) {
     c->L->getq(dim3(c->grid_q), c->L->q_smem, c->stream, q);
     return check_launch(c, "getq");
 }
+
+int keep_blocks(hfem_ctx* c) { return c->res_blocks ? form_blocks(c) : 0; }
+int show_blocks(hfem_ctx* c) { return c->res_eager ? keep_blocks(c) : 0; }
 
 long long nvec(hfem_ctx* c) { return (long long)c->dims.nf * c->bsz; }
 
@@ -1682,6 +1690,7 @@ int hfem_set_master(hfem_ctx* c, const double* shapvt, const double* shapvg, con
         if (perm[i] < 0 || perm[i] >= d.npv) return fail(c, HFEM_E_ARG, "perm[%d] = %d out of range", i, perm[i]);
     int rc;
     CK(cudaSetDevice(c->device));
+    if (int rk = keep_blocks(c)) return rk;
     const size_t v1 = (size_t)d.ngv * d.npv * (d.nd + 1), v2 = (size_t)d.npv * d.npv * d.ngv * (d.nd + 1);
     const size_t f1 = (size_t)d.ngf * d.npf * d.nd, f2 = (size_t)d.npf * d.npf * d.ngf * d.nd;
     if ((rc = upload(c, &c->shapvt, shapvt, v1)) || (rc = upload(c, &c->shapvg, shapvg, v1)) ||
@@ -1740,6 +1749,7 @@ int hfem_set_mesh(hfem_ctx* c, const double* dgnodes, const int* elcon, const in
     }
     int rc;
     CK(cudaSetDevice(c->device));
+    if (int rk = keep_blocks(c)) return rk;
     std::vector<int> colface(colidx, colidx + nblk);
     if ((rc = upload(c, &c->dgnodes, dgnodes, (size_t)ne * d.npv * d.nd)) ||
         (rc = upload(c, &c->elcon, elcon, (size_t)ne * ndf)) || (rc = upload(c, &c->rowstart, rowstart, (size_t)nf + 1)) ||
@@ -1755,7 +1765,6 @@ int hfem_set_mesh(hfem_ctx* c, const double* dgnodes, const int* elcon, const in
     c->h_rowstart.assign(rowstart, rowstart + nf + 1);
     c->h_colidx.assign(colidx, colidx + nblk);
     c->have_order = false;
-    c->res_blocks = false;
     if (c->bf) { pool_free(c->bf); c->bf = nullptr; }      // boundary flags belong to the old mesh
     c->have_mesh = true;
     return 0;
@@ -1788,6 +1797,7 @@ int hfem_set_boundary(hfem_ctx* c, const int* bf, int nbnd, const int* bcm, cons
     }
     int rc;
     CK(cudaSetDevice(c->device));
+    if (int rk = keep_blocks(c)) return rk;
     if (!any) {
         if (c->bf) { pool_free(c->bf); c->bf = nullptr; }
         c->nbnd = 0;
@@ -1798,7 +1808,6 @@ int hfem_set_boundary(hfem_ctx* c, const int* bf, int nbnd, const int* bcm, cons
         return rc;
     CK(cudaStreamSynchronize(c->stream));
     c->nbnd = nbnd;
-    c->res_blocks = false;
     c->assembled = false;
     return 0;
 }
@@ -1807,8 +1816,8 @@ int hfem_set_app(hfem_ctx* c, int appname) {
     if (!c) return HFEM_E_ARG;
     if (appname != 0 && appname != 1)
         return fail(c, HFEM_E_UNSUPPORTED, "appname %d (supported: 0 Euler, 1 Navier-Stokes)", appname);
+    if (int rk = keep_blocks(c)) return rk;
     c->appname = appname;
-    c->res_blocks = false;
     c->assembled = false;
     return 0;
 }
@@ -1820,18 +1829,18 @@ int hfem_set_models(hfem_ctx* c, int conv_stab, int viscosity_model) {
                     conv_stab);
     if (viscosity_model < 0 || viscosity_model > 1)
         return fail(c, HFEM_E_UNSUPPORTED, "viscosityModel %d (supported: 0 constant, 1 Sutherland)", viscosity_model);
+    if (int rk = keep_blocks(c)) return rk;
     c->conv_stab = conv_stab;
     c->visc_model = viscosity_model;
-    c->res_blocks = false;
     c->assembled = false;
     return 0;
 }
 
 int hfem_set_physics(hfem_ctx* c, const double* param, int tdep, double fc_u, double fc_q, double time) {
     if (!c || !param) return HFEM_E_ARG;
-    c->res_blocks = false;
     if (!(param[0] > 1.0) || !(param[2] > 0.0) || !(param[3] > 0.0))
         return fail(c, HFEM_E_ARG, "physicsparam needs gamma > 1, Re > 0, Pr > 0");
+    if (int rk = keep_blocks(c)) return rk;
     for (int i = 0; i < 6; i++) c->param[i] = param[i];
     c->tdep = tdep;
     c->fc_u = fc_u;
@@ -1847,6 +1856,7 @@ static int set_solution_common(hfem_ctx* c, const double* udg, const double* uh,
     const size_t nudg = (size_t)d.ne * d.npv * c->nc, nuh = (size_t)d.nf * c->bsz;
     int rc;
     CK(cudaSetDevice(c->device));
+    if (int rk = keep_blocks(c)) return rk;
     if (!c->udg) {
         if ((rc = dalloc(c, &c->udg, nudg)) || (rc = dalloc(c, &c->uh, nuh)) || (rc = dalloc(c, &c->sh, nudg))) return rc;
     }
@@ -1856,7 +1866,6 @@ static int set_solution_common(hfem_ctx* c, const double* udg, const double* uh,
     else CK(cudaMemsetAsync(c->sh, 0, sizeof(double) * nudg, c->stream));
     c->have_sol = true;
     c->assembled = false;
-    c->res_blocks = false;
     return 0;
 }
 
@@ -1928,6 +1937,7 @@ int hfem_get_solution(hfem_ctx* c, double* udg, double* uh) {
 int hfem_getq(hfem_ctx* c) {
     int rc = ready(c);
     if (rc) return rc;
+    if (int rk = keep_blocks(c)) return rk;
     if ((rc = launch_getq(c, nullptr, 0.0))) return rc;
     CK(cudaStreamSynchronize(c->stream));
     flush_timer(c);
@@ -1937,7 +1947,10 @@ int hfem_getq(hfem_ctx* c) {
 
 int hfem_assemble(hfem_ctx* c, double* rnorm) { return run_assembly(c, true, rnorm); }
 
-int hfem_residual(hfem_ctx* c, double* rnorm) { return run_assembly(c, false, rnorm); }
+int hfem_residual(hfem_ctx* c, double* rnorm) {
+    const int rc = run_assembly(c, false, rnorm);
+    return rc ? rc : show_blocks(c);
+}
 
 int hfem_gmres(hfem_ctx* c, int precond, int restart, double tol, int maxit, int* conv, int* iters, double* hist,
                int hist_len) {
@@ -1947,13 +1960,14 @@ int hfem_gmres(hfem_ctx* c, int precond, int restart, double tol, int maxit, int
 
 int hfem_update(hfem_ctx* c, double alpha) {
     if (!c) return HFEM_E_ARG;
+    if (int rk = keep_blocks(c)) return rk;
     return update_impl(c, alpha);
 }
 
 // solveNonlinearProblem (solvers/dgsolvers.cpp:106-205), damped Newton with the
 // reference's line search: halve alpha (stepping back from the previous trial)
 // while the residual grows, down to alphaMin = 1e-4.
-int hfem_newton(hfem_ctx* c, double newton_tol, int newton_maxiter, int precond, int restart, double gmres_tol,
+static int newton_impl(hfem_ctx* c, double newton_tol, int newton_maxiter, int precond, int restart, double gmres_tol,
                 int gmres_maxit, double* hist, int hist_len, int* niter, int* converged) {
     if (!c) return HFEM_E_ARG;
     int rc = ready(c);
@@ -1986,6 +2000,7 @@ int hfem_newton(hfem_ctx* c, double newton_tol, int newton_maxiter, int precond,
                     if (robust == 0) {
                         robust = 1;
                         alpha = -2.0 * std::fabs(alpha);
+                        if ((rc = keep_blocks(c))) return rc;
                         if ((rc = update_impl(c, alpha))) return rc;
                     }
                     break;
@@ -2001,13 +2016,21 @@ int hfem_newton(hfem_ctx* c, double newton_tol, int newton_maxiter, int precond,
     return 0;
 }
 
+int hfem_newton(hfem_ctx* c, double newton_tol, int newton_maxiter, int precond, int restart, double gmres_tol,
+                int gmres_maxit, double* hist, int hist_len, int* niter, int* converged) {
+    const int rc = newton_impl(c, newton_tol, newton_maxiter, precond, restart, gmres_tol, gmres_maxit, hist, hist_len,
+                               niter, converged);
+    const int rs = c ? show_blocks(c) : 0;
+    return rc ? rc : rs;
+}
+
 // One time step of solveUnsteadyProblem (solvers/dgsolvers.cpp:221-444): for
 // each DIRK stage set time = t + dt c_i, fc_u = d_ii/dt, fc_q = 1, form the
 // stage source SH from the step's initial state and the previous stage
 // (dgsolvers.cpp:319-348, q part zeroed) and solve the stage with the Newton
 // driver.  A stage that does not converge returns HFEM_E_SINGULAR (the
 // reference calls error() and exits).
-int hfem_dirk_step(hfem_ctx* c, double dt, int stages, int order, double newton_tol, int newton_maxiter,
+static int dirk_impl(hfem_ctx* c, double dt, int stages, int order, double newton_tol, int newton_maxiter,
                    int precond, int restart, double gmres_tol, int gmres_maxit, int* newton_iters) {
     if (!c) return HFEM_E_ARG;
     int rc = ready(c);
@@ -2015,6 +2038,7 @@ int hfem_dirk_step(hfem_ctx* c, double dt, int stages, int order, double newton_
     double d[9], t[3];
     if (!(dt > 0.0) || !dirk_table(stages, order, d, t))
         return fail(c, HFEM_E_ARG, "unsupported DIRK(%d,%d) or dt <= 0", stages, order);
+    if (newton_maxiter < 1 && (rc = keep_blocks(c))) return rc;     // else the first assembly replaces them
     const hfem_dims& dm = c->dims;
     const long long n = (long long)dm.ne * dm.npv * c->nc;
     if (!c->udgi && (rc = dalloc(c, &c->udgi, (size_t)n))) return rc;
@@ -2043,7 +2067,7 @@ int hfem_dirk_step(hfem_ctx* c, double dt, int stages, int order, double newton_
         c->fc_q = 1.0;
         c->tdep = 1;
         int it = 0, conv = 0;
-        if ((rc = hfem_newton(c, newton_tol, newton_maxiter, precond, restart, gmres_tol, gmres_maxit, nullptr, 0,
+        if ((rc = newton_impl(c, newton_tol, newton_maxiter, precond, restart, gmres_tol, gmres_maxit, nullptr, 0,
                               &it, &conv)))
             return rc;
         total_iters += it;
@@ -2055,6 +2079,14 @@ int hfem_dirk_step(hfem_ctx* c, double dt, int stages, int order, double newton_
     c->time = t0 + dt;
     if (newton_iters) *newton_iters = total_iters;
     return 0;
+}
+
+int hfem_dirk_step(hfem_ctx* c, double dt, int stages, int order, double newton_tol, int newton_maxiter, int precond,
+                   int restart, double gmres_tol, int gmres_maxit, int* newton_iters) {
+    const int rc = dirk_impl(c, dt, stages, order, newton_tol, newton_maxiter, precond, restart, gmres_tol, gmres_maxit,
+                             newton_iters);
+    const int rs = c ? show_blocks(c) : 0;
+    return rc ? rc : rs;
 }
 
 // Several independent problems packed into this context's mesh (a disjoint
@@ -2070,6 +2102,7 @@ int hfem_set_problem_map(hfem_ctx* c, int nprob, const int* eprob, const int* fp
         if (fprob[f] < 0 || fprob[f] >= nprob) return fail(c, HFEM_E_ARG, "fprob[%d] out of range", f);
     int rc;
     CK(cudaSetDevice(c->device));
+    if (int rk = keep_blocks(c)) return rk;
     if ((rc = upload(c, &c->eprob, eprob, (size_t)d.ne)) || (rc = upload(c, &c->fprob, fprob, (size_t)d.nf)) ||
         (rc = upload(c, &c->pparam, params, (size_t)nprob * 8)) || (rc = dalloc(c, &c->palpha, (size_t)nprob)))
         return rc;
@@ -2124,6 +2157,7 @@ int hfem_update_problems(hfem_ctx* c, const double* alpha) {
     if (!c || !alpha) return HFEM_E_ARG;
     if (!c->nprob) return fail(c, HFEM_E_STATE, "no problem map");
     if (!c->assembled || !c->x) return fail(c, HFEM_E_STATE, "assemble and solve before update");
+    if (int rk = keep_blocks(c)) return rk;
     int rc;
     CK(cudaMemcpyAsync(c->palpha, alpha, sizeof(double) * c->nprob, cudaMemcpyHostToDevice, c->stream));
     axpy_prob_kernel<<<sms(c->device) * 4, 256, 0, c->stream>>>(nvec(c), c->bsz, c->fprob, c->palpha, c->x, c->uh);
@@ -2256,6 +2290,8 @@ int hfem_graph_capture(hfem_ctx** ctxs, int n, void* stream, hfem_graph** out) {
         int rc = ready(ctxs[i]);
         if (rc) return rc;
         if ((rc = ensure_assembly_buffers(ctxs[i]))) return rc;
+        if ((rc = keep_blocks(ctxs[i]))) return rc;
+        ctxs[i]->res_eager = true;          // a launch of the graph does not pass through the context
         CK(cudaStreamSynchronize(ctxs[i]->stream));
     }
     CK(cudaSetDevice(c0->device));
@@ -2363,8 +2399,8 @@ int hfem_set_precision(hfem_ctx* c, int mode) {
         return fail(c, HFEM_E_ARG, "precision mode must be 0 (FP64), 1 (3xTF32 element contractions, TF32 Schur, "
                                    "FP32 preconditioner), 2 (FP32 preconditioner) or 3 (3xTF32 element "
                                    "contractions, FP32 preconditioner)");
+    if (int rk = keep_blocks(c)) return rk;
     c->precision = mode;
-    c->res_blocks = false;
     c->assembled = false;
     return 0;
 }
@@ -2403,6 +2439,10 @@ int device_buffer(hfem_ctx* c, int what, const double** src, size_t* need) {
 
 int hfem_device_buffer(hfem_ctx* c, int what, const double** ptr, size_t* count) {
     if (!c || !ptr || !count) return HFEM_E_ARG;
+    if (what == 5 || what == 6 || what == 8 || what == 9 || what == 10 || what == 13) {
+        if (int rk = keep_blocks(c)) return rk;
+        c->res_eager = true;
+    }
     CK(cudaStreamSynchronize(c->stream));
     return device_buffer(c, what, ptr, count);
 }

@@ -266,11 +266,11 @@ int hfem_gmres_problems(hfem_ctx* ctx, int precond, int restart, double tol, int
  * (nb*nb*ne), 6 condensed element Rh (nb*ne), 7 GMRES solution x (nf*bsz),
  * 10 element K (nb*n*ne), 12 element Rh before condensation (nb*ne),
  * 13 element D^-1 after an
- * assembly (n*n*ne; D itself after a residual-only pass), 14 ||Ru_e||^2 before
- * condensation (ne).  hfem_residual forms no element blocks; 5, 6, 10 and 13
- * asked for after it are H, Rh and K before condensation and D, formed then, as
- * long as the state it was taken at is unchanged (after a change: the blocks of
- * the last assembly). */
+ * assembly (n*n*ne), 14 ||Ru_e||^2 before condensation (ne).  After a
+ * residual-only pass 5, 6 and 10 are before condensation and 13 is D itself, at
+ * the state of that pass (hfem_residual forms them when they are asked for or
+ * before what they depend on changes, or at once in a context whose element
+ * blocks or state hfem_device_buffer has handed out or which is part of a graph). */
 int hfem_download(hfem_ctx* ctx, int what, double* host, size_t count);
 
 /* Per-kernel device time (ms) accumulated since the last reset, when timing
