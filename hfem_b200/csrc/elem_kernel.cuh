@@ -1,6 +1,6 @@
 // Element assembly on the FP64 tensor cores (sm_100a, mma.sync m8n8k4 f64).
 //
-// One CTA owns one element at a time (persistent grid, 2 CTAs per SM).  Every
+// One CTA owns one element at a time (persistent grid, 512 threads per SM).  Every
 // contraction after the pointwise fluxes is a GEMM with rows over (test node,
 // equation, variable) and a B operand resident in shared memory (restating
 // elementassembly.cpp elementint 307-572 and faceint 717-1321):
@@ -22,6 +22,14 @@
 // whose trace rows take the boundary flux while their element rows keep fhat,
 // are lifted here in full.  The face mass product uses shapfgdotshapfc = shapfg .* shapfc (its
 // definition, mkmasterelement.m:113-115) in factored form.
+//
+// Bound by no one unit: of 330k cycles per tetrahedron p = 3 the face rows take 123k
+// (their stores of K and H and the reductions into D, not the products), the volume
+// product 90k (A fragments formed from wrl as they are used), flux and Cholesky 33k,
+// the B operands 41k.  Before -> now (ms), Y and dual-number flux columns in memory
+// against fragments on the fly and flux Jacobians contracted as they are formed:
+// 13,182 3D p3 10.4 -> 7.7; 7,938 2D p4 1.22 -> 0.65; 2,048 2D p2 0.134 -> 0.066.  The
+// 3xTF32 form keeps Y and the dual-number flux, so that its results do not change.
 #pragma once
 #include <cuda_runtime.h>
 #include <type_traits>
