@@ -26,6 +26,11 @@ __device__ __forceinline__ void bulk_bar_init(uint64_t* bar) {
 // later async-proxy (bulk copy) writes to it
 __device__ __forceinline__ void bulk_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// orders this thread's earlier stores to global memory before later bulk loads from
+// it; every thread that stored runs it, ahead of the CTA barrier that precedes the
+// load (a barrier orders the generic proxy alone)
+__device__ __forceinline__ void bulk_proxy_fence_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+
 __device__ __forceinline__ void bulk_bar_expect(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bulk_smem_addr(bar)), "r"(bytes)
                  : "memory");

@@ -582,6 +582,8 @@ __global__ void __launch_bounds__(S::NT, 512 / S::NT) element_kernel(ElemArgs A)
         }
         boundary_fluxes(tid, NT);
         }
+        // the faces' Jacobian slices are read back by bulk copies (face_rows)
+        bulk_proxy_fence_global();
         __syncthreads();
         // M^-1 C and M^-1 E in place, one column per thread
         for (int t = tid; t < NPV * ND + NDF * ND; t += NT) chol_solve_col_axpy<NPV>(M, sm.rdg, &Cm[NPV * t]);
