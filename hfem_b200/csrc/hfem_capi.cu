@@ -1478,8 +1478,13 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
     }
     std::vector<int> its(P);
     CK(cudaMemcpyAsync(its.data(), c->gm_its, sizeof(int) * P, cudaMemcpyDeviceToHost, c->stream));
-    if (want_hist) CK(cudaMemcpyAsync(hist, c->gm_hist, sizeof(double) * hist_len, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    // the iterations' entries alone: what lies past them was not written by this call
+    if (want_hist && its[0] > 0) {
+        const size_t done = std::min(its[0], hist_len);
+        CK(cudaMemcpyAsync(hist, c->gm_hist, sizeof(double) * done, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+    }
     flush_timer(c);
     for (int p = 0; p < P; p++) {
         if (conv) conv[p] = state[p] == 1 ? 1 : (state[p] == 0 ? 0 : -1);
