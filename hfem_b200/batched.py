@@ -76,8 +76,8 @@ def autotune(solver, key, device=0, reps=3, cache=CACHE, refresh=False):
 class MixedOrderAssembly:
     """All meshes' assembly as one graph launch (one context per element shape).
 
-    precision 1 with tune: the TF32 condensation on the shapes where it is
-    faster than the tuned FP64 kernels (the others stay FP64, `fp64_shapes`)."""
+    precision 1 with tune: mixed precision on the shapes where its kernels are
+    faster than the tuned FP64 ones (the others stay FP64, `fp64_shapes`)."""
 
     def __init__(self, probs, device=0, precision=0, tune=True, stream=None):
         import torch
@@ -97,7 +97,7 @@ class MixedOrderAssembly:
                 self.tiles[k] = autotune(b.s, f"{k[0]}d_p{k[1]}", device=device)[:2]
             b.s.set_precision(precision)
             if tune and precision == 1 and not self._tf32_pays(b):
-                b.s.set_precision(0)         # this shape's tuned FP64 condensation is faster
+                b.s.set_precision(0)         # this shape's tuned FP64 kernels are faster
                 self.fp64_shapes.append(k)
             self.solvers.append(b)
         self.ne = sum(p.mesh.ne for p in probs)
@@ -110,11 +110,15 @@ class MixedOrderAssembly:
             raise HfemError(f"graph capture failed ({rc}): {msg}")
         self.graph = g
 
+    # what differs between the two modes: the element kernel's arithmetic, and the
+    # condensation with the passes around it (the FP64 kernel has the lift and Rh inside)
+    MODE_KERNELS = ("element", "lift_F", "schur_tc", "schur_fused", "gemm_DinvF", "gemm_schur", "gemv_Rh")
+
     @staticmethod
     def _tf32_pays(b, reps=2):
-        """Time the condensation of one shape both ways (the TF32 tensor-core
-        kernel against the tuned FP64 kernels); True when TF32 is faster."""
-        def cond_ms(prec):
+        """Time the kernels of one shape that differ between FP64 and mixed
+        precision both ways; True when mixed precision is faster."""
+        def mode_ms(prec):
             b.s.set_precision(prec)
             b.s.assembleLinearSystem()
             b.s.set_timing(True)
@@ -122,8 +126,8 @@ class MixedOrderAssembly:
                 b.s.assembleLinearSystem()
             kt = b.s.kernel_times()
             b.s.set_timing(False)
-            return sum(v[0] for k, v in kt.items() if k in ("schur_tc", "schur_fused", "gemm_DinvF", "gemm_schur"))
-        t_fp64, t_tf32 = cond_ms(0), cond_ms(1)
+            return sum(v[0] for k, v in kt.items() if k in MixedOrderAssembly.MODE_KERNELS)
+        t_fp64, t_tf32 = mode_ms(0), mode_ms(1)
         return t_tf32 < t_fp64
 
     def launch(self):
