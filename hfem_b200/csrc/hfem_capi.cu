@@ -475,6 +475,14 @@ int lift_F(hfem_ctx* c) {
     return check_launch(c, "lift_F");
 }
 
+// Rh -= K (D^-1 Ru), after the batched GEMMs or the tensor-core condensation.
+int gemv_Rh(hfem_ctx* c) {
+    Timed t(c, "gemv_Rh");
+    batched_dgemv_kernel<<<sms(c->device) * 8, 256, 0, c->stream>>>(
+        c->dims.ne, c->nb, c->n, -1.0, c->K, (long long)c->nb * c->n, c->DinvRu, c->n, c->Rh, c->nb);
+    return check_launch(c, "gemv_Rh");
+}
+
 int ready(hfem_ctx* c) {
     if (!c) return HFEM_E_ARG;
     if (!c->have_master || !c->have_mesh || !c->have_phys || !c->have_sol)
@@ -557,12 +565,7 @@ int enqueue_assembly(hfem_ctx* c, bool matrix) {
             c->L->schur_tc(dim3(c->grid_tc), c->L->tc_smem, c->stream, ta);
             if ((rc = check_launch(c, "schur_tc"))) return rc;
         }
-        if (!fused) {
-            Timed t(c, "gemv_Rh");
-            batched_dgemv_kernel<<<sms(c->device) * 8, 256, 0, c->stream>>>(ne, nb, n, -1.0, c->K, (long long)nb * n,
-                                                                           c->DinvRu, n, c->Rh, nb);
-            if ((rc = check_launch(c, "gemv_Rh"))) return rc;
-        }
+        if (!fused && (rc = gemv_Rh(c))) return rc;
         {
             Timed t(c, "scatter");
             c->L->scatter_h(dim3(std::max(1, std::min((c->dims.nblocks + 7) / 8, sms(c->device) * 8))), c->stream, sa);
@@ -2242,20 +2245,20 @@ int hfem_autotune(hfem_ctx* c, int reps, int* best, double* ms) {
             if (ms) ms[which * cand.size() + k] = per;
             if (per < bt[which]) bt[which] = per, bi[which] = (int)k;
         }
-    // the pair needs the lift pass in front of it
-    double lift = 0.0;
-    {
-        if ((rc = lift_F(c))) return rc;                   // warm-up
+    // the pair needs the lift pass in front of it and the Rh pass behind it
+    double around = 0.0;
+    for (int (*pass)(hfem_ctx*) : {lift_F, gemv_Rh}) {
+        if ((rc = pass(c))) return rc;                     // warm-up
         CK(cudaEventRecord(e0, c->stream));
         for (int r = 0; r < reps; r++)
-            if ((rc = lift_F(c))) return rc;
+            if ((rc = pass(c))) return rc;
         CK(cudaEventRecord(e1, c->stream));
         CK(cudaEventSynchronize(e1));
         float t = 0.f;
         CK(cudaEventElapsedTime(&t, e0, e1));
-        lift = (double)t / reps;
+        around += (double)t / reps;
     }
-    // the fused kernel does both products and the lift: kept when it beats them
+    // the fused kernel does both products, the lift and Rh: kept when it beats them
     {
         c->L->schur_fused(c->stream, fused_args(c));       // warm-up
         if ((rc = check_launch(c, "autotune"))) return rc;
@@ -2265,7 +2268,7 @@ int hfem_autotune(hfem_ctx* c, int reps, int* best, double* ms) {
         CK(cudaEventSynchronize(e1));
         float t = 0.f;
         CK(cudaEventElapsedTime(&t, e0, e1));
-        if ((double)t / reps <= bt[0] + bt[1] + lift) bi[0] = bi[1] = -1;
+        if ((double)t / reps <= bt[0] + bt[1] + around) bi[0] = bi[1] = -1;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
