@@ -94,6 +94,7 @@ struct hfem_ctx {
     int grid_res[2] = {}, grid_q = 0;   // residual-only pass [gen]; q recovery
     bool res_blocks = false;            // D, K, H, Rh of the last residual-only pass not formed yet (form_blocks)
     bool res_eager = false;             // a caller may see or change them unnoticed: formed after each call
+    double* res_tmp = nullptr;          // form_blocks: what it does not keep of the element kernel's vectors
     // element-wise state arriving in pieces (hfem_assemble_host): the element
     // kernel of piece k waits for chunk_ev[k]
     cudaStream_t copy_stream = nullptr;
@@ -585,6 +586,12 @@ int enqueue_assembly(hfem_ctx* c, bool matrix) {
     return check_launch(c, "pass_status");
 }
 
+int wait_failure(hfem_ctx* c, int err) {
+    if (err == 1) return fail(c, HFEM_E_CUDA, "tensor-core Schur kernel: an MMA completion wait expired");
+    if (err == 2) return fail(c, HFEM_E_CUDA, "element kernel: a bulk-copy completion wait expired");
+    return 0;
+}
+
 // Wait for an enqueued assembly, check the element LUs (and the tensor-core
 // kernel) and read the residual norm.
 int finish_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
@@ -593,8 +600,7 @@ int finish_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
     CK(cudaStreamSynchronize(c->stream));
     if (matrix && st.bad_elem >= 0)
         return fail(c, HFEM_E_SINGULAR, "element %d: singular local matrix (pivot %d)", st.bad_elem, st.bad_pivot);
-    if (st.wait_err == 1) return fail(c, HFEM_E_CUDA, "tensor-core Schur kernel: an MMA completion wait expired");
-    if (st.wait_err == 2) return fail(c, HFEM_E_CUDA, "element kernel: a bulk-copy completion wait expired");
+    if (int rw = wait_failure(c, st.wait_err)) return rw;
     if (matrix) c->assembled = true;
     if (!matrix) c->res_blocks = true;
     flush_timer(c);
@@ -615,15 +621,30 @@ int run_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
 // that changes what they depend on (keep_blocks), and at the end of each call once
 // the caller holds a device pointer to them or to the state, or has captured the
 // context's assembly (res_eager).
+// What the residual pass itself wrote (its rows Ro and ||Ru||^2, summed in another
+// order by the element kernel) stays as it is, and Rh is Ro.
 int form_blocks(hfem_ctx* c) {
     CK(cudaSetDevice(c->device));
     const int tf = (c->precision == 1 || c->precision == 3) ? 1 : 0;
     const int gen = (c->conv_stab != 0 || c->visc_model != 0) ? 1 : 0;
-    c->L->element_v[tf][gen](dim3(c->grid_elem_v[tf][gen]), c->L->elem_smem, c->stream, elem_args(c));
-    int rc = check_launch(c, "element");
-    if (rc) return rc;
-    c->res_blocks = false;
+    const size_t ne = c->dims.ne, nr = ne * c->nb;
+    int rc;
+    if (!c->res_tmp && (rc = dalloc(c, &c->res_tmp, nr + ne))) return rc;
+    ElemArgs a = elem_args(c);
+    a.Rh = a.Ro = c->res_tmp;
+    a.ru2 = c->res_tmp + nr;
+    {
+        Timed t(c, "element_blocks");
+        c->L->element_v[tf][gen](dim3(c->grid_elem_v[tf][gen]), c->L->elem_smem, c->stream, a);
+        if ((rc = check_launch(c, "element"))) return rc;
+    }
+    CK(cudaMemcpyAsync(c->Rh, c->Ro, sizeof(double) * nr, cudaMemcpyDeviceToDevice, c->stream));
+    int err = 0;
+    CK(cudaMemcpyAsync(&err, c->tc_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    flush_timer(c);
+    if ((rc = wait_failure(c, err))) return rc;
+    c->res_blocks = false;
     return 0;
 }
 
@@ -1658,7 +1679,7 @@ int hfem_destroy(hfem_ctx* c) {
     cudaStreamSynchronize(c->stream);
     void* ptrs[] = {c->shapvt, c->shapvg, c->svsv, c->shapft, c->shapfg, c->sfsf, c->perm, c->dgnodes, c->elcon,
                     c->rowstart, c->colidx, c->blk_src, c->face_src, c->rowface, c->colface, c->udg, c->uh, c->sh,
-                    c->D, c->F, c->K, c->H, c->Ru, c->DinvRu, c->Rh, c->Ro, c->ru2, c->Hg, c->Rg, c->Rr, c->status, c->ws, c->DinvF,
+                    c->D, c->F, c->K, c->H, c->Ru, c->DinvRu, c->Rh, c->Ro, c->ru2, c->Hg, c->Rg, c->Rr, c->status, c->ws, c->res_tmp, c->DinvF,
                     c->info, c->Minv, c->V, c->w, c->x, c->pb, c->binfo, c->udgi,
                     c->eprob, c->fprob, c->pparam, c->palpha, c->seg_one.pstart, c->seg_one.pseg, c->seg_one.p0,
                     c->seg_one.ticket, c->seg_one.part, c->seg_map.pstart, c->seg_map.pseg, c->seg_map.p0,
