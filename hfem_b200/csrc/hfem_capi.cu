@@ -7,11 +7,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <queue>
 #include <string>
@@ -81,6 +83,9 @@ struct SegTab {
     size_t cyc_part_n = 0;
 };
 
+// Launches of graphs that hold a context's assembly: they pass the context by.
+using GraphRuns = std::atomic<unsigned long long>;
+
 struct hfem_ctx {
     hfem_dims dims{};
     int device = 0;
@@ -92,9 +97,18 @@ struct hfem_ctx {
     int grid_elem = 0, grid_inv = 0, grid_tc = 0;
     int grid_elem_v[2][2] = {};         // per element-kernel variant [tf][gen], at most grid_elem
     int grid_res[2] = {}, grid_q = 0;   // residual-only pass [gen]; q recovery
-    bool res_blocks = false;            // D, K, H, Rh of the last residual-only pass not formed yet (form_blocks)
-    bool res_eager = false;             // a caller may see or change them unnoticed: formed after each call
-    double* res_tmp = nullptr;          // form_blocks: what it does not keep of the element kernel's vectors
+    // D, K, H, Rh of the last residual-only pass (form_blocks): not formed yet, and from what
+    bool res_blocks = false;
+    bool res_eager = false;             // a caller may read or change them unnoticed: formed after each call
+    bool res_track = false;             // a caller may change u and uhat unnoticed: set aside after each call
+    int res_saved = 0;                  // of the pass's inputs, set aside: 1 u and uhat, 2 the source
+    int res_tf = 0, res_gen = 0;
+    unsigned long long res_runs = 0;    // *runs at the pass
+    ElemArgs res_args;
+    double *res_udg = nullptr, *res_uh = nullptr, *res_sh = nullptr;
+    cudaEvent_t res_ev = nullptr;       // after the copies
+    double* res_tmp = nullptr;          // what form_blocks does not keep of the element kernel's vectors
+    std::shared_ptr<GraphRuns> runs = std::make_shared<GraphRuns>(0);
     // element-wise state arriving in pieces (hfem_assemble_host): the element
     // kernel of piece k waits for chunk_ev[k]
     cudaStream_t copy_stream = nullptr;
@@ -602,50 +616,109 @@ int finish_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
         return fail(c, HFEM_E_SINGULAR, "element %d: singular local matrix (pivot %d)", st.bad_elem, st.bad_pivot);
     if (int rw = wait_failure(c, st.wait_err)) return rw;
     if (matrix) c->assembled = true;
-    if (!matrix) c->res_blocks = true;
     flush_timer(c);
     if (rnorm_out) *rnorm_out = st.rnorm;
     return 0;
 }
 
-int run_assembly(hfem_ctx* c, bool matrix, double* rnorm_out) {
+// After a residual-only pass the element blocks are D, K, H and Rh at its state
+// (hfem_download).  They are formed when one of them is asked for, from the inputs of
+// the pass: the scalars and pointers are noted with it, u, uhat and the source set
+// aside before a call that changes them (500 doubles per tetrahedron p = 3, where the
+// blocks have 70,000).  Once a caller holds a device pointer to u or uhat, those are set
+// aside at the end of each call; once it holds one to a block, or has captured a pass
+// into a graph of its own, the blocks are formed there.  A launch of hfem_graph_launch
+// after the pass replaces its blocks.
+bool blocks_pending(const hfem_ctx* c) { return c->res_blocks && c->res_runs == *c->runs; }
+
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
+
+// The inputs of the last residual-only pass that are not set aside yet; what: 1 u and
+// uhat, 2 the source.
+int set_aside(hfem_ctx* c, int what) {
+    const size_t nu = (size_t)c->dims.ne * c->dims.npv * c->nc, nuh = (size_t)c->dims.nf * c->bsz;
+    const int todo = what & ~c->res_saved;
+    int rc;
+    if (todo & 1) {
+        if (!c->res_udg && ((rc = dalloc(c, &c->res_udg, nu)) || (rc = dalloc(c, &c->res_uh, nuh)))) return rc;
+        CK(cudaMemcpyAsync(c->res_udg, c->udg, sizeof(double) * nu, cudaMemcpyDeviceToDevice, c->stream));
+        CK(cudaMemcpyAsync(c->res_uh, c->uh, sizeof(double) * nuh, cudaMemcpyDeviceToDevice, c->stream));
+        c->res_args.udg = c->res_udg;
+        c->res_args.uh = c->res_uh;
+    }
+    if (todo & 2) {
+        if (!c->res_sh && (rc = dalloc(c, &c->res_sh, nu))) return rc;
+        CK(cudaMemcpyAsync(c->res_sh, c->sh, sizeof(double) * nu, cudaMemcpyDeviceToDevice, c->stream));
+        c->res_args.sh = c->res_sh;
+    }
+    if (todo) {
+        if (!c->res_ev) CK(cudaEventCreateWithFlags(&c->res_ev, cudaEventDisableTiming));
+        CK(cudaEventRecord(c->res_ev, c->stream));
+    }
+    c->res_saved |= todo;
+    return 0;
+}
+
+// aside: a residual-only pass whose u and uhat are set aside with it
+int run_assembly(hfem_ctx* c, bool matrix, double* rnorm_out, bool aside = false) {
     int rc = ready(c);
     if (rc) return rc;
     if ((rc = ensure_assembly_buffers(c))) return rc;
+    c->res_blocks = false;
     if ((rc = enqueue_assembly(c, matrix))) return rc;
-    return finish_assembly(c, matrix, rnorm_out);
+    if (!matrix) {
+        c->res_args = elem_args(c);
+        c->res_tf = (c->precision == 1 || c->precision == 3) ? 1 : 0;
+        c->res_gen = (c->conv_stab != 0 || c->visc_model != 0) ? 1 : 0;
+        c->res_runs = *c->runs;
+        c->res_saved = 0;
+        if (aside && (rc = set_aside(c, 1))) return rc;
+    }
+    if ((rc = finish_assembly(c, matrix, rnorm_out))) return rc;
+    c->res_blocks = !matrix;
+    return 0;
 }
 
-// After a residual-only pass the element blocks are D, K, H and Rh at its state
-// (hfem_download).  They are formed when one of them is asked for, before a call
-// that changes what they depend on (keep_blocks), and at the end of each call once
-// the caller holds a device pointer to them or to the state, or has captured the
-// context's assembly (res_eager).
 // What the residual pass itself wrote (its rows Ro and ||Ru||^2, summed in another
 // order by the element kernel) stays as it is, and Rh is Ro.
 int form_blocks(hfem_ctx* c) {
     CK(cudaSetDevice(c->device));
-    const int tf = (c->precision == 1 || c->precision == 3) ? 1 : 0;
-    const int gen = (c->conv_stab != 0 || c->visc_model != 0) ? 1 : 0;
     const size_t ne = c->dims.ne, nr = ne * c->nb;
     int rc;
-    if (!c->res_tmp && (rc = dalloc(c, &c->res_tmp, nr + ne))) return rc;
-    ElemArgs a = elem_args(c);
-    a.Rh = a.Ro = c->res_tmp;
-    a.ru2 = c->res_tmp + nr;
-    {
-        Timed t(c, "element_blocks");
-        c->L->element_v[tf][gen](dim3(c->grid_elem_v[tf][gen]), c->L->elem_smem, c->stream, a);
-        if ((rc = check_launch(c, "element"))) return rc;
-    }
-    CK(cudaMemcpyAsync(c->Rh, c->Ro, sizeof(double) * nr, cudaMemcpyDeviceToDevice, c->stream));
-    int err = 0;
-    CK(cudaMemcpyAsync(&err, c->tc_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    flush_timer(c);
-    if ((rc = wait_failure(c, err))) return rc;
-    c->res_blocks = false;
-    return 0;
+    // while the caller captures the stream: outside the capture, on the context's own
+    // stream (the pass itself has been waited for)
+    const bool aside = capturing(c->stream);
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (aside) CK(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaStream_t saved = c->stream;
+    if (aside) c->stream = c->own;
+    auto form = [&]() -> int {
+        if (!c->res_tmp && (rc = dalloc(c, &c->res_tmp, nr + ne))) return rc;
+        if (aside && c->res_saved) CK(cudaStreamWaitEvent(c->stream, c->res_ev, 0));
+        ElemArgs a = c->res_args;
+        a.Rh = a.Ro = c->res_tmp;
+        a.ru2 = c->res_tmp + nr;
+        {
+            Timed t(c, "element_blocks");
+            c->L->element_v[c->res_tf][c->res_gen](dim3(c->grid_elem_v[c->res_tf][c->res_gen]), c->L->elem_smem,
+                                                   c->stream, a);
+            if ((rc = check_launch(c, "element"))) return rc;
+        }
+        CK(cudaMemcpyAsync(c->Rh, c->Ro, sizeof(double) * nr, cudaMemcpyDeviceToDevice, c->stream));
+        int err = 0;
+        CK(cudaMemcpyAsync(&err, c->tc_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        flush_timer(c);
+        return wait_failure(c, err);
+    };
+    rc = form();
+    c->stream = saved;
+    if (aside) cudaThreadExchangeStreamCaptureMode(&mode);
+    if (rc == 0) c->res_blocks = false;
+    return rc;
 }
 
 int launch_getq(hfem_ctx* c, const double* duh, double alpha) {
@@ -669,8 +742,25 @@ int launch_getq(hfem_ctx* c, const double* duh, double alpha) {
     return check_launch(c, "getq");
 }
 
-int keep_blocks(hfem_ctx* c) { return c->res_blocks ? form_blocks(c) : 0; }
-int show_blocks(hfem_ctx* c) { return c->res_eager ? keep_blocks(c) : 0; }
+// Before a call that changes the tables, the mesh, the boundary or the problem map.
+int keep_blocks(hfem_ctx* c) { return blocks_pending(c) ? form_blocks(c) : 0; }
+// Before a call that changes u and uhat (1) or the source (2).
+int keep_state(hfem_ctx* c, int what) { return blocks_pending(c) ? set_aside(c, what) : 0; }
+// A captured call changes the state or the blocks each time its graph runs, unseen.
+int keep_captured(hfem_ctx* c) {
+    if (!capturing(c->stream)) return 0;
+    c->res_eager = true;
+    return keep_blocks(c);
+}
+// At the end of a call with residual-only passes.
+int show_blocks(hfem_ctx* c) {
+    if (!blocks_pending(c)) return 0;
+    if (c->res_eager) return form_blocks(c);
+    if (!c->res_track || (c->res_saved & 1)) return 0;
+    if (int rc = set_aside(c, 1)) return rc;
+    CK(cudaStreamSynchronize(c->stream));
+    return 0;
+}
 
 long long nvec(hfem_ctx* c) { return (long long)c->dims.nf * c->bsz; }
 
@@ -1679,7 +1769,7 @@ int hfem_destroy(hfem_ctx* c) {
     cudaStreamSynchronize(c->stream);
     void* ptrs[] = {c->shapvt, c->shapvg, c->svsv, c->shapft, c->shapfg, c->sfsf, c->perm, c->dgnodes, c->elcon,
                     c->rowstart, c->colidx, c->blk_src, c->face_src, c->rowface, c->colface, c->udg, c->uh, c->sh,
-                    c->D, c->F, c->K, c->H, c->Ru, c->DinvRu, c->Rh, c->Ro, c->ru2, c->Hg, c->Rg, c->Rr, c->status, c->ws, c->res_tmp, c->DinvF,
+                    c->D, c->F, c->K, c->H, c->Ru, c->DinvRu, c->Rh, c->Ro, c->ru2, c->Hg, c->Rg, c->Rr, c->status, c->ws, c->res_tmp, c->res_udg, c->res_uh, c->res_sh, c->DinvF,
                     c->info, c->Minv, c->V, c->w, c->x, c->pb, c->binfo, c->udgi,
                     c->eprob, c->fprob, c->pparam, c->palpha, c->seg_one.pstart, c->seg_one.pseg, c->seg_one.p0,
                     c->seg_one.ticket, c->seg_one.part, c->seg_map.pstart, c->seg_map.pseg, c->seg_map.p0,
@@ -1697,6 +1787,7 @@ int hfem_destroy(hfem_ctx* c) {
     }
     if (c->bilu_exec) cudaGraphExecDestroy(c->bilu_exec);
     for (cudaEvent_t ev : c->chunk_ev) cudaEventDestroy(ev);
+    if (c->res_ev) cudaEventDestroy(c->res_ev);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
@@ -1845,7 +1936,6 @@ int hfem_set_app(hfem_ctx* c, int appname) {
     if (!c) return HFEM_E_ARG;
     if (appname != 0 && appname != 1)
         return fail(c, HFEM_E_UNSUPPORTED, "appname %d (supported: 0 Euler, 1 Navier-Stokes)", appname);
-    if (int rk = keep_blocks(c)) return rk;
     c->appname = appname;
     c->assembled = false;
     return 0;
@@ -1858,7 +1948,6 @@ int hfem_set_models(hfem_ctx* c, int conv_stab, int viscosity_model) {
                     conv_stab);
     if (viscosity_model < 0 || viscosity_model > 1)
         return fail(c, HFEM_E_UNSUPPORTED, "viscosityModel %d (supported: 0 constant, 1 Sutherland)", viscosity_model);
-    if (int rk = keep_blocks(c)) return rk;
     c->conv_stab = conv_stab;
     c->visc_model = viscosity_model;
     c->assembled = false;
@@ -1869,7 +1958,6 @@ int hfem_set_physics(hfem_ctx* c, const double* param, int tdep, double fc_u, do
     if (!c || !param) return HFEM_E_ARG;
     if (!(param[0] > 1.0) || !(param[2] > 0.0) || !(param[3] > 0.0))
         return fail(c, HFEM_E_ARG, "physicsparam needs gamma > 1, Re > 0, Pr > 0");
-    if (int rk = keep_blocks(c)) return rk;
     for (int i = 0; i < 6; i++) c->param[i] = param[i];
     c->tdep = tdep;
     c->fc_u = fc_u;
@@ -1885,7 +1973,8 @@ static int set_solution_common(hfem_ctx* c, const double* udg, const double* uh,
     const size_t nudg = (size_t)d.ne * d.npv * c->nc, nuh = (size_t)d.nf * c->bsz;
     int rc;
     CK(cudaSetDevice(c->device));
-    if (int rk = keep_blocks(c)) return rk;
+    if (int rk = keep_captured(c)) return rk;
+    if (int rk = keep_state(c, 3)) return rk;
     if (!c->udg) {
         if ((rc = dalloc(c, &c->udg, nudg)) || (rc = dalloc(c, &c->uh, nuh)) || (rc = dalloc(c, &c->sh, nudg))) return rc;
     }
@@ -1924,6 +2013,7 @@ int hfem_assemble_host(hfem_ctx* c, const double* udg, const double* uh, const d
         CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         c->chunk_ev.push_back(ev);
     }
+    c->res_blocks = false;                  // the assembly replaces the blocks
     // the copies overwrite the state only after the work queued before them
     CK(cudaEventRecord(c->chunk_ev[0], c->stream));
     CK(cudaStreamWaitEvent(c->copy_stream, c->chunk_ev[0], 0));
@@ -1966,7 +2056,7 @@ int hfem_get_solution(hfem_ctx* c, double* udg, double* uh) {
 int hfem_getq(hfem_ctx* c) {
     int rc = ready(c);
     if (rc) return rc;
-    if (int rk = keep_blocks(c)) return rk;
+    if (int rk = keep_state(c, 1)) return rk;
     if ((rc = launch_getq(c, nullptr, 0.0))) return rc;
     CK(cudaStreamSynchronize(c->stream));
     flush_timer(c);
@@ -1977,7 +2067,7 @@ int hfem_getq(hfem_ctx* c) {
 int hfem_assemble(hfem_ctx* c, double* rnorm) { return run_assembly(c, true, rnorm); }
 
 int hfem_residual(hfem_ctx* c, double* rnorm) {
-    const int rc = run_assembly(c, false, rnorm);
+    const int rc = run_assembly(c, false, rnorm, c && c->res_track && !c->res_eager);
     return rc ? rc : show_blocks(c);
 }
 
@@ -1989,7 +2079,7 @@ int hfem_gmres(hfem_ctx* c, int precond, int restart, double tol, int maxit, int
 
 int hfem_update(hfem_ctx* c, double alpha) {
     if (!c) return HFEM_E_ARG;
-    if (int rk = keep_blocks(c)) return rk;
+    if (int rk = keep_state(c, 1)) return rk;
     return update_impl(c, alpha);
 }
 
@@ -2029,7 +2119,7 @@ static int newton_impl(hfem_ctx* c, double newton_tol, int newton_maxiter, int p
                     if (robust == 0) {
                         robust = 1;
                         alpha = -2.0 * std::fabs(alpha);
-                        if ((rc = keep_blocks(c))) return rc;
+                        if ((rc = keep_state(c, 1))) return rc;
                         if ((rc = update_impl(c, alpha))) return rc;
                     }
                     break;
@@ -2067,7 +2157,7 @@ static int dirk_impl(hfem_ctx* c, double dt, int stages, int order, double newto
     double d[9], t[3];
     if (!(dt > 0.0) || !dirk_table(stages, order, d, t))
         return fail(c, HFEM_E_ARG, "unsupported DIRK(%d,%d) or dt <= 0", stages, order);
-    if (newton_maxiter < 1 && (rc = keep_blocks(c))) return rc;     // else the first assembly replaces them
+    if (newton_maxiter < 1 && (rc = keep_state(c, 3))) return rc;   // else the first assembly replaces the blocks
     const hfem_dims& dm = c->dims;
     const long long n = (long long)dm.ne * dm.npv * c->nc;
     if (!c->udgi && (rc = dalloc(c, &c->udgi, (size_t)n))) return rc;
@@ -2186,7 +2276,7 @@ int hfem_update_problems(hfem_ctx* c, const double* alpha) {
     if (!c || !alpha) return HFEM_E_ARG;
     if (!c->nprob) return fail(c, HFEM_E_STATE, "no problem map");
     if (!c->assembled || !c->x) return fail(c, HFEM_E_STATE, "assemble and solve before update");
-    if (int rk = keep_blocks(c)) return rk;
+    if (int rk = keep_state(c, 1)) return rk;
     int rc;
     CK(cudaMemcpyAsync(c->palpha, alpha, sizeof(double) * c->nprob, cudaMemcpyHostToDevice, c->stream));
     axpy_prob_kernel<<<sms(c->device) * 4, 256, 0, c->stream>>>(nvec(c), c->bsz, c->fprob, c->palpha, c->x, c->uh);
@@ -2204,6 +2294,7 @@ int hfem_assemble_async(hfem_ctx* c) {
     int rc = ready(c);
     if (rc) return rc;
     if ((rc = ensure_assembly_buffers(c))) return rc;
+    if ((rc = keep_captured(c))) return rc;
     return enqueue_assembly(c, true);
 }
 
@@ -2306,6 +2397,7 @@ struct hfem_graph {
     cudaGraphExec_t exec = nullptr;
     std::vector<cudaStream_t> side;
     std::vector<cudaEvent_t> ev;
+    std::vector<std::shared_ptr<GraphRuns>> runs;   // of the contexts in it
 };
 
 // One CUDA graph holding the assembly of several contexts (e.g. one per
@@ -2320,11 +2412,11 @@ int hfem_graph_capture(hfem_ctx** ctxs, int n, void* stream, hfem_graph** out) {
         if (rc) return rc;
         if ((rc = ensure_assembly_buffers(ctxs[i]))) return rc;
         if ((rc = keep_blocks(ctxs[i]))) return rc;
-        ctxs[i]->res_eager = true;          // a launch of the graph does not pass through the context
         CK(cudaStreamSynchronize(ctxs[i]->stream));
     }
     CK(cudaSetDevice(c0->device));
     auto* g = new hfem_graph();
+    for (int i = 0; i < n; i++) g->runs.push_back(ctxs[i]->runs);
     g->side.resize(n);
     g->ev.resize(n + 1);
     for (int i = 0; i < n; i++) CK(cudaStreamCreateWithFlags(&g->side[i], cudaStreamNonBlocking));
@@ -2366,7 +2458,9 @@ int hfem_graph_capture(hfem_ctx** ctxs, int n, void* stream, hfem_graph** out) {
 
 int hfem_graph_launch(hfem_graph* g, void* stream) {
     if (!g || !g->exec || !stream) return HFEM_E_ARG;
-    return cudaGraphLaunch(g->exec, (cudaStream_t)stream) == cudaSuccess ? 0 : HFEM_E_CUDA;
+    if (cudaGraphLaunch(g->exec, (cudaStream_t)stream) != cudaSuccess) return HFEM_E_CUDA;
+    for (auto& r : g->runs) ++*r;
+    return 0;
 }
 
 int hfem_graph_destroy(hfem_graph* g) {
@@ -2428,7 +2522,6 @@ int hfem_set_precision(hfem_ctx* c, int mode) {
         return fail(c, HFEM_E_ARG, "precision mode must be 0 (FP64), 1 (3xTF32 element contractions, TF32 Schur, "
                                    "FP32 preconditioner), 2 (FP32 preconditioner) or 3 (3xTF32 element "
                                    "contractions, FP32 preconditioner)");
-    if (int rk = keep_blocks(c)) return rk;
     c->precision = mode;
     c->assembled = false;
     return 0;
@@ -2441,7 +2534,7 @@ int hfem_gmres_problems(hfem_ctx* c, int precond, int restart, double tol, int m
 
 int device_buffer(hfem_ctx* c, int what, const double** src, size_t* need) {
     const hfem_dims& d = c->dims;
-    if (c->res_blocks && (what == 5 || what == 6 || what == 10 || what == 13)) {
+    if (blocks_pending(c) && (what == 5 || what == 6 || what == 10 || what == 13)) {
         int rc = form_blocks(c);
         if (rc) return rc;
     }
@@ -2468,9 +2561,12 @@ int device_buffer(hfem_ctx* c, int what, const double** src, size_t* need) {
 
 int hfem_device_buffer(hfem_ctx* c, int what, const double** ptr, size_t* count) {
     if (!c || !ptr || !count) return HFEM_E_ARG;
-    if (what == 5 || what == 6 || what == 8 || what == 9 || what == 10 || what == 13) {
+    if (what == 5 || what == 6 || what == 10 || what == 13) {
         if (int rk = keep_blocks(c)) return rk;
         c->res_eager = true;
+    } else if (what == 8 || what == 9) {
+        if (int rk = keep_state(c, 1)) return rk;
+        c->res_track = true;
     }
     CK(cudaStreamSynchronize(c->stream));
     return device_buffer(c, what, ptr, count);

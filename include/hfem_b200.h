@@ -268,9 +268,10 @@ int hfem_gmres_problems(hfem_ctx* ctx, int precond, int restart, double tol, int
  * 13 element D^-1 after an
  * assembly (n*n*ne), 14 ||Ru_e||^2 before condensation (ne).  After a
  * residual-only pass 5, 6 and 10 are before condensation and 13 is D itself, at
- * the state of that pass (hfem_residual forms them when they are asked for or
- * before what they depend on changes, or at once in a context whose element
- * blocks or state hfem_device_buffer has handed out or which is part of a graph). */
+ * the state of that pass: hfem_residual notes its inputs, and they are formed when
+ * they are asked for, or at once in a context that has handed out pointers to them
+ * (hfem_device_buffer) or whose assembly the caller has captured into a graph of its
+ * own.  A later assembly or hfem_graph_launch replaces them. */
 int hfem_download(hfem_ctx* ctx, int what, double* host, size_t count);
 
 /* Per-kernel device time (ms) accumulated since the last reset, when timing
