@@ -1308,6 +1308,12 @@ const void* cycle_kernel(int bsz) {
     }
 }
 
+// The device, or the part of it that the stream may use, does not hold a whole
+// cooperative grid at once (anything else is an error).
+bool cooperative_refused(cudaError_t e) {
+    return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported;
+}
+
 // Rows of the one-kernel cycle: one CTA per SM, each a contiguous range of block
 // rows, cut at the problems' boundaries into pieces.  cyc_grid stays 0 for systems
 // that the cycle does not take: slices above CYC_MAXL entries (their steps are bound
@@ -1524,6 +1530,9 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
             CK(cudaMemsetAsync(c->gm_bar, 0, 4 * sizeof(unsigned), c->stream));
         }
         CK(cudaFuncSetAttribute(cyc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        int per_sm = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cyc, CYC_THREADS, cyc_smem));
+        if (per_sm * sms(c->device) < T.cyc_grid) cyc = nullptr;
         const size_t ld = (size_t)(restart + 1) * P;
         CA = CycleArgs{c->rowstart, c->colidx, c->Hg,
                        !prec ? nullptr : (c->precision >= 1 ? (const void*)c->Minv32 : (const void*)c->Minv), c->V, n,
@@ -1554,11 +1563,18 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
         // V_0 = M^-1 b - M^-1 A x (x = 0 in the first cycle), beta = |V_0|
         if (!first && (rc = op(c->x, c->V, nullptr))) return rc;
         run.start(c, SP, GS, first);
+        // A launch that the device cannot hold whole is refused, as on a stream that has
+        // part of the SMs: the kernels per step take over, from the same state.
         auto cycle = [&](int j0, int j1) -> int {
             CA.j0 = j0;
             CA.j1 = j1;
             void* args[] = {(void*)&CA, (void*)&GS};
-            CK(cudaLaunchCooperativeKernel(cyc, dim3(T.cyc_grid), dim3(CYC_THREADS), args, cyc_smem, c->stream));
+            const cudaError_t e =
+                cudaLaunchCooperativeKernel(cyc, dim3(T.cyc_grid), dim3(CYC_THREADS), args, cyc_smem, c->stream);
+            if (e == cudaSuccess) return 0;
+            if (!cooperative_refused(e)) return fail(c, HFEM_E_CUDA, "GMRES cycle kernel: %s", cudaGetErrorString(e));
+            cudaGetLastError();
+            cyc = nullptr;
             return 0;
         };
         if (cyc) CK(cudaMemsetAsync(c->gm_bar, 0, 3 * sizeof(unsigned), c->stream));
@@ -1567,12 +1583,17 @@ int gmres_impl(hfem_ctx* c, bool map, int precond, int restart, double tol, int 
             if ((rc = cycle(0, restart))) return rc;
         }
         for (int j = 0; j < restart && live && (!cyc || ext); j++) {
-            if ((rc = op(c->V + (size_t)j * n, c->V + (size_t)(j + 1) * n, ext ? nullptr : c->gm_sc + (size_t)j * P))) return rc;
-            {
+            double *vj = c->V + (size_t)j * n, *vn = vj + n;
+            const double* scj = c->gm_sc + (size_t)j * P;
+            if ((rc = op(vj, vn, cyc ? nullptr : scj))) return rc;
+            if (cyc) {
                 Timed t(c, "orthogonalise");
-                if (ext) rc = cycle(j, j + 1);
-                else run.step(c, SP, GS, n, j);
-                if (rc) return rc;
+                if ((rc = cycle(j, j + 1))) return rc;
+                if (!cyc && (rc = op(vj, vn, scj))) return rc;
+            }
+            if (!cyc) {
+                Timed t(c, "orthogonalise");
+                run.step(c, SP, GS, n, j);
             }
             if ((rc = check_launch(c, "arnoldi"))) return rc;
             if (((j + 1) % GM_CHECK == 0 || j + 1 == restart) && (rc = any_running(live))) return rc;
