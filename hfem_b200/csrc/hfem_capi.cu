@@ -642,6 +642,7 @@ int set_aside(hfem_ctx* c, int what) {
     const size_t nu = (size_t)c->dims.ne * c->dims.npv * c->nc, nuh = (size_t)c->dims.nf * c->bsz;
     const int todo = what & ~c->res_saved;
     int rc;
+    CK(cudaSetDevice(c->device));
     if (todo & 1) {
         if (!c->res_udg && ((rc = dalloc(c, &c->res_udg, nu)) || (rc = dalloc(c, &c->res_uh, nuh)))) return rc;
         CK(cudaMemcpyAsync(c->res_udg, c->udg, sizeof(double) * nu, cudaMemcpyDeviceToDevice, c->stream));
@@ -2283,6 +2284,7 @@ int hfem_set_problem_map(hfem_ctx* c, int nprob, const int* eprob, const int* fp
 int hfem_problem_rnorms(hfem_ctx* c, double* rnorm) {
     if (!c || !rnorm) return HFEM_E_ARG;
     if (!c->nprob || !c->ru2) return fail(c, HFEM_E_STATE, "no problem map or no residual yet");
+    CK(cudaSetDevice(c->device));
     problem_norm_kernel<<<c->nprob * NORM_SPLIT, NORM_THREADS, 0, c->stream>>>(ProblemNormArgs{
         c->bsz, c->ru2, c->Rr, c->eprob, c->fprob, c->pn_range, c->pn_part, c->pn_ticket, c->pn_out});
     int rc = check_launch(c, "problem_norm");
@@ -2299,6 +2301,7 @@ int hfem_update_problems(hfem_ctx* c, const double* alpha) {
     if (!c->assembled || !c->x) return fail(c, HFEM_E_STATE, "assemble and solve before update");
     if (int rk = keep_state(c, 1)) return rk;
     int rc;
+    CK(cudaSetDevice(c->device));
     CK(cudaMemcpyAsync(c->palpha, alpha, sizeof(double) * c->nprob, cudaMemcpyHostToDevice, c->stream));
     axpy_prob_kernel<<<sms(c->device) * 4, 256, 0, c->stream>>>(nvec(c), c->bsz, c->fprob, c->palpha, c->x, c->uh);
     if ((rc = check_launch(c, "uh update"))) return rc;
