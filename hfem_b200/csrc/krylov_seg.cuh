@@ -424,11 +424,12 @@ __global__ void __launch_bounds__(SEG_THREADS) seg_combine_kernel(SegPieces P, l
 }
 
 // z = xsc M^-1 (Hg x) with one warp per block row (xsc: a factor per segment,
-// NULL: 1).  A row's blocks are contiguous
-// in Hg, so the row is one column-major BSZ x (nblk * BSZ) matrix; the warp's
-// lanes form G = 32 / BSZ column groups of BSZ rows (R = 2 rows per lane when
-// BSZ > 32), and the groups' partial sums are added in group order.  Rows of
-// inactive segments (act[rseg[i]] == 0; rseg NULL: one segment) are skipped.
+// NULL: 1), for block sizes below 20.  A row's blocks are contiguous in Hg, so the row
+// is one column-major BSZ x (nblk * BSZ) matrix; the warp's lanes form G groups of
+// columns, and the groups' partial sums are added in group order.  Even block sizes: a
+// lane reads two rows of a column as one 16-byte load, BSZ / 2 lanes per column (2D p=2:
+// 0.91 -> 0.66 ms per 62 products).  Rows of inactive segments (act[rseg[i]] == 0; rseg
+// NULL: one segment) are skipped.
 template <int BSZ, typename MT>
 __global__ void __launch_bounds__(256) bsr_matvec_warp_kernel(int nrows, const int* __restrict__ rowstart,
                                                               const int* __restrict__ colidx,
@@ -438,99 +439,58 @@ __global__ void __launch_bounds__(256) bsr_matvec_warp_kernel(int nrows, const i
                                                               const double* __restrict__ xsc, double* __restrict__ z,
                                                               const int* __restrict__ rseg,
                                                               const unsigned char* __restrict__ act) {
-    constexpr int G = BSZ <= 32 ? 32 / BSZ : 1;
-    constexpr int R = (BSZ + 31) / 32;
-    constexpr int LDY = R * 32;
-    // even block sizes up to 32: a lane reads two rows of a column as one
-    // 16-byte load, BSZ / 2 lanes per column and G2 columns at a time (2D p=2:
-    // 0.91 -> 0.66 ms per 62 products; for BSZ = 50 the 25 busy lanes of this
-    // form were slower than two 8-byte loads per lane)
-    constexpr bool PAIRS = BSZ % 2 == 0 && BSZ <= 32;
-    constexpr int L2 = PAIRS ? BSZ / 2 : 1;
-    constexpr int G2 = PAIRS ? 32 / L2 : 1;
-    constexpr int GY = PAIRS ? G2 : G;
-    __shared__ double ys[8][GY][LDY];
+    static_assert(BSZ <= 32, "a lane per row");
+    constexpr bool PAIRS = BSZ % 2 == 0;
+    constexpr int LC = PAIRS ? BSZ / 2 : BSZ, G = 32 / LC;      // lanes per column, columns at a time
+    __shared__ double ys[8][G][32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int g = BSZ <= 32 ? lane / BSZ : 0;
-    const int r0 = BSZ <= 32 ? lane % BSZ : lane;
-    const bool on = g < G;
+    const int g = lane / LC, q = lane - g * LC;
     const int nwarps = gridDim.x * 8;
     for (int i = blockIdx.x * 8 + wib; i < nrows; i += nwarps) {
         if (act && !act[rseg ? rseg[i] : 0]) continue;
         const int k0 = rowstart[i], k1 = rowstart[i + 1];
         const int ncol = (k1 - k0) * BSZ;
         const double* A = Hg + (size_t)k0 * BSZ * BSZ;
-        double acc[R];
-#pragma unroll
-        for (int t = 0; t < R; t++) acc[t] = 0.0;
-        if constexpr (PAIRS) {
-            const int g2 = lane / L2, q = lane - g2 * L2;
-            if (g2 < G2) {
-                double a0 = 0.0, a1 = 0.0;
-#pragma unroll 4
-                for (int cc = g2; cc < ncol; cc += G2) {
-                    const int kb = cc / BSZ, c = cc - kb * BSZ;
-                    const double xv = __ldg(&x[(size_t)colidx[k0 + kb] * BSZ + c]);
-                    const double2 av = __ldg(reinterpret_cast<const double2*>(A + (size_t)cc * BSZ) + q);
-                    a0 += av.x * xv;
-                    a1 += av.y * xv;
-                }
-                ys[wib][g2][2 * q] = a0;
-                ys[wib][g2][2 * q + 1] = a1;
-            }
-        } else if (on) {
+        if (g < G) {
+            double a0 = 0.0, a1 = 0.0;
 #pragma unroll 4
             for (int cc = g; cc < ncol; cc += G) {
                 const int kb = cc / BSZ, c = cc - kb * BSZ;
                 const double xv = __ldg(&x[(size_t)colidx[k0 + kb] * BSZ + c]);
-#pragma unroll
-                for (int t = 0; t < R; t++) {
-                    const int r = r0 + 32 * t;
-                    if (r < BSZ) acc[t] += __ldg(&A[(size_t)cc * BSZ + r]) * xv;
+                if constexpr (PAIRS) {
+                    const double2 av = __ldg(reinterpret_cast<const double2*>(A + (size_t)cc * BSZ) + q);
+                    a0 += av.x * xv;
+                    a1 += av.y * xv;
+                } else {
+                    a0 += __ldg(&A[(size_t)cc * BSZ + q]) * xv;
                 }
             }
-#pragma unroll
-            for (int t = 0; t < R; t++) {
-                const int r = r0 + 32 * t;
-                if (r < BSZ) ys[wib][g][r] = acc[t];
+            if constexpr (PAIRS) {
+                ys[wib][g][2 * q] = a0;
+                ys[wib][g][2 * q + 1] = a1;
+            } else {
+                ys[wib][g][q] = a0;
             }
         }
         __syncwarp();
-        double y[R];
+        double y = 0.0;
+        if (lane < BSZ)
 #pragma unroll
-        for (int t = 0; t < R; t++) {
-            const int r = lane + 32 * t;
-            double s = 0.0;
-            if (r < BSZ)
-#pragma unroll
-                for (int gg = 0; gg < GY; gg++) s += ys[wib][gg][r];
-            y[t] = xsc ? s * xsc[rseg ? rseg[i] : 0] : s;
-        }
+            for (int gg = 0; gg < G; gg++) y += ys[wib][gg][lane];
+        if (xsc) y *= xsc[rseg ? rseg[i] : 0];
         __syncwarp();
         if (!Minv) {
-#pragma unroll
-            for (int t = 0; t < R; t++) {
-                const int r = lane + 32 * t;
-                if (r < BSZ) z[(size_t)i * BSZ + r] = y[t];
-            }
+            if (lane < BSZ) z[(size_t)i * BSZ + lane] = y;
             continue;
         }
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-            const int r = lane + 32 * t;
-            if (r < BSZ) ys[wib][0][r] = y[t];
-        }
+        if (lane < BSZ) ys[wib][0][lane] = y;
         __syncwarp();
         const MT* m = Minv + (size_t)i * BSZ * BSZ;
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-            const int r = lane + 32 * t;
-            if (r < BSZ) {
-                double s = 0.0;
+        if (lane < BSZ) {
+            double s = 0.0;
 #pragma unroll 4
-                for (int c = 0; c < BSZ; c++) s += (double)__ldg(&m[(size_t)c * BSZ + r]) * ys[wib][0][c];
-                z[(size_t)i * BSZ + r] = s;
-            }
+            for (int c = 0; c < BSZ; c++) s += (double)__ldg(&m[(size_t)c * BSZ + lane]) * ys[wib][0][c];
+            z[(size_t)i * BSZ + lane] = s;
         }
         __syncwarp();
     }
@@ -546,7 +506,7 @@ __global__ void __launch_bounds__(256) bsr_matvec_warp_kernel(int nrows, const i
 template <int BSZ>
 struct RowMv {
     static constexpr int L2 = BSZ / 2;
-    static constexpr int G = BSZ >= 50 ? 8 : (BSZ >= 30 ? 8 : 12);
+    static constexpr int G = BSZ >= 30 ? 8 : 12;
     static constexpr int USED = L2 * G;
     static constexpr int THREADS = (USED + 31) / 32 * 32;
     static constexpr int MC = (BSZ + G - 1) / G;      // columns of M^-1 per thread
