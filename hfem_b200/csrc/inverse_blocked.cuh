@@ -279,6 +279,7 @@ __global__ void __launch_bounds__(32 * WINV_WARPS) inverse_warp_kernel(int ne, d
     __shared__ __align__(16) double2 buf[WINV_WARPS][2][NB2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int e = blockIdx.x * WINV_WARPS + warp; e < ne; e += gridDim.x * WINV_WARPS) {
+        __syncwarp();       // the last matrix's reads of buf before this one's first pivot row
         double* De = D + (size_t)e * N * N;
         const int row = lane < N ? lane : N - 1;
         double a[2 * NB2];
