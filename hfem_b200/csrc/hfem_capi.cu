@@ -2324,6 +2324,7 @@ int hfem_assemble_async(hfem_ctx* c) {
 
 int hfem_assemble_finish(hfem_ctx* c, double* rnorm) {
     if (!c) return HFEM_E_ARG;
+    if (!c->info) return fail(c, HFEM_E_STATE, "no assembly to finish");
     return finish_assembly(c, true, rnorm);
 }
 
