@@ -23,10 +23,11 @@
 // are lifted here in full.  The face mass product uses shapfgdotshapfc = shapfg .* shapfc (its
 // definition, mkmasterelement.m:113-115) in factored form.
 //
-// Bound by no one unit: of 330k cycles per tetrahedron p = 3 the face rows take 123k
-// (their stores of K and H and the reductions into D, not the products), the volume
-// product 90k (A fragments formed from wrl as they are used), flux and Cholesky 33k,
-// the B operands 41k.  Before -> now (ms), Y and dual-number flux columns in memory
+// Bound by no one unit (DMMA pipe 50 % active, L1 58 %, DRAM 19 % over tetrahedra
+// p = 3): of 330k cycles per tetrahedron p = 3 the face rows take 129k (their stores of
+// K and H and the reductions into D, not the products), the volume product 87k (A
+// fragments formed from wrl as they are used), flux and Cholesky 32k, the B operands
+// 40k.  Before -> now (ms), Y and dual-number flux columns in memory
 // against fragments on the fly and flux Jacobians contracted as they are formed:
 // 13,182 3D p3 10.4 -> 7.7; 7,938 2D p4 1.22 -> 0.65; 2,048 2D p2 0.134 -> 0.066.  The
 // 3xTF32 form keeps Y and the dual-number flux, so that its results do not change.

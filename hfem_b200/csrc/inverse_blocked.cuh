@@ -266,7 +266,8 @@ __global__ void __launch_bounds__(InvBlk<N>::THREADS, 2)
 // subtracts g = f / pivot times the unscaled pivot row (broadcast through shared
 // memory) from every other row, and every row takes its own 1 / pivot once at the
 // end.  The pivots are the blocked kernel's (the first row of maximal |.|).
-// Bound by FP64 issue (a division and N + 2 operations per step).  Against the
+// Bound by the latency of a step's chain (the pivot search's warp reductions and the
+// pivot row through shared memory; FP64 pipe 16 % active, issue 30 %).  Against the
 // blocked kernel (us): 7,200 matrices of order 12, 39 -> 23; 2,048 of order 24, 29 ->
 // 25; 10,368 of order 20, 93 -> 63.
 constexpr int WINV_WARPS = 4;

@@ -2,10 +2,11 @@
 // sm_100a: Ru = Ru_vol + P Rh and Rh of every element, without the Jacobian blocks.
 //
 // The line search of a Newton iteration asks for the residual alone; the element
-// kernel formed all four blocks for it (1.74 ms per pass over 1,296 tetrahedra
-// p = 3, 14 of 47 ms of a DIRK step together with the matrix passes; this kernel:
-// 0.058 ms).  Bound by FP64 latency in the point states and fluxes: no block
-// products, so 128 threads and about 33 KB of shared memory, six CTAs per SM.
+// kernel formed all four blocks for it (0.87 ms per pass over 1,296 tetrahedra
+// p = 3, 7 of 47 ms of a DIRK step; this kernel: 0.058 ms).  Bound by FP64 latency in
+// the point states and fluxes (FP64 pipe 11 % active; stalls on global loads, on
+// fixed-latency results and at barriers, in this order): no block products, so 128
+// threads; four CTAs per SM, as many as 128 registers a thread allow.
 #pragma once
 #include <cuda_runtime.h>
 #include "elem_kernels.cuh"

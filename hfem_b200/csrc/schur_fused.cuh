@@ -13,7 +13,7 @@
 // writes the X strip over it, and strips are disjoint.
 // Bound by the FP64 tensor pipe (3D p=3: 24.4k DMMAs per element, 16.4 ms for
 // 48,000 at the measured 37 TFLOP/s).  13,182 tetrahedra p = 3: 8.27 -> 6.19 ms
-// (21.9 TFLOP/s algorithmic) against A tiles staged through a cp.async ring with a
+// (25.6 TFLOP/s) against A tiles staged through a cp.async ring with a
 // barrier per 20 columns and alpha A formed for every fragment.
 #pragma once
 #include <cuda_runtime.h>
