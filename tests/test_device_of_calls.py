@@ -1,6 +1,6 @@
 """Calls that a thread may make with another device current select the context's device
-ahead of their first launch, allocation or event, checked in the source (the boxes of
-this project have one GPU).
+ahead of their first launch, allocation or event, checked in the source (a run would
+need a second GPU).
 """
 import os
 import re
